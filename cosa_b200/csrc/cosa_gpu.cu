@@ -133,7 +133,8 @@ struct cosa_ctx {
   int *d_status = nullptr;
   int *d_row = nullptr;
   double *d_hist = nullptr;
-  const cosa_params *d_halo_p = nullptr;  // flow-condition slots read by k_halo (default: d_p)
+  BcPar *d_bcp = nullptr;                 // boundary values per flow-condition slot and level (k_bcpar)
+  const BcPar *d_halo_bcp = nullptr;      // those of the served solves' slots, read by k_halo instead of d_bcp
   // residual norms reduced per segment of tiles (one per served solve) when
   // set: segment s = tiles [d_seg[2s], +d_seg[2s+1]) with seg_ncell[s] cells
   int nseg = 0;
@@ -191,6 +192,7 @@ int build_level(cosa_ctx *c, LevelState &L, const cosa_level_desc &d, const int6
     if (x.im < 3 || x.jm < 3 || x.km < 2) return COSA_ERR_ARG;
     x.I3 = x.im + 3; x.J3 = x.jm + 3;
     x.P3 = (int64_t)(x.im + 3) * (x.jm + 3) * (x.km + 3);
+    if (x.P3 >= (int64_t)1 << 31) return COSA_ERR_ARG;  // 32-bit cell indices; 2^31 cells are 86 GB a state
     x.op3 = a3; x.op2 = a2; x.op1 = a1; x.of0 = a0; x.om1 = am;
     if (offs) { x.op3 = offs[3 * b]; x.op2 = offs[3 * b + 1]; x.op1 = offs[3 * b + 2]; }
     x.obct = (int)ab; x.nbcs = d.nbcs[b];
@@ -242,13 +244,13 @@ int build_level(cosa_ctx *c, LevelState &L, const cosa_level_desc &d, const int6
       for (int i3 = istrt[ic3]; i3 <= iend[ic3]; ++i3)
         for (int i2 = istrt[ic2]; i2 <= iend[ic2]; ++i2) {
           HaloItem it{};
-          it.dblk = it.sblk = b; it.type = type; it.idir = idir; it.mask = 3; it.sgn = sgn;
+          it.dblk = it.sblk = b; it.type = type; it.idir = (signed char)idir; it.mask = 3; it.sgn = (signed char)sgn;
           int i, j, k;
-          pcell(idir, ibcpt, i2, i3, i, j, k); it.h1 = p3_cell(x, i, j, k);
-          pcell(idir, ibcpt2, i2, i3, i, j, k); it.h2 = p3_cell(x, i, j, k);
-          pcell(idir, ibcn, i2, i3, i, j, k); it.c1 = p3_cell(x, i, j, k);
-          pcell(idir, ibcn2, i2, i3, i, j, k); it.c2 = p3_cell(x, i, j, k);
-          pcell(idir, ibcm, i2, i3, i, j, k); it.mface = i + I2 * (j + J2 * (int64_t)k);
+          pcell(idir, ibcpt, i2, i3, i, j, k); it.h1 = (int)p3_cell(x, i, j, k);
+          pcell(idir, ibcpt2, i2, i3, i, j, k); it.h2 = (int)p3_cell(x, i, j, k);
+          pcell(idir, ibcn, i2, i3, i, j, k); it.c1 = (int)p3_cell(x, i, j, k);
+          pcell(idir, ibcn2, i2, i3, i, j, k); it.c2 = (int)p3_cell(x, i, j, k);
+          pcell(idir, ibcm, i2, i3, i, j, k); it.mface = (unsigned)(i + I2 * (j + J2 * (int64_t)k));
           L.items.push_back(it);
         }
     }
@@ -281,20 +283,20 @@ int build_level(cosa_ctx *c, LevelState &L, const cosa_level_desc &d, const int6
         p1[ic1] = ibcpt; p1[ic2] = istr1[ic2] + isgn1[ic2] * i2; p1[ic3] = istr1[ic3] + isgn1[ic3] * i3;
         p2[jc1] = inr; p2[jc2] = istr2[jc2] + isgn2[jc2] * i2; p2[jc3] = istr2[jc3] + isgn2[jc3] * i3;
         HaloItem it{};
-        it.dblk = b1; it.sblk = b2; it.type = -1; it.idir = idir1; it.mask = 3; it.sgn = 1;
-        it.h1 = p3_cell(x1, p1[1], p1[2], p1[3]);
+        it.dblk = b1; it.sblk = b2; it.type = -1; it.idir = (signed char)idir1; it.mask = 3; it.sgn = 1;
+        it.h1 = (int)p3_cell(x1, p1[1], p1[2], p1[3]);
         p1[ic1] += ibcinc;
-        it.h2 = p3_cell(x1, p1[1], p1[2], p1[3]);
-        it.c1 = p3_cell(x2, p2[1], p2[2], p2[3]);
+        it.h2 = (int)p3_cell(x1, p1[1], p1[2], p1[3]);
+        it.c1 = (int)p3_cell(x2, p2[1], p2[2], p2[3]);
         p2[jc1] += inrinc;
-        it.c2 = p3_cell(x2, p2[1], p2[2], p2[3]);
+        it.c2 = (int)p3_cell(x2, p2[1], p2[2], p2[3]);
         it.mface = 0;
         L.items.push_back(it);
       }
   }
   if (bps)
     for (HaloItem &it : L.items) it.ps = bps[it.dblk];
-  for (HaloItem &it : L.items) it.nl = L.nl;
+  for (HaloItem &it : L.items) it.nl = (signed char)L.nl;
   // last writer of every halo cell keeps its write (reference order)
   {
     std::unordered_map<int64_t, int64_t> owner;
@@ -311,7 +313,7 @@ int build_level(cosa_ctx *c, LevelState &L, const cosa_level_desc &d, const int6
       int m = 0;
       if (owner[base + it.h1] == (int64_t)t * 2) m |= 1;
       if (owner[base + it.h2] == (int64_t)t * 2 + 1) m |= 2;
-      it.mask = m;
+      it.mask = (signed char)m;
     }
   }
   // ---- strong-boundary flags (muscl_b*, src/flux.f90:1318-1349, 1376-1406)
@@ -515,6 +517,35 @@ FaceVel face_vel_of(const cosa_ctx *c, const LevelState &L) {
 int after_launch(cosa_ctx *c) {
   c->launches++;
   return cuda_ok(cudaGetLastError());
+}
+
+// k_halo over `n` items from `items`.  Two threads per item while the launch
+// is smaller than kHaloSplit threads, which leaves most of the chip idle: one
+// cycle of the 64 x 32 x 2 channel (2.2 k items) 199 us split, 210 us not;
+// twenty of the 128 x 64 x 2 channel (5.6 k) 3.00 and 3.21 ms.  Above, the
+// doubled item reads and index work cost more than they hide.
+constexpr int64_t kHaloSplit = 75000;
+template <bool CONS>
+int launch_halo(cosa_ctx *c, LevelState &L, const HaloItem *items, int n, double *q, const double *si,
+                const double *sj, const double *sk, const double *dist, FaceVel fvel) {
+  const HaloPar h = make_halo_par(c->p);
+  const bool split = (int64_t)n * h.S * 2 <= kHaloSplit;
+  const dim3 g((unsigned)(((split ? 2 : 1) * (int64_t)n + 127) / 128), h.S);
+  const BcPar *bcp = c->d_halo_bcp ? c->d_halo_bcp : c->d_bcp;
+  auto k = c->p.npde > 5 ? (split ? k_halo<CONS, 7, true> : k_halo<CONS, 7, false>)
+                         : (split ? k_halo<CONS, 5, true> : k_halo<CONS, 5, false>);
+  k<<<g, 128, 0, c->s>>>(L.d_blocks, items, n, h, c->d_p, bcp, q, si, sj, sk, c->d_status, dist, fvel);
+  return after_launch(c);
+}
+const FaceVel kNoFaceVel{{nullptr, nullptr, nullptr}};
+
+// face halos of dst in conservative form from the primitive ones of src
+int launch_halo_p2c(cosa_ctx *c, LevelState &L, const double *src, double *dst) {
+  const int S = 2 * c->p.nharms + 1, n = (int)L.items.size();
+  const dim3 g((unsigned)((n + 127) / 128), S);
+  if (c->p.npde > 5) k_halo_p2c<7><<<g, 128, 0, c->s>>>(L.d_blocks, L.d_items, n, S, c->p.gamma, src, dst);
+  else k_halo_p2c<5><<<g, 128, 0, c->s>>>(L.d_blocks, L.d_items, n, S, c->p.gamma, src, dst);
+  return after_launch(c);
 }
 
 // CTAs along x for a multi-block launch over nb blocks of at most n items
@@ -768,9 +799,8 @@ int irs_apply(cosa_ctx *c, LevelState &L, double *res, double *ores, const doubl
     const int ncut = (int)L.items.size() - L.n_bc_items;
     for (int its = 0; its < 2; ++its) {
       if (ncut > 0) {
-        k_halo<false><<<grid_for((int64_t)ncut * S), 256, 0, c->s>>>(L.d_blocks, L.d_items + L.n_bc_items, ncut, c->d_p,
-                                                                    res, nullptr, nullptr, nullptr, c->d_status);
-        if ((r = after_launch(c))) return r;
+        if ((r = launch_halo<false>(c, L, L.d_items + L.n_bc_items, ncut, res, nullptr, nullptr, nullptr, nullptr, kNoFaceVel)))
+          return r;
       }
       if ((r = sweeps(ores, 1))) return r;
     }
@@ -919,12 +949,8 @@ int launch_stage(cosa_ctx *c, int nl, LevelState &L, double *qin, double *qout, 
   const int S = 2 * p.nharms + 1;
   const cosa_level_ptrs &P = L.ptrs;
   if (!L.items.empty()) {
-    const int64_t n = (int64_t)L.items.size() * S;
-    if (c->prof.on) cudaEventRecord(c->prof.ev[0][0], c->s);
-    k_halo<true><<<grid_for(n), 256, 0, c->s>>>(L.d_blocks, L.d_items, (int)L.items.size(),
-                                                c->d_halo_p ? c->d_halo_p : c->d_p, qin, P.si, P.sj, P.sk,
-                                                c->d_status, nullptr, face_vel_of(c, L));
-    int r = after_launch(c);
+        if (c->prof.on) cudaEventRecord(c->prof.ev[0][0], c->s);
+    int r = launch_halo<true>(c, L, L.d_items, (int)L.items.size(), qin, P.si, P.sj, P.sk, nullptr, face_vel_of(c, L));
     if (r) return r;
     if (c->prof.on) prof_stop(c, 0);
   }
@@ -1359,12 +1385,14 @@ int cosa_gpu_init(const cosa_params *p, int32_t nlevels, const cosa_level_desc *
   c->nlevels = nlevels;
   int r = 0;
   if ((r = cuda_ok(cudaStreamCreateWithFlags(&c->s, cudaStreamNonBlocking))) ||
-      (r = dalloc(c, &c->d_p, 1)) || (r = dalloc(c, &c->d_status, 1)) || (r = dalloc(c, &c->d_row, 1)) ||
+      (r = dalloc(c, &c->d_p, 1)) || (r = dalloc(c, &c->d_bcp, COSA_MAX_LEVELS)) ||
+      (r = dalloc(c, &c->d_status, 1)) || (r = dalloc(c, &c->d_row, 1)) ||
       (r = set_smem_attrs())) {
     cosa_gpu_finalize(c);
     return r;
   }
   cudaMemcpy(c->d_p, p, sizeof(cosa_params), cudaMemcpyHostToDevice);
+  k_bcpar<<<1, 32, 0, c->s>>>(c->d_p, 1, c->d_bcp);
   cudaMemset(c->d_status, 0, sizeof(int));
   cudaMemset(c->d_row, 0, sizeof(int));
   for (int l = 0; l < nlevels; ++l) {
@@ -1397,6 +1425,8 @@ int cosa_gpu_set_params(cosa_ctx *c, const cosa_params *p) {
   if (p->npde != c->p.npde || p->nharms != c->p.nharms) return COSA_ERR_ARG;
   c->p = *p;
   CK(cudaMemcpyAsync(c->d_p, p, sizeof(cosa_params), cudaMemcpyHostToDevice, c->s));
+  k_bcpar<<<1, 32, 0, c->s>>>(c->d_p, 1, c->d_bcp);
+  CK(cudaGetLastError());
   CK(cudaStreamSynchronize(c->s));
   drop_graphs(c);
   return COSA_OK;
@@ -1483,11 +1513,7 @@ int cosa_gpu_bc(cosa_ctx *c, int32_t nl, double *q, const double *si, const doub
   LevelState *L = level(c, nl);
   if (!L || !q) return COSA_ERR_ARG;
   if (L->n_bc_items == 0) return COSA_OK;
-  const int S = 2 * c->p.nharms + 1;
-  k_halo<false><<<grid_for((int64_t)L->n_bc_items * S), 256, 0, c->s>>>(L->d_blocks, L->d_items, L->n_bc_items,
-                                                                       c->d_p, q, si, sj, sk, c->d_status, dist,
-                                                                       face_vel_of(c, *L));
-  return after_launch(c);
+  return launch_halo<false>(c, *L, L->d_items, L->n_bc_items, q, si, sj, sk, dist, face_vel_of(c, *L));
 }
 
 int cosa_gpu_cutman_q(cosa_ctx *c, int32_t nl, double *q) {
@@ -1495,10 +1521,7 @@ int cosa_gpu_cutman_q(cosa_ctx *c, int32_t nl, double *q) {
   if (!L || !q) return COSA_ERR_ARG;
   const int ncut = (int)L->items.size() - L->n_bc_items;
   if (ncut == 0) return COSA_OK;
-  const int S = 2 * c->p.nharms + 1;
-  k_halo<false><<<grid_for((int64_t)ncut * S), 256, 0, c->s>>>(L->d_blocks, L->d_items + L->n_bc_items, ncut, c->d_p, q,
-                                                              nullptr, nullptr, nullptr, c->d_status);
-  return after_launch(c);
+  return launch_halo<false>(c, *L, L->d_items + L->n_bc_items, ncut, q, nullptr, nullptr, nullptr, nullptr, kNoFaceVel);
 }
 
 int cosa_gpu_prtest(cosa_ctx *c, int32_t nl, const double *q) {
@@ -1734,11 +1757,7 @@ int cosa_gpu_smooth(cosa_ctx *c, int32_t nl, int32_t niter, int32_t mgit0, int32
   // (the k-omega stage converts them itself, src/update.f90:1875-2084)
   if (niter > 0 && !L->items.empty() && !routine_stage(c->p)) {
     double *last_in = (c->p.nstage % 2 == 0) ? L->d_T : L->ptrs.q;
-    const int S = 2 * c->p.nharms + 1;
-    k_halo_p2c<<<grid_for((int64_t)L->items.size() * S), 256, 0, c->s>>>(L->d_blocks, L->d_items,
-                                                                        (int)L->items.size(), c->d_p, last_in,
-                                                                        L->ptrs.q);
-    if ((r = after_launch(c))) return r;
+    if ((r = launch_halo_p2c(c, *L, last_in, L->ptrs.q))) return r;
   }
   if (hist) {
     std::vector<double> h(rows.size() * (npde + 1));
@@ -2130,10 +2149,7 @@ int issue_smooth_level(cosa_ctx *c, int nl, int niter, bool from_fine, bool to_c
   // (the k-omega stage converts them itself)
   if (niterp > 0 && !L.items.empty() && !routine_stage(p)) {
     double *last_in = (to_coarse || p.nstage % 2 == 1) ? L.ptrs.q : L.d_T;
-    const int S = 2 * p.nharms + 1;
-    k_halo_p2c<<<grid_for((int64_t)L.items.size() * S), 256, 0, c->s>>>(L.d_blocks, L.d_items, (int)L.items.size(),
-                                                                       c->d_p, last_in, L.ptrs.q);
-    if ((r = after_launch(c))) return r;
+    if ((r = launch_halo_p2c(c, L, last_in, L.ptrs.q))) return r;
   }
   return COSA_OK;
 }
@@ -2338,9 +2354,7 @@ int cosa_gpu_rkuns(cosa_ctx *c, int32_t ntime, int32_t iprint, double *hist) {
   }
   if (ntime > 0 && !L->items.empty()) {
     double *last_in = (p.nstage % 2 == 0) ? L->d_T : L->ptrs.q;
-    k_halo_p2c<<<grid_for((int64_t)L->items.size()), 256, 0, c->s>>>(L->d_blocks, L->d_items, (int)L->items.size(),
-                                                                      c->d_p, last_in, L->ptrs.q);
-    if ((r = after_launch(c))) return r;
+    if ((r = launch_halo_p2c(c, *L, last_in, L->ptrs.q))) return r;
   }
   if (hist) {
     const int npde = p.npde;
@@ -3166,10 +3180,8 @@ int launch_rans_stage(cosa_ctx *c, int nl, LevelState &L, int irk, const IterOpt
   if ((r = cosa_gpu_cons2prim(c, nl, 0, q))) return r;
   if (!L.items.empty()) {
     // BC patches then cuts, last writers as in the reference
-    k_halo<false><<<grid_for((int64_t)L.items.size() * S), 256, 0, c->s>>>(
-        L.d_blocks, L.d_items, (int)L.items.size(), c->d_p, q, P.si, P.sj, P.sk, c->d_status, P.dist,
-        face_vel_of(c, L));
-    if ((r = after_launch(c))) return r;
+    if ((r = launch_halo<false>(c, L, L.d_items, (int)L.items.size(), q, P.si, P.sj, P.sk, P.dist, face_vel_of(c, L))))
+      return r;
   }
   if (o.first_cycle && o.force && irk == 1 && !p.prd_all_lvls) {
     // coarse-level mut from the restricted (primitive) state at the first
@@ -3372,10 +3384,8 @@ int launch_lsp_stage(cosa_ctx *c, int nl, LevelState &L, int irk, const IterOpts
     return r;
   if ((r = cosa_gpu_cons2prim(c, nl, 0, q))) return r;
   if (!L.items.empty()) {
-    k_halo<false><<<grid_for((int64_t)L.items.size() * S), 256, 0, c->s>>>(
-        L.d_blocks, L.d_items, (int)L.items.size(), c->d_p, q, P.si, P.sj, P.sk, c->d_status, P.dist,
-        face_vel_of(c, L));
-    if ((r = after_launch(c))) return r;
+    if ((r = launch_halo<false>(c, L, L.d_items, (int)L.items.size(), q, P.si, P.sj, P.sk, P.dist, face_vel_of(c, L))))
+      return r;
   }
   if ((r = for_blocks(c, L, cnt_all, [&](auto b, dim3 g) { k_prtest<<<g, 256, 0, c->s>>>(b, c->d_p, q, c->d_status); })))
     return r;

@@ -28,17 +28,20 @@
 #include "physics.cuh"
 #include "kernels_ref.cuh"
 
-struct HaloItem {
+// one boundary or cut face cell: 48 bytes, read as three 16-byte words.
+// Cell indices inside a block fit 32 bits (2^31 cells are 17 GB a variable).
+struct __align__(16) HaloItem {
+  int h1, h2;       // halo cells (p3 cell index in dblk)
+  int c1, c2;       // interior cells (p3 cell index in sblk)
   int dblk, sblk;   // destination / source block (0-based)
-  int type;         // BC type, -1 = cut copy
-  int idir;         // direction of the face (1..3)
-  int mask;         // bit0: write first halo layer, bit1: second
-  int sgn;          // sign applied to the face normal
-  int64_t h1, h2;   // halo cells (p3 cell index in dblk)
-  int64_t c1, c2;   // interior cells (p3 cell index in sblk)
-  int64_t mface;    // metric cell index (i + I2*(j + J2*k)) of the face in dblk
+  unsigned mface;   // metric cell index (i + I2*(j + J2*k)) of the face in dblk
   int ps;           // slot of the flow conditions (BC values) in the params array
-  int nl;           // multigrid level of the item's block (the low-speed cut-off epsp(nl))
+  int type;         // BC type, -1 = cut copy
+  signed char idir; // direction of the face (1..3)
+  signed char mask; // bit0: write first halo layer, bit1: second
+  signed char sgn;  // sign applied to the face normal
+  signed char nl;   // multigrid level of the item's block (the low-speed cut-off epsp(nl))
+  int pad[2];
 };
 
 struct Tile {
@@ -66,91 +69,145 @@ struct FaceVel {
   const double *f[3];
 };
 
-template <bool CONS>
-__global__ void k_halo(const DevBlock *__restrict__ blocks, const HaloItem *__restrict__ items, int nitems,
-                       const cosa_params *__restrict__ Pp, double *__restrict__ q,
-                       const double *__restrict__ si, const double *__restrict__ sj,
-                       const double *__restrict__ sk, int *status, const double *__restrict__ dist = nullptr,
-                       FaceVel fvel = FaceVel{{nullptr, nullptr, nullptr}}) {
-  const cosa_params &P = *Pp;
-  const int npde = P.npde, S = 2 * P.nharms + 1, S2 = 2 * P.nharms * P.hbmove + 1;
-  const int64_t total = (int64_t)nitems * S;
+// the boundary values of every flow-condition slot and level (make_bcpar:
+// sines, cosines and a power), once per upload of the parameters instead of
+// once per halo cell and stage.  With them inside k_halo took 19.7 us on the
+// 128 x 64 x 2 channel and 92 us on the 4.2 M-cell duct (463 k items); with
+// this, 48-byte items and one snapshot per grid row twenty channel cycles
+// went from 3.34 to 2.90 ms, a cycle of the 30.7 M-cell duct from 21.8 to
+// 21.3 ms, five of the pitching aerofoil (S = 5) from 2.71 to 2.24 ms
+__global__ void k_bcpar(const cosa_params *__restrict__ Pp, int nslots, BcPar *__restrict__ out) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < nslots * COSA_MAX_LEVELS) out[t] = make_bcpar(Pp[t / COSA_MAX_LEVELS], t % COSA_MAX_LEVELS + 1);
+}
+
+// scalars of k_halo, passed by value
+struct HaloPar {
+  int S, S2, hbmove;
+  double gamma, qmin_rho, qmin_p;
+};
+inline HaloPar make_halo_par(const cosa_params &P) {
+  HaloPar h;
+  h.S = 2 * P.nharms + 1; h.S2 = 2 * P.nharms * P.hbmove + 1; h.hbmove = P.hbmove;
+  h.gamma = P.gamma; h.qmin_rho = P.qmin[0]; h.qmin_p = P.qmin[4];
+  return h;
+}
+
+// Bound by the latency of one item's chain on small grids, by the strided
+// cells of the i faces on large ones.  SPLIT: two threads per item, one per
+// halo layer (neighbouring lanes share the item), for launches that leave the
+// chip idle anyway: the subsonic inlet's two Newton iterations, the longest
+// chain here (powers), run side by side (kHaloSplit in cosa_gpu.cu).
+// Snapshot n = blockIdx.y.
+template <bool CONS, int NV, bool SPLIT>
+__global__ void __launch_bounds__(128)
+k_halo(const DevBlock *__restrict__ blocks, const HaloItem *__restrict__ items, int nitems,
+       const HaloPar H, const cosa_params *__restrict__ Pp, const BcPar *__restrict__ bcp,
+       double *__restrict__ q, const double *__restrict__ si, const double *__restrict__ sj,
+       const double *__restrict__ sk, int *status, const double *__restrict__ dist = nullptr,
+       FaceVel fvel = FaceVel{{nullptr, nullptr, nullptr}}) {
+  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int64_t item = SPLIT ? t >> 1 : t;
+  if (item >= nitems) return;
+  const int n = blockIdx.y;
+  const HaloItem it = items[item];
+  // the layers of this thread; a layer that a later item overwrites is not
+  // written, but an inlet's Newton iteration is checked wherever it stands
+  const int mine = SPLIT ? 1 << (int)(t & 1) : 3;
+  int write = it.mask & mine;
+  if (!write && it.type != 21) return;
   int st = 0;
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-    const HaloItem it = items[t % nitems];
-    const int n = (int)(t / nitems);
-    const DevBlock sb = blocks[it.sblk], db = blocks[it.dblk];
-    double c1[7], c2[7], h1[7], h2[7];
-    for (int v = 0; v < npde; ++v) {
-      const int64_t base = p3_var(sb, npde, S, v + 1, n);
-      c1[v] = q[base + it.c1];
-      c2[v] = q[base + it.c2];
+  const DevBlock &db = blocks[it.dblk], &sb = blocks[it.sblk];
+  const double *qs = q + p3_var(sb, NV, H.S, 1, n);
+  const int64_t sP3 = sb.P3, dP3 = db.P3;
+  double h1[NV], h2[NV];
+  if (it.type < 0) {
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+      if (mine & 1) h1[v] = qs[v * sP3 + it.c1];
+      if (mine & 2) h2[v] = qs[v * sP3 + it.c2];
     }
     if (CONS) {
-      if (npde > 5) { c2p7(P.gamma, c1); c2p7(P.gamma, c2); }
-      else { c2p5(P.gamma, c1); c2p5(P.gamma, c2); }
+      if (mine & 1) { if (NV > 5) c2p7(H.gamma, h1); else c2p5(H.gamma, h1); }
+      if (mine & 2) { if (NV > 5) c2p7(H.gamma, h2); else c2p5(H.gamma, h2); }
+    }
+  } else {
+    double c1[NV], c2[NV];
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+      c1[v] = qs[v * sP3 + it.c1];
+      c2[v] = qs[v * sP3 + it.c2];
+    }
+    double nx = 0, ny = 0, nz = 0;
+    if (it.type == 14 || it.type == 21 || it.type == 30 || it.type == 31 || (NV > 5 && it.type / 100 == 15)) {
+      const double *s = it.idir == 1 ? si : (it.idir == 2 ? sj : sk);
+      const int64_t I2 = db.im + 2, J2 = db.jm + 2, K2 = db.km + 2;
+      const int64_t e = ((db.op2 * H.S2) + (int64_t)(n * H.hbmove) * I2 * J2 * K2 + it.mface) * 4;
+      const double2 a = __ldg(reinterpret_cast<const double2 *>(s + e));
+      nx = a.x * it.sgn; ny = a.y * it.sgn; nz = __ldg(s + e + 2) * it.sgn;
+    }
+    if (CONS) {
+      if (NV > 5) { c2p7(H.gamma, c1); c2p7(H.gamma, c2); }
+      else { c2p5(H.gamma, c1); c2p5(H.gamma, c2); }
+    }
+    const BcPar &B = bcp[it.ps * COSA_MAX_LEVELS + it.nl - 1];
+    int err = 0;
+    // moving walls: the velocity of the wall face (snapshot nh)
+    double wv[3];
+    const double *wvp = nullptr;
+    const double *f = it.idir == 1 ? fvel.f[0] : (it.idir == 2 ? fvel.f[1] : fvel.f[2]);
+    if ((it.type == 14 || it.type / 100 == 15) && f) {
+      const int64_t I2 = db.im + 2, J2 = db.jm + 2, K2 = db.km + 2;
+      const int64_t e = ((db.op2 * H.S2) + (int64_t)(n * H.hbmove) * I2 * J2 * K2 + it.mface) * 3;
+      wv[0] = f[e]; wv[1] = f[e + 1]; wv[2] = f[e + 2];
+      wvp = wv;
     }
     int mask = 0;
-    if (it.type < 0) {
-      for (int v = 0; v < npde; ++v) { h1[v] = c1[v]; h2[v] = c2[v]; }
-      mask = 3;
-    } else {
-      double nx = 0, ny = 0, nz = 0;
-      if (it.type == 14 || it.type == 21 || it.type == 30 || it.type == 31 || (it.type / 100 == 15 && npde > 5)) {
-        const double *s = it.idir == 1 ? si : (it.idir == 2 ? sj : sk);
-        const int nh = n * P.hbmove;
-        const int64_t I2 = db.im + 2, J2 = db.jm + 2, K2 = db.km + 2;
-        const int64_t e = ((db.op2 * S2) + (int64_t)nh * I2 * J2 * K2 + it.mface) * 4;
-        nx = s[e] * it.sgn; ny = s[e + 1] * it.sgn; nz = s[e + 2] * it.sgn;
-      }
-      const BcPar B = make_bcpar(Pp[it.ps], it.nl);
-      int err = 0;
-      // moving walls: the velocity of the wall face (snapshot nh)
-      double wv[3];
-      const double *wvp = nullptr;
-      if ((it.type == 14 || it.type / 100 == 15) && fvel.f[it.idir - 1]) {
-        const int64_t I2 = db.im + 2, J2 = db.jm + 2, K2 = db.km + 2;
-        const int64_t e = ((db.op2 * S2) + (int64_t)(n * P.hbmove) * I2 * J2 * K2 + it.mface) * 3;
-        const double *f = fvel.f[it.idir - 1];
-        wv[0] = f[e]; wv[1] = f[e + 1]; wv[2] = f[e + 2];
-        wvp = wv;
-      }
-      switch (it.type) {
-        case 80: mask = bc_sym(it.idir, npde, c1, c2, h1, h2); break;
-        case 4: mask = bc_extrapol(npde, c1, h1, h2); break;
-        case 14: mask = bc_walinv(npde, nx, ny, nz, c1, c2, h1, h2, wvp); break;
-        case 21: mask = bc_insub(B, nx, ny, nz, c1, c2, h1, h2, &err); break;
-        case 91: mask = bc_outsub(B, c1, c2, h1, h2); break;
-        case 30: mask = bc_far0(B, nx, ny, nz, c1, h1, h2); break;
-        case 31: mask = bc_far1(B, nx, ny, nz, c1, h1, h2); break;
-        default:
-          if (it.type / 100 == 15) {
-            mask = bc_walvis(P.gamma, c1, c2, h1, h2, wvp);
-            if (npde > 5) {
-              // k-omega wall values from the wall distance of the first cell
-              if (!dist) { st |= COSA_ERR_ARG; break; }
-              const int64_t I3 = db.I3, J3 = db.J3;
-              const int ci = (int)(it.c1 % I3) - 1, cj = (int)((it.c1 / I3) % J3) - 1;
-              const int ck = (int)(it.c1 / (I3 * J3)) - 1;
-              bc_walvis_kom(P, nx, ny, nz, dist[p1_idx(db, 1, ci, cj, ck, 0)], c1, h1, h2, wvp);
-            }
-          } else {
-            st |= COSA_ERR_UNSUPPORTED;
+    switch (it.type) {
+      case 80: mask = bc_sym(it.idir, NV, c1, c2, h1, h2); break;
+      case 4: mask = bc_extrapol(NV, c1, h1, h2); break;
+      case 14: mask = bc_walinv(NV, nx, ny, nz, c1, c2, h1, h2, wvp); break;
+      case 21:
+        if (SPLIT) {
+          bc_insub_layer<NV>(B, nx, ny, nz, c1, c2, (int)(t & 1), h1, &err);
+#pragma unroll
+          for (int v = 0; v < NV; ++v) h2[v] = h1[v];
+        } else {
+          bc_insub_layer<NV>(B, nx, ny, nz, c1, c2, 0, h1, &err);
+          bc_insub_layer<NV>(B, nx, ny, nz, c1, c2, 1, h2, &err);
+        }
+        mask = 3;
+        break;
+      case 91: mask = bc_outsub<NV>(B, c1, c2, h1, h2); break;
+      case 30: mask = bc_far0<NV>(B, nx, ny, nz, c1, h1, h2); break;
+      case 31: mask = bc_far1<NV>(B, nx, ny, nz, c1, h1, h2); break;
+      default:
+        if (it.type / 100 == 15) {
+          mask = bc_walvis(H.gamma, c1, c2, h1, h2, wvp);
+          if (NV > 5) {
+            // k-omega wall values from the wall distance of the first cell
+            if (!dist) { st |= COSA_ERR_ARG; break; }
+            const int I3 = db.I3, J3 = db.J3;
+            const int ci = it.c1 % I3 - 1, cj = (it.c1 / I3) % J3 - 1, ck = it.c1 / (I3 * J3) - 1;
+            bc_walvis_kom(*Pp, nx, ny, nz, dist[p1_idx(db, 1, ci, cj, ck, 0)], c1, h1, h2, wvp);
           }
-          break;
-      }
-      if (err) st |= COSA_ERR_INFLOW;
+        } else {
+          st |= COSA_ERR_UNSUPPORTED;
+        }
+        break;
     }
-    mask &= it.mask;
-    for (int v = 0; v < npde; ++v) {
-      const int64_t base = p3_var(db, npde, S, v + 1, n);
-      if (mask & 1) q[base + it.h1] = h1[v];
-      if (mask & 2) q[base + it.h2] = h2[v];
-    }
-    if (CONS && it.idir == 1) {  // bprtest also checks the i halos of the state (src/cosa.f90:1000)
-      if (mask & 1) { if (h1[4] <= P.qmin[4]) st |= COSA_ERR_NEG_P; else if (h1[0] <= P.qmin[0]) st |= COSA_ERR_NEG_RHO; }
-      if (mask & 2) { if (h2[4] <= P.qmin[4]) st |= COSA_ERR_NEG_P; else if (h2[0] <= P.qmin[0]) st |= COSA_ERR_NEG_RHO; }
-    }
+    if (err) st |= COSA_ERR_INFLOW;
+    write &= mask;
+  }
+  double *qd = q + p3_var(db, NV, H.S, 1, n);
+#pragma unroll
+  for (int v = 0; v < NV; ++v) {
+    if (write & 1) qd[v * dP3 + it.h1] = h1[v];
+    if (write & 2) qd[v * dP3 + it.h2] = h2[v];
+  }
+  if (CONS && it.idir == 1) {  // bprtest also checks the i halos of the state (src/cosa.f90:1000)
+    if (write & 1) { if (h1[4] <= H.qmin_p) st |= COSA_ERR_NEG_P; else if (h1[0] <= H.qmin_rho) st |= COSA_ERR_NEG_RHO; }
+    if (write & 2) { if (h2[4] <= H.qmin_p) st |= COSA_ERR_NEG_P; else if (h2[0] <= H.qmin_rho) st |= COSA_ERR_NEG_RHO; }
   }
   if (st) atomicOr(status, st);
 }
@@ -566,22 +623,25 @@ __global__ void k_copy_interior(BS bs_, int nvar_snap, const double *__restrict_
 // ---- stage finalisation: face halos of q in conservative form ----------------------------
 // After smooth(), the reference's q holds prim2cons of the last stage's
 // halo values (src/cosa.f90:1908).  src holds those values in primitive form.
+template <int NV>
 __global__ void k_halo_p2c(const DevBlock *__restrict__ blocks, const HaloItem *__restrict__ items, int nitems,
-                           const cosa_params *__restrict__ Pp, const double *__restrict__ src, double *__restrict__ dst) {
-  const cosa_params &P = *Pp;
-  const int npde = P.npde, S = 2 * P.nharms + 1;
-  const int64_t total = (int64_t)nitems * S;
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-    const HaloItem it = items[t % nitems];
-    const int n = (int)(t / nitems);
-    const DevBlock db = blocks[it.dblk];
-    for (int layer = 0; layer < 2; ++layer) {
-      if (!((it.mask >> layer) & 1)) continue;
-      const int64_t c = layer ? it.h2 : it.h1;
-      double v[7];
-      for (int m = 0; m < npde; ++m) v[m] = src[p3_var(db, npde, S, m + 1, n) + c];
-      p2c(P.gamma, v, npde);
-      for (int m = 0; m < npde; ++m) dst[p3_var(db, npde, S, m + 1, n) + c] = v[m];
-    }
+                           int S, double gamma, const double *__restrict__ src, double *__restrict__ dst) {
+  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (t >= nitems) return;
+  const HaloItem it = items[t];
+  const DevBlock &db = blocks[it.dblk];
+  const int64_t P3 = db.P3, o = p3_var(db, NV, S, 1, blockIdx.y);
+  double v[2][NV];
+#pragma unroll
+  for (int m = 0; m < NV; ++m) {
+    v[0][m] = src[o + m * P3 + it.h1];
+    v[1][m] = src[o + m * P3 + it.h2];
+  }
+  p2c(gamma, v[0], NV);
+  p2c(gamma, v[1], NV);
+#pragma unroll
+  for (int m = 0; m < NV; ++m) {
+    if (it.mask & 1) dst[o + m * P3 + it.h1] = v[0][m];
+    if (it.mask & 2) dst[o + m * P3 + it.h2] = v[1][m];
   }
 }

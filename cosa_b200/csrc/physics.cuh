@@ -616,10 +616,11 @@ __device__ __forceinline__ int bc_walinv(int npde, double nx, double ny, double 
   return 3;
 }
 // bc_insub (src/bc.f90:875-1175): subsonic inlet, Newton on the normal
-// velocity; n already multiplied by sgnm.  Returns mask, sets *err on a
-// Newton iteration count of 10 (the reference stops there).
-__device__ __forceinline__ int bc_insub(const BcPar &B, double nx, double ny, double nz, const double *c1,
-                                        const double *c2, double *h1, double *h2, int *err) {
+// velocity; n already multiplied by sgnm.  Fills one halo layer (lay 0 or 1)
+// and sets *err on a Newton iteration count of 10 (the reference stops there).
+template <int NV>
+__device__ __forceinline__ void bc_insub_layer(const BcPar &B, double nx, double ny, double nz, const double *c1,
+                                               const double *c2, int lay, double *h, int *err) {
   const double g = B.g;
   const double rho1 = c1[0], rho2 = c2[0];
   const double un1 = c1[1] * nx + c1[2] * ny + c1[3] * nz;
@@ -644,39 +645,36 @@ __device__ __forceinline__ int bc_insub(const BcPar &B, double nx, double ny, do
   const double dot = B.sx * nx + B.sy * ny + B.sz * nz;
   const double con1 = 0.5 / (h0inl * (dot * dot));
   const double con2 = 2 * con1 * g / (g - 1);
-  for (int icell = 1; icell <= 2; ++icell) {
-    double p, un, rc, rcun;
-    if (icell == 1) {
-      p = 2 * p1 - p2; un = 2 * un1 - un2; rc = 2 * rc1 - rc2; rcun = 2 * rcun1 - rcun2;
-    } else {
-      p = 3 * p1 - 2 * p2; un = 3 * un1 - 2 * un2; rc = 3 * rc1 - 2 * rc2; rcun = 3 * rcun1 - 2 * rcun2;
-    }
-    const double con3 = p - rcun;
-    double dun = 1.0;
-    int count = 0;
-    while (fabs(dun) > 1.0e-10) {
-      count = count + 1;
-      if (count == 10) { *err = 1; break; }
-      const double par = 1.0 - con1 * (un * un);
-      p = B.p0 * pow(par, g / (g - 1));
-      const double f = p - rc * un - con3;
-      const double fp = -con2 * un * p / par - rc;
-      dun = -f / fp;
-      un = un + dun;
-    }
-    p = +rc * un + con3;
-    const double modv = un / dot;
-    double *h = icell == 1 ? h1 : h2;
-    h[0] = g * p / ((g - 1) * (h0inl - 0.5 * (modv * modv)));
-    h[1] = modv * B.sx; h[2] = modv * B.sy; h[3] = modv * B.sz; h[4] = p;
-    if (B.npde > 5) { h[5] = B.tkefar; h[6] = B.omefar; }
+  double p, un, rc, rcun;
+  if (lay == 0) {
+    p = 2 * p1 - p2; un = 2 * un1 - un2; rc = 2 * rc1 - rc2; rcun = 2 * rcun1 - rcun2;
+  } else {
+    p = 3 * p1 - 2 * p2; un = 3 * un1 - 2 * un2; rc = 3 * rc1 - 2 * rc2; rcun = 3 * rcun1 - 2 * rcun2;
   }
-  return 3;
+  const double con3 = p - rcun;
+  double dun = 1.0;
+  int count = 0;
+  while (fabs(dun) > 1.0e-10) {
+    count = count + 1;
+    if (count == 10) { *err = 1; break; }
+    const double par = 1.0 - con1 * (un * un);
+    p = B.p0 * pow(par, g / (g - 1));
+    const double f = p - rc * un - con3;
+    const double fp = -con2 * un * p / par - rc;
+    dun = -f / fp;
+    un = un + dun;
+  }
+  p = +rc * un + con3;
+  const double modv = un / dot;
+  h[0] = g * p / ((g - 1) * (h0inl - 0.5 * (modv * modv)));
+  h[1] = modv * B.sx; h[2] = modv * B.sy; h[3] = modv * B.sz; h[4] = p;
+  if (NV > 5) { h[5] = B.tkefar; h[6] = B.omefar; }
 }
 // bc_outsub (src/bc.f90:1178-1455): static-pressure outlet
+template <int NV>
 __device__ __forceinline__ int bc_outsub(const BcPar &B, const double *c1, const double *c2, double *h1, double *h2) {
   const double g = B.g;
-  const int npde = B.npde;
+  constexpr int npde = NV;
   const bool kom = npde > 5;
   double qc1[7], qc2[7];
   const double tke1 = kom ? c1[5] : 0.0, tke2 = kom ? c2[5] : 0.0;
@@ -733,13 +731,14 @@ __device__ __forceinline__ int bc_outsub(const BcPar &B, const double *c1, const
 }
 // bc_far0 (src/bc.f90:124-483): Riemann-invariant far field, aircraft free
 // stream; s = face normal times sgnm
+template <int NV>
 __device__ __forceinline__ int bc_far0(const BcPar &B, double sx, double sy, double sz, const double *c1,
                                        double *h1, double *h2) {
   if (B.lomach) {
     // low-speed preconditioning: both layers frozen at the free stream (src/bc.f90:264-276, 409-414)
     for (int v = 0; v < 5; ++v) h1[v] = B.qfst[v];
-    if (B.npde > 5) { h1[5] = B.tkefar; h1[6] = B.omefar; }
-    for (int v = 0; v < B.npde; ++v) h2[v] = h1[v];
+    if (NV > 5) { h1[5] = B.tkefar; h1[6] = B.omefar; }
+    for (int v = 0; v < NV; ++v) h2[v] = h1[v];
     return 3;
   }
   const double g = B.g;
@@ -767,7 +766,7 @@ __device__ __forceinline__ int bc_far0(const BcPar &B, double sx, double sy, dou
       h1[4] = p;
     }
     mask = 3;
-    if (B.npde > 5) { h1[5] = B.tkefar; h1[6] = B.omefar; }
+    if (NV > 5) { h1[5] = B.tkefar; h1[6] = B.omefar; }
   } else if (qdotn > 0.0) {
     if (fabs(mach) >= 1.0) {
       for (int v = 0; v < 5; ++v) h1[v] = c1[v];
@@ -781,9 +780,9 @@ __device__ __forceinline__ int bc_far0(const BcPar &B, double sx, double sy, dou
       h1[4] = p;
     }
     mask = 3;
-    if (B.npde > 5) { h1[5] = c1[5]; h1[6] = c1[6]; }
+    if (NV > 5) { h1[5] = c1[5]; h1[6] = c1[6]; }
   }
-  for (int v = 0; v < B.npde; ++v) h2[v] = h1[v];
+  for (int v = 0; v < NV; ++v) h2[v] = h1[v];
   return mask;
 }
 
@@ -794,6 +793,7 @@ __device__ __forceinline__ int bc_far0(const BcPar &B, double sx, double sy, dou
 // preconditioning: boundary normal velocity and pressure from the mean of
 // the interior and free-stream states plus the acoustic jump, density from
 // the isentrope of the upwind side; s = face normal times sgnm
+template <int NV>
 __device__ __forceinline__ int bc_far1(const BcPar &B, double sx, double sy, double sz, const double *c1,
                                        double *h1, double *h2) {
   const double g = B.g;
@@ -828,7 +828,7 @@ __device__ __forceinline__ int bc_far1(const BcPar &B, double sx, double sy, dou
       h1[4] = pb;
     }
     mask = 3;
-    if (B.npde > 5) { h1[5] = B.tkefar; h1[6] = B.omefar; }
+    if (NV > 5) { h1[5] = B.tkefar; h1[6] = B.omefar; }
   } else if (unb > 0.0) {
     if (fabs(mach) >= 1.0) {
       for (int v = 0; v < 5; ++v) h1[v] = c1[v];
@@ -840,9 +840,9 @@ __device__ __forceinline__ int bc_far1(const BcPar &B, double sx, double sy, dou
       h1[4] = pb;
     }
     mask = 3;
-    if (B.npde > 5) { h1[5] = c1[5]; h1[6] = c1[6]; }
+    if (NV > 5) { h1[5] = c1[5]; h1[6] = c1[6]; }
   }
-  for (int v = 0; v < B.npde; ++v) h2[v] = h1[v];
+  for (int v = 0; v < NV; ++v) h2[v] = h1[v];
   return mask;
 }
 

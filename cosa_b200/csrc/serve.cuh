@@ -85,6 +85,7 @@ struct cosa_serve {
   std::deque<int64_t> queue;
   std::vector<int64_t> active;       // ids in the merged level's block order
   cosa_params *d_ps = nullptr;
+  BcPar *d_bcp = nullptr;  // their boundary values (k_bcpar)
   int ps_cap = 0;
   int *d_bad = nullptr;  // per-block positivity flags of the merged level
   int bad_cap = 0;
@@ -194,13 +195,17 @@ int serve_rebuild(cosa_serve *e) {
   // per-solve flow conditions on the scheme's parameters
   if (e->ps_cap < na) {
     if (e->d_ps) { cudaFree(e->d_ps); e->d_ps = nullptr; }
+    if (e->d_bcp) { cudaFree(e->d_bcp); e->d_bcp = nullptr; }
     CK(cudaMalloc(&e->d_ps, (size_t)na * sizeof(cosa_params)));
+    CK(cudaMalloc(&e->d_bcp, (size_t)na * COSA_MAX_LEVELS * sizeof(BcPar)));
     e->ps_cap = na;
   }
   std::vector<cosa_params> ps((size_t)na);
   for (int a = 0; a < na; ++a) ps[(size_t)a] = e->solves[(size_t)e->active[a]].flow;
   CK(cudaMemcpyAsync(e->d_ps, ps.data(), ps.size() * sizeof(cosa_params), cudaMemcpyHostToDevice, c->s));
-  c->d_halo_p = e->d_ps;
+  k_bcpar<<<(na * COSA_MAX_LEVELS + 63) / 64, 64, 0, c->s>>>(e->d_ps, na, e->d_bcp);
+  CK(cudaGetLastError());
+  c->d_halo_bcp = e->d_bcp;
   // residual-norm segments and their output rows
   if ((r = ensure_hist(c, na))) return r;
   // each solve's CFL number on its blocks (the flow conditions' cfl, else the scheme's)
@@ -301,9 +306,7 @@ int serve_retire(cosa_serve *e, const std::vector<int64_t> &done) {
   // face halos of the state in conservative form, as after smooth()
   if (!L.items.empty()) {
     const double *last_in = (c->p.nstage % 2 == 1) ? e->Q : e->T;
-    k_halo_p2c<<<grid_for((int64_t)L.items.size()), 256, 0, c->s>>>(L.d_blocks, L.d_items, (int)L.items.size(),
-                                                                   c->d_p, last_in, e->Q);
-    int r = after_launch(c);
+    const int r = launch_halo_p2c(c, L, last_in, e->Q);
     if (r) return r;
   }
   for (int64_t id : done) {
@@ -361,6 +364,7 @@ int cosa_serve_destroy(cosa_serve *e) {
   cudaSetDevice(c->device);
   cudaStreamSynchronize(c->s);
   if (e->d_ps) cudaFree(e->d_ps);
+  if (e->d_bcp) cudaFree(e->d_bcp);
   if (e->d_bad) cudaFree(e->d_bad);
   if (c->d_seg) cudaFree(c->d_seg);
   if (c->d_seg_ncell) cudaFree(c->d_seg_ncell);

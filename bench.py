@@ -6,8 +6,8 @@ segment lengths from {24, ..., 160}), M = 0.6, 4-stage RK, CFL 2, Roe + MUSCL
 (kappa = 1/3, smooth limiter), FP64 state.  A step is one RK cycle (4 stages)
 over all cells; the metric is Mcell-stage/s = cells * 4 * steps / time.
 
-Our arm times cosa_gpu_smooth (halo fill, line-marching face kernels and the
-cell pass of the face-split schedule, or the fused tile kernel, whichever the
+Our arm times cosa_gpu_smooth (halo fill and line-marching face kernels, the
+chain schedule or the store schedule with its cell pass, whichever the
 autotuner picks, replayed from a CUDA graph with the state resident in HBM)
 with CUDA events on the library's stream; the state (1.4 GB) is larger than
 the 126 MB L2, so no flush is needed between steps.  It also reports the
@@ -50,14 +50,10 @@ B_ALG_HB_MOVING = 330
 # (7 variables, the face inverse metrics, mut and the k-omega work arrays)
 # per snapshot
 B_ALG_KOM_HB_MOVING = 960
-# bytes the face-split schedule's face kernels (k_faces_line, i-face and
-# marching launches) move per cell: state reads 3 x 40 (once per family) +
-# face metrics 96 + face fluxes written 120
-B_FACES_OWN = 336
-# DRAM bytes (read + write) per cell of one stage's two k_faces_line
-# launches in an ncu capture of the 4.2 M-cell duct (k_faces_line<fp64>,
-# scaled by the cells of the launch)
-FACES_TRAFFIC_B_PER_CELL = 311.7
+# bytes the chain schedule's three launches move per cell-stage: state reads 3 x
+# 40 (once per family), face metrics 96, the running balance written and read
+# twice (160), base state 40, dt/V 8, new state 40
+CHAIN_B_PER_CELL = 464
 
 
 def _peaks():
@@ -270,7 +266,7 @@ def main():
     ap.add_argument("--no-hb", action="store_true", help="skip the pitching harmonic-balance leg")
     ap.add_argument("--hb-cycles", type=int, default=400, help="RK cycles of each harmonic-balance run")
     ap.add_argument("--schedule", type=int, default=0, choices=[0, 1, 2],
-                    help="0: autotune the stage schedule, 1: fused tile kernel, 2: face-split")
+                    help="0: autotune the stage schedule, 1: store, 2: chain")
     ap.add_argument("--precision", default="fp64", choices=["fp64", "mixed"],
                     help="precision of the main timed leg (profiling runs; the default line reports both)")
     ap.add_argument("--leg", default="all", choices=["all", "laminar", "kom"],
@@ -321,8 +317,8 @@ def main():
     ctx.bind_level(1, q=q, qold=qold, dtvol=dtvol, si=si, sj=sj, sk=sk, vol=vol)
     nstage = p.nstage
 
-    # ---- stage schedule: the autotuner times the fused tile kernel and the
-    # face-split schedule on this grid and keeps the faster (state restored)
+    # ---- stage schedule: the autotuner times the store and the chain
+    # schedule on this grid and keeps the faster (state restored)
     sched_fp64 = ctx.autotune(1, 3) if not args.schedule else (None, None, args.schedule - 1)
     if args.schedule:
         ctx.set_schedule(1, args.schedule - 1)
@@ -346,7 +342,7 @@ def main():
     # the dominant kernel is charged the whole stage's algorithmic bytes
     kms, kcnt = ctx.profile(1, 3)
     peak, peak_kind = _peaks()
-    split = sched_fp64[2] == 1
+    chain = sched_fp64[2] == 1
     alg_bytes = B_ALG_STAGE * ncells
     achieved = alg_bytes / (kms[1] / 1e3) / 1e9
     stage_gbs = B_ALG_STAGE * ncells * nstage * args.steps / (ms / 1e3) / 1e9
@@ -491,18 +487,16 @@ def main():
                        "parallelism": f"replicas x{ws}" if ws > 1 else "1 GPU"},
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak,
-                         "traffic": FACES_TRAFFIC_B_PER_CELL * ncells if split else None,
-                         "traffic_source": "ncu dram read+write of k_faces_line (both launches of a stage) per "
-                                           "cell on the 4.2 M-cell duct, x cells",
-                         "kernel": "k_faces_line<fp64> (i-face + marching launches)" if split
-                                   else "k_stage_tile<32,7,fp64>",
-                         "kernel_ms": kms[1], "halo_ms": kms[0], "cells_kernel_ms": kms[3] if split else None,
-                         "alg_bytes_per_cell": B_ALG_STAGE, "kernel_own_bytes_per_cell": B_FACES_OWN if split else None,
+                         "traffic": CHAIN_B_PER_CELL * ncells if chain else None,
+                         "traffic_source": "bytes the chain's three launches move per cell, counted from its accesses",
+                         "kernel": "k_line_chain<fp64> (i, j, k launches)" if chain else "k_line_store<fp64>",
+                         "kernel_ms": kms[1], "halo_ms": kms[0], "cells_kernel_ms": None if chain else kms[3],
+                         "alg_bytes_per_cell": B_ALG_STAGE, "kernel_own_bytes_per_cell": CHAIN_B_PER_CELL if chain else None,
                          "peak_kind": peak_kind, "stage_gbs_alg": stage_gbs, "stage_frac": stage_gbs / peak},
-            "schedule": {"fp64": {"tile_ms_per_step": sched_fp64[0], "split_ms_per_step": sched_fp64[1],
-                                  "chosen": ["tile", "split"][sched_fp64[2]]},
-                         "mixed": {"tile_ms_per_step": sched_mixed[0], "split_ms_per_step": sched_mixed[1],
-                                   "chosen": ["tile", "split"][sched_mixed[2]]}},
+            "schedule": {"fp64": {"store_ms_per_step": sched_fp64[0], "chain_ms_per_step": sched_fp64[1],
+                                  "chosen": ["store", "chain"][sched_fp64[2]]},
+                         "mixed": {"store_ms_per_step": sched_mixed[0], "chain_ms_per_step": sched_mixed[1],
+                                   "chosen": ["store", "chain"][sched_mixed[2]]}},
             "mixed": {"value": value_mixed, "ms_per_step": ms_mixed / args.steps,
                       "speedup_vs_fp64": value_mixed / value if value else None,
                       "main_kernel_ms": kms_m[1], "cells_kernel_ms": kms_m[3]},

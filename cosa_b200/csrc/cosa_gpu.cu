@@ -17,8 +17,8 @@
 #include "mg.cuh"
 #include "visc.cuh"
 #include "kom.cuh"
-#include "split.cuh"
 #include "faces.cuh"
+#include "split.cuh"
 #include "moving.cuh"
 #include "force.cuh"
 #include "unsteady.cuh"
@@ -34,8 +34,6 @@ inline bool blend(const cosa_params &p) { return p.kom_bsl || p.kom_sst; }
 // dual time: src_uns enters the residual unless rkimp without IRS on one
 // level, where update_b takes the physical-time term alone (src/cosa.f90:1910-1915)
 inline bool dual_src_in_res(const cosa_params &p) { return p.dualt && (!p.rkimp || p.irsop > 0 || p.nlevel > 1); }
-
-constexpr int kTI = 32, kTJ = 7;  // tile of the fused stage kernel (7 rows + the boundary-face warp = 256 threads)
 
 struct LevelState {
   int nb = 0;
@@ -53,12 +51,10 @@ struct LevelState {
   HaloItem *d_items = nullptr;
   uint8_t *d_strong = nullptr;
   StrongMap *d_smap = nullptr;
-  Tile *d_tiles = nullptr;
-  int ntiles = 0, kchunk = 0;
   bool bound = false;
   cosa_level_ptrs ptrs{};
   double *d_T = nullptr;      // second state buffer of the fused stages
-  double *d_part = nullptr;   // per-tile / per-CTA partial sums (8 doubles each)
+  double *d_part = nullptr;   // partial sums of the norms (8 doubles each)
   double *d_res = nullptr;    // residual of the IRS path (P3, zero halos)
   double *d_ores = nullptr;   // right-hand side copy of the cut-aware IRS
   double *d_irs_scr = nullptr;  // tridiagonal pivots, 2 doubles per P3 cell and snapshot
@@ -89,12 +85,21 @@ struct LevelState {
   // cut-offs (interior layout x S, the reference's p_cutoff_pgr / p_cutoff_vis)
   double *d_cut_pgr = nullptr, *d_cut_vis = nullptr;
   double *d_tbeta[3] = {nullptr, nullptr, nullptr};
-  // stage schedule: 0 = fused tile kernel, 1 = face-split (k_faces + k_cells),
-  // set by cosa_gpu_autotune
-  int schedule = 0;
-  double *d_cflux = nullptr;  // convective face fluxes of the split schedule (3 x F0)
-  FaceTask *d_ftasks = nullptr;  // warp tasks of k_faces_line: i-face tasks first
-  int nftasks = 0, nftasks1 = 0;
+  // stage schedule: 0 = store (face fluxes to memory, then k_cells), 1 =
+  // chain (the families' flux differences summed launch by launch); -1 until
+  // chosen by size (default_schedule), cosa_gpu_autotune or cosa_gpu_set_schedule
+  int schedule = -1;
+  // store: face fluxes of one group of blocks at a time (3 x F0 x 5 x S); the
+  // groups reuse the buffer, so its size is bounded (kStoreCells)
+  double *d_cflux = nullptr;
+  int64_t cflux_n0 = 0;            // F0 cells of its family stride
+  FaceTask *d_ftasks = nullptr;    // block after block
+  struct Group { int b0, nb; int64_t t0, nt; };
+  std::vector<Group> groups;
+  // chain: running flux balance (F0 x 5 x S) and the three families' tasks
+  double *d_div = nullptr;
+  FaceTask *d_ctasks = nullptr;
+  int64_t nctasks[3] = {0, 0, 0};
   // wall faces of each force surface (key: surface number), built on first use
   struct ForceList {
     ForceFace *d_faces = nullptr;
@@ -109,8 +114,7 @@ struct LevelState {
 
 struct ProfState {
   bool on = false;
-  // kinds: 0 halo fill, 1 main kernel (k_stage_tile, or k_faces of the split
-  // schedule), 2 the split schedule's k_cells
+  // kinds: 0 halo fill, 1 face kernels, 2 the store schedule's k_cells
   cudaEvent_t ev[3][2] = {{nullptr, nullptr}, {nullptr, nullptr}, {nullptr, nullptr}};  // [kind][start/stop]
   double ms[3] = {0, 0, 0};
   long long n[3] = {0, 0, 0};
@@ -135,8 +139,8 @@ struct cosa_ctx {
   double *d_hist = nullptr;
   BcPar *d_bcp = nullptr;                 // boundary values per flow-condition slot and level (k_bcpar)
   const BcPar *d_halo_bcp = nullptr;      // those of the served solves' slots, read by k_halo instead of d_bcp
-  // residual norms reduced per segment of tiles (one per served solve) when
-  // set: segment s = tiles [d_seg[2s], +d_seg[2s+1]) with seg_ncell[s] cells
+  // residual norms reduced per segment of k_cells' partial rows (one per served
+  // solve) when set: segment s = rows [d_seg[2s], +d_seg[2s+1]), seg_ncell[s] cells
   int nseg = 0;
   double *d_cfl_blk = nullptr;  // serving: CFL number of each block's solve
   int *d_seg = nullptr;
@@ -462,37 +466,18 @@ int build_level(cosa_ctx *c, LevelState &L, const cosa_level_desc &d, const int6
     L.ncutx = (int)cutx.size();
   }
 
-  // ---- tiles of the fused stage kernel
-  std::vector<Tile> tiles;
-  const int S = 2 * c->p.nharms + 1;
-  const int kc = 32;
-  L.kchunk = kc;
-  // snapshots innermost: the S tiles of one region run together, so the
-  // harmonic-balance coupling re-reads the other snapshots from L2
-  for (int b = 0; b < L.nb; ++b) {
-    const DevBlock &x = L.hb[b];
-    for (int k0 = 1; k0 <= x.km - 1; k0 += kc)
-      for (int j0 = 1; j0 <= x.jm - 1; j0 += kTJ)
-        for (int i0 = 1; i0 <= x.im - 1; i0 += kTI)
-          for (int n = 0; n < S; ++n)
-            tiles.push_back(Tile{b, n, i0, j0, k0, std::min(k0 + kc - 1, x.km - 1)});
-  }
-  L.ntiles = (int)tiles.size();
-
   int r = 0;
   if ((r = dalloc(c, &L.d_blocks, L.hb.size()))) return r;
   if ((r = dalloc(c, &L.d_bct, std::max<size_t>(L.bct.size(), 1)))) return r;
   if ((r = dalloc(c, &L.d_items, std::max<size_t>(L.items.size(), 1)))) return r;
   if ((r = dalloc(c, &L.d_strong, std::max<size_t>(flags.size(), 1)))) return r;
   if ((r = dalloc(c, &L.d_smap, smap.size()))) return r;
-  if ((r = dalloc(c, &L.d_tiles, std::max<size_t>(tiles.size(), 1)))) return r;
   CK(cudaMemcpy(L.d_blocks, L.hb.data(), L.hb.size() * sizeof(DevBlock), cudaMemcpyHostToDevice));
   if (!L.bct.empty()) CK(cudaMemcpy(L.d_bct, L.bct.data(), L.bct.size() * sizeof(int), cudaMemcpyHostToDevice));
   if (!L.items.empty())
     CK(cudaMemcpy(L.d_items, L.items.data(), L.items.size() * sizeof(HaloItem), cudaMemcpyHostToDevice));
   if (!flags.empty()) CK(cudaMemcpy(L.d_strong, flags.data(), flags.size(), cudaMemcpyHostToDevice));
   CK(cudaMemcpy(L.d_smap, smap.data(), smap.size() * sizeof(StrongMap), cudaMemcpyHostToDevice));
-  if (!tiles.empty()) CK(cudaMemcpy(L.d_tiles, tiles.data(), tiles.size() * sizeof(Tile), cudaMemcpyHostToDevice));
   if ((r = dalloc(c, &L.d_walls, std::max<size_t>(L.walls.size(), 1)))) return r;
   if ((r = dalloc(c, &L.d_cutx, std::max<size_t>(cutx.size(), 1)))) return r;
   if ((r = dalloc(c, &L.d_cutv, std::max<size_t>(cutv.size(), 1)))) return r;
@@ -520,15 +505,14 @@ int after_launch(cosa_ctx *c) {
 }
 
 // k_halo over `n` items from `items`.  Two threads per item while the launch
-// is smaller than kHaloSplit threads, which leaves most of the chip idle: one
-// cycle of the 64 x 32 x 2 channel (2.2 k items) 199 us split, 210 us not;
-// twenty of the 128 x 64 x 2 channel (5.6 k) 3.00 and 3.21 ms.  Above, the
-// doubled item reads and index work cost more than they hide.
+// is smaller than kHaloSplit threads (the chip holds 148 x 16 warps of it):
+// the 128 x 64 x 2 channel's cycle (4.3 k items) takes 151 us split, 165 us
+// not; the 30.7 M-cell duct's (1.6 M items) 22.8 ms split, 21.8 ms not.
 constexpr int64_t kHaloSplit = 75000;
 template <bool CONS>
 int launch_halo(cosa_ctx *c, LevelState &L, const HaloItem *items, int n, double *q, const double *si,
-                const double *sj, const double *sk, const double *dist, FaceVel fvel) {
-  const HaloPar h = make_halo_par(c->p);
+                const double *sj, const double *sk, const double *dist, FaceVel fvel, int test = CONS) {
+  const HaloPar h = make_halo_par(c->p, test);
   const bool split = (int64_t)n * h.S * 2 <= kHaloSplit;
   const dim3 g((unsigned)(((split ? 2 : 1) * (int64_t)n + 127) / 128), h.S);
   const BcPar *bcp = c->d_halo_bcp ? c->d_halo_bcp : c->d_bcp;
@@ -580,22 +564,6 @@ int64_t cnt_interior(const DevBlock &b, const cosa_params &p) {
 }
 int64_t cnt_all(const DevBlock &b, const cosa_params &p) {
   return (int64_t)(b.im + 3) * (b.jm + 3) * (b.km + 3) * (2 * p.nharms + 1) * p.npde;
-}
-
-// once per process; contexts driven from several host threads (the serving
-// engine's context lane) may reach it together
-int set_smem_attrs() {
-  static std::mutex mu;
-  static bool done = false;
-  std::lock_guard<std::mutex> lock(mu);
-  if (done) return COSA_OK;
-  const int smem = (int)stage_smem_bytes<kTI, kTJ>();
-  CK(cudaFuncSetAttribute(k_stage_tile<kTI, kTJ, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  CK(cudaFuncSetAttribute(k_stage_tile<kTI, kTJ, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  CK(cudaFuncSetAttribute(k_stage_tile<kTI, kTJ, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  CK(cudaFuncSetAttribute(k_stage_tile<kTI, kTJ, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  done = true;
-  return COSA_OK;
 }
 
 // the k-omega stage runs routine by routine (launch_rans_iteration); Wilcox,
@@ -821,23 +789,17 @@ void prof_stop(cosa_ctx *c, int k) {
 int launch_edges(cosa_ctx *c, LevelState &L, double *q, double *mut);
 
 // x extent of a (x, nblocks[, 3]) grid covering `n` items per block
-// viscous part of one stage on the halo-filled state qin: primitive copy,
+// viscous part of one stage on the primitive copy of the halo-filled state:
 // q_edges, [time step], face fluxes, wall faces, flux balance -> L.d_vres
-int launch_visc(cosa_ctx *c, LevelState &L, const double *qin, bool dt, double *bx, double *by, double *bz,
-                bool have_prim = false) {
+int launch_visc(cosa_ctx *c, LevelState &L, bool dt, double *bx, double *by, double *bz) {
   const cosa_params &p = c->p;
   const int S = 2 * p.nharms + 1;
-  int64_t m3 = 0, mc = 0, mf = 0;
+  int64_t mc = 0, mf = 0;
   for (const DevBlock &x : L.hb) {
-    m3 = std::max<int64_t>(m3, x.P3 * S);
     mc = std::max<int64_t>(mc, (int64_t)(x.im - 1) * (x.jm - 1) * (x.km - 1) * S);
     mf = std::max<int64_t>(mf, (int64_t)x.im * x.jm * x.km * S);
   }
   int r = 0;
-  if (!have_prim) {
-    k_prim<<<dim3(grid_x(m3, L.nb), L.nb), 256, 0, c->s>>>(L.d_blocks, c->d_p, qin, L.d_qprim);
-    if ((r = after_launch(c))) return r;
-  }
   if ((r = launch_edges(c, L, L.d_qprim, nullptr))) return r;
   const cosa_level_ptrs &P = L.ptrs;
   if (dt) {
@@ -860,107 +822,137 @@ int launch_visc(cosa_ctx *c, LevelState &L, const double *qin, bool dt, double *
   return after_launch(c);
 }
 
-constexpr int kCellsGX = 64;  // CTAs per block of k_cells (fixed: deterministic norm partials)
+constexpr int kRmsMidRows = 4096, kRmsMid = 148;  // partial rows summed by one CTA; rows left by k_rms_mid
+// CTAs per block of k_cells (its norm partials' rows): 64, and enough for two
+// per SM over all blocks; a served solve's must not depend on the others: 64
+constexpr int kCellsGX = 64;
+int cells_gx(const cosa_ctx *c, const LevelState &L) {
+  return c->nseg > 0 ? kCellsGX : std::max(kCellsGX, 2 * 148 / L.nb);
+}
 
-// split schedule after the halo fill (and, for viscous flows, the primitive
-// copy): face fluxes, cell epilogue, norm reduction.  qsrc is the stage input
-// (conv: interior cells converted on load) or the primitive copy.
-int launch_split_tail(cosa_ctx *c, int nl, LevelState &L, StageArgs &A, bool want_rms, const double *qsrc,
-                      bool conv) {
+// sum `rows` partial rows and write the norm row of the level
+int launch_rms(cosa_ctx *c, LevelState &L, int64_t rows) {
+  const int S = 2 * c->p.nharms + 1, npde = c->p.npde;
+  int64_t ncell = 0;
+  for (auto &b : L.hb) ncell += (int64_t)(b.im - 1) * (b.jm - 1) * (b.km - 1);
+  // resg_rms_hb averages over the snapshots as well (src/cosa.f90:4620-4626)
+  const double cnt = (double)ncell * (c->p.harbal ? S : 1);
+  const double *part = L.d_part;
+  int r = 0;
+  if (rows > kRmsMidRows) {
+    // the chain's rows: one warp each, too many for one CTA
+    k_rms_mid<<<kRmsMid, 256, 0, c->s>>>(part, (int)rows, npde, L.d_part + rows * 8);
+    if ((r = after_launch(c))) return r;
+    part = L.d_part + rows * 8;
+    rows = kRmsMid;
+  }
+  k_rms_final<<<1, 256, 0, c->s>>>(part, (int)rows, npde, cnt, c->d_hist, c->d_row, c->hist_cap);
+  return after_launch(c);
+}
+
+// the stage after the halo fill (and, for viscous flows, the primitive copy):
+// time step, faces, cells, norm.  qsrc: the stage input or its primitive
+// copy; conv: its interior is conservative
+int launch_faces(cosa_ctx *c, LevelState &L, StageArgs &A, bool want_rms, const double *qsrc, bool conv) {
   const cosa_params &p = c->p;
   const int S = 2 * p.nharms + 1;
-  const bool mixed = p.precision == COSA_PREC_MIXED;
+  // viscous flows take the FP64 faces in mixed precision too: their viscous
+  // terms are FP64 anyway, and the FP32 face is 5 % faster at best
+  const bool mixed = p.precision == COSA_PREC_MIXED && !p.viscous, lim1 = p.ilimf == 1;
   int r = 0;
   if (A.compute_dt) {
     int64_t mc = 0;
     for (const DevBlock &x : L.hb) mc = std::max<int64_t>(mc, (int64_t)(x.im - 1) * (x.jm - 1) * (x.km - 1) * S);
     const dim3 g(grid_x(mc, L.nb), L.nb);
     const CellVel cv = p.moving ? CellVel{{L.ptrs.xdot, L.ptrs.ydot, L.ptrs.zdot}} : CellVel{{nullptr, nullptr, nullptr}};
-    if (conv)
-      k_dt_euler<true><<<g, 256, 0, c->s>>>(L.d_blocks, c->d_p, qsrc, A.si, A.sj, A.sk, A.dtvol, A.bx, A.by, A.bz,
-                                            cv);
-    else
-      k_dt_euler<false><<<g, 256, 0, c->s>>>(L.d_blocks, c->d_p, qsrc, A.si, A.sj, A.sk, A.dtvol, A.bx, A.by, A.bz,
-                                             cv);
+    auto k = conv ? k_dt_euler<true> : k_dt_euler<false>;
+    k<<<g, 256, 0, c->s>>>(L.d_blocks, c->d_p, qsrc, A.si, A.sj, A.sk, A.dtvol, A.bx, A.by, A.bz, cv, A.cfl_blk);
     if ((r = after_launch(c))) return r;
   }
   A.part = want_rms ? L.d_part : nullptr;
-  // i-face tasks, then the marching j- and k-face tasks
-  auto faces = [&](int b0, int nb, cudaStream_t st) {
-    (void)b0; (void)nb;
-    const FaceTask *tk[2] = {L.d_ftasks, L.d_ftasks + L.nftasks1};
-    const LinePar lp = make_line_par(p);
-    const int nt[2] = {L.nftasks1, L.nftasks - L.nftasks1};
-#define COSA_FACES_LINE(M, CV, IF)                                                                               \
-  k_faces_line<M, CV, IF><<<(nt[IF ? 0 : 1] + 3) / 4, 128, 0, st>>>(                                           \
-      L.d_blocks, tk[IF ? 0 : 1], nt[IF ? 0 : 1], lp, qsrc, A.si, A.sj, A.sk, L.d_strong, L.d_smap,              \
-      A.first_order, L.n0, L.d_cflux, c->d_status)
-#define COSA_FACES_MOVING(M, CV, IF)                                                                            \
-  k_faces_line<M, CV, IF, true><<<(nt[IF ? 0 : 1] + 3) / 4, 128, 0, st>>>(                                     \
-      L.d_blocks, tk[IF ? 0 : 1], nt[IF ? 0 : 1], lp, qsrc, A.si, A.sj, A.sk, L.d_strong, L.d_smap,              \
-      A.first_order, L.n0, L.d_cflux, c->d_status, fvel)
-    const FaceVel fvel = face_vel_of(c, L);
-    // moving grids: the face speeds; viscous runs read the primitive copy (CV false)
-    if (p.moving && conv && mixed) { COSA_FACES_MOVING(true, true, true); COSA_FACES_MOVING(true, true, false); }
-    else if (p.moving && conv) { COSA_FACES_MOVING(false, true, true); COSA_FACES_MOVING(false, true, false); }
-    else if (p.moving && mixed) { COSA_FACES_MOVING(true, false, true); COSA_FACES_MOVING(true, false, false); }
-    else if (p.moving) { COSA_FACES_MOVING(false, false, true); COSA_FACES_MOVING(false, false, false); }
-    else if (mixed && conv) { COSA_FACES_LINE(true, true, true); COSA_FACES_LINE(true, true, false); }
-    else if (mixed) { COSA_FACES_LINE(true, false, true); COSA_FACES_LINE(true, false, false); }
-    else if (conv) { COSA_FACES_LINE(false, true, true); COSA_FACES_LINE(false, true, false); }
-    else { COSA_FACES_LINE(false, false, true); COSA_FACES_LINE(false, false, false); }
-#undef COSA_FACES_LINE
-#undef COSA_FACES_MOVING
-  };
-  auto cells = [&](int b0, int nb, cudaStream_t st) {
-    const dim3 gc(kCellsGX, nb);
-    if (want_rms) k_cells<true><<<gc, 256, 0, st>>>(L.d_blocks, c->d_p, A, L.d_cflux, L.n0, b0);
-    else k_cells<false><<<gc, 256, 0, st>>>(L.d_blocks, c->d_p, A, L.d_cflux, L.n0, b0);
-  };
-  // one launch per kernel over all blocks: per-block launches on two streams
-  // (cell pass of block b beside the faces of block b+1) measured slower, the
-  // small blocks underfill the GPU
-  if (c->prof.on) cudaEventRecord(c->prof.ev[1][0], c->s);
-  faces(0, L.nb, c->s);
-  if ((r = after_launch(c))) return r;
-  if (c->prof.on) {
-    prof_stop(c, 1);
-    cudaEventRecord(c->prof.ev[2][0], c->s);
+  const LinePar lp = make_line_par(p);
+  LineArgs la{L.d_blocks, nullptr, qsrc, {A.si, A.sj, A.sk}, L.d_strong, L.d_smap, A.first_order, 0, nullptr,
+              c->d_status, face_vel_of(c, L)};
+  if (L.schedule == 1 && !p.moving) {
+    la.cf = L.d_div;
+    if (c->prof.on) cudaEventRecord(c->prof.ev[1][0], c->s);
+    int64_t t0 = 0;
+    for (int fam = 1; fam <= 3; ++fam) {
+      la.tasks = L.d_ctasks + t0;
+      const unsigned n = (unsigned)L.nctasks[fam - 1];
+      t0 += n;
+#define COSA_CHAIN(M, CV, LM)                                                                                   \
+  (fam == 1 ? k_line_chain<1, M, CV, LM, false> : fam == 2 ? k_line_chain<2, M, CV, LM, false>                  \
+                                                : want_rms ? k_line_chain<3, M, CV, LM, true>                   \
+                                                           : k_line_chain<3, M, CV, LM, false>)
+      auto k = mixed ? (conv ? (lim1 ? COSA_CHAIN(true, true, true) : COSA_CHAIN(true, true, false))
+                             : (lim1 ? COSA_CHAIN(true, false, true) : COSA_CHAIN(true, false, false)))
+                     : (conv ? (lim1 ? COSA_CHAIN(false, true, true) : COSA_CHAIN(false, true, false))
+                             : (lim1 ? COSA_CHAIN(false, false, true) : COSA_CHAIN(false, false, false)));
+#undef COSA_CHAIN
+      k<<<n, 32, 0, c->s>>>(lp, la, A, c->d_p);
+      if ((r = after_launch(c))) return r;
+    }
+    if (c->prof.on) prof_stop(c, 1);
+    return want_rms ? launch_rms(c, L, L.nctasks[2]) : COSA_OK;
   }
-  cells(0, L.nb, c->s);
-  if ((r = after_launch(c))) return r;
-  if (c->prof.on) prof_stop(c, 2);
-  if (want_rms) {
-    int64_t ncell = 0;
-    for (auto &b : L.hb) ncell += (int64_t)(b.im - 1) * (b.jm - 1) * (b.km - 1);
-    const double cnt = (double)ncell * (p.harbal ? S : 1);
-    k_rms_final<<<1, 256, 0, c->s>>>(L.d_part, L.nb * kCellsGX, p.npde, cnt, c->d_hist, c->d_row, c->hist_cap);
+  for (const LevelState::Group &G : L.groups) {
+    // the buffer holds the group's fluxes from its first block on
+    la.cf = L.d_cflux - L.hb[G.b0].of0 * 5 * S;
+    la.n0 = L.cflux_n0;
+    la.tasks = L.d_ftasks + G.t0;
+    if (c->prof.on) cudaEventRecord(c->prof.ev[1][0], c->s);
+#define COSA_STORE(M, CV, MV) (lim1 ? k_line_store<M, CV, MV, true> : k_line_store<M, CV, MV, false>)
+    auto k = p.moving ? (mixed ? (conv ? COSA_STORE(true, true, true) : COSA_STORE(true, false, true))
+                               : (conv ? COSA_STORE(false, true, true) : COSA_STORE(false, false, true)))
+                      : (mixed ? (conv ? COSA_STORE(true, true, false) : COSA_STORE(true, false, false))
+                               : (conv ? COSA_STORE(false, true, false) : COSA_STORE(false, false, false)));
+#undef COSA_STORE
+    k<<<(unsigned)G.nt, 32, 0, c->s>>>(lp, la);
     if ((r = after_launch(c))) return r;
+    if (c->prof.on) {
+      prof_stop(c, 1);
+      cudaEventRecord(c->prof.ev[2][0], c->s);
+    }
+    const dim3 gc(cells_gx(c, L), G.nb);
+    if (want_rms) k_cells<true><<<gc, 256, 0, c->s>>>(L.d_blocks, c->d_p, A, la.cf, la.n0, G.b0);
+    else k_cells<false><<<gc, 256, 0, c->s>>>(L.d_blocks, c->d_p, A, la.cf, la.n0, G.b0);
+    if ((r = after_launch(c))) return r;
+    if (c->prof.on) prof_stop(c, 2);
   }
-  (void)nl;
-  return COSA_OK;
+  if (!want_rms) return COSA_OK;
+  if (c->nseg > 0) {
+    k_rms_seg<<<c->nseg, 256, 0, c->s>>>(L.d_part, c->d_seg, c->d_seg_ncell, p.npde, c->d_hist);
+    return after_launch(c);
+  }
+  return launch_rms(c, L, (int64_t)L.nb * cells_gx(c, L));
 }
 
-// one stage: halo fill + tile kernel (+ norm reduction)
+// one stage: halo fill, faces and cells (+ norm reduction).  prim_in: the
+// interior of qin is primitive (stored so by the stage before, prim_out)
 int launch_stage(cosa_ctx *c, int nl, LevelState &L, double *qin, double *qout, const double *qold,
                  double *qold_copy, int irk, int compute_dt, bool want_rms, int update, double *res_out,
-                 double *rhs = nullptr, int rhs_mode = 0) {
+                 double *rhs = nullptr, int rhs_mode = 0, bool prim_in = false, bool prim_out = false) {
   const cosa_params &p = c->p;
   const int S = 2 * p.nharms + 1;
   const cosa_level_ptrs &P = L.ptrs;
+  int r = 0;
+  if (L.schedule == 1 && !p.moving ? !L.d_div : L.groups.empty()) return COSA_ERR_ARG;
   if (!L.items.empty()) {
-        if (c->prof.on) cudaEventRecord(c->prof.ev[0][0], c->s);
-    int r = launch_halo<true>(c, L, L.d_items, (int)L.items.size(), qin, P.si, P.sj, P.sk, nullptr, face_vel_of(c, L));
+    if (c->prof.on) cudaEventRecord(c->prof.ev[0][0], c->s);
+    const int n = (int)L.items.size();
+    r = prim_in ? launch_halo<false>(c, L, L.d_items, n, qin, P.si, P.sj, P.sk, nullptr, face_vel_of(c, L), 1)
+                : launch_halo<true>(c, L, L.d_items, n, qin, P.si, P.sj, P.sk, nullptr, face_vel_of(c, L));
     if (r) return r;
     if (c->prof.on) prof_stop(c, 0);
   }
   StageArgs A{};
   A.qin = qin; A.qout = qout; A.qold = qold; A.qold_copy = qold_copy;
   A.dtvol = P.dtvol; A.si = P.si; A.sj = P.sj; A.sk = P.sk;
-  A.part = want_rms ? L.d_part : nullptr;
   A.rhs = rhs;
   A.rhs_mode = rhs ? rhs_mode : 0;
   A.res_out = res_out;
+  A.prim_out = prim_out;
   if (compute_dt && p.irsop >= 2) {
     A.bx = P.betaxi ? P.betaxi : L.d_beta[0];
     A.by = P.betaeta ? P.betaeta : L.d_beta[1];
@@ -976,58 +968,18 @@ int launch_stage(cosa_ctx *c, int nl, LevelState &L, double *qin, double *qout, 
   A.first_order = nl >= p.nl_crs;
   A.update = update;
   A.cfl_blk = c->d_cfl_blk;
-  const bool split =
-      L.schedule == 1 && c->nseg == 0 && L.d_cflux && (L.d_qprim || !p.viscous) && L.d_ftasks && !p.rkimp;
-  if (split && p.viscous) {
-    // primitive copy (with bprtest) shared by the viscous and convective faces
-    int64_t m3 = 0;
-    for (const DevBlock &x : L.hb) m3 = std::max<int64_t>(m3, x.P3 * S);
-    k_prim<<<dim3(grid_x(m3, L.nb), L.nb), 256, 0, c->s>>>(L.d_blocks, c->d_p, qin, L.d_qprim, c->d_status);
-    int r = after_launch(c);
-    if (r) return r;
-  }
-  if (p.viscous) {
-    // the viscous terms and, on stage 1, the viscous time step come first
-    if (!L.d_vm || !L.d_vres || !P.vol) return COSA_ERR_ARG;
-    int r = launch_visc(c, L, qin, compute_dt != 0, A.bx, A.by, A.bz, split);
-    if (r) return r;
-    A.vres = L.d_vres;
-    A.compute_dt = 0;
-    A.bx = A.by = A.bz = nullptr;
-  }
-  if (split) return launch_split_tail(c, nl, L, A, want_rms, p.viscous ? L.d_qprim : qin, !p.viscous);
-  if (p.moving) return COSA_ERR_UNSUPPORTED;  // the tile kernel has no face speeds
-  const size_t smem = stage_smem_bytes<kTI, kTJ>();
-  if (c->prof.on) cudaEventRecord(c->prof.ev[1][0], c->s);
-  // the residual-norm partials are a separate instantiation: their
-  // accumulators would otherwise hold registers in every launch
-  const int nthr = stage_threads<kTI, kTJ>();
-  const bool mixed = p.precision == COSA_PREC_MIXED;
-  if (mixed && want_rms)
-    k_stage_tile<kTI, kTJ, true, true><<<L.ntiles, nthr, smem, c->s>>>(L.d_blocks, L.d_tiles, c->d_p, A);
-  else if (mixed)
-    k_stage_tile<kTI, kTJ, true, false><<<L.ntiles, nthr, smem, c->s>>>(L.d_blocks, L.d_tiles, c->d_p, A);
-  else if (want_rms)
-    k_stage_tile<kTI, kTJ, false, true><<<L.ntiles, nthr, smem, c->s>>>(L.d_blocks, L.d_tiles, c->d_p, A);
-  else
-    k_stage_tile<kTI, kTJ, false, false><<<L.ntiles, nthr, smem, c->s>>>(L.d_blocks, L.d_tiles, c->d_p, A);
-  int r = after_launch(c);
-  if (r) return r;
-  if (c->prof.on) prof_stop(c, 1);
-  if (want_rms && c->nseg > 0) {
-    k_rms_seg<<<c->nseg, 256, 0, c->s>>>(L.d_part, c->d_seg, c->d_seg_ncell, p.npde, c->d_hist);
-    r = after_launch(c);
-    if (r) return r;
-  } else if (want_rms) {
-    int64_t ncell = 0;
-    for (auto &b : L.hb) ncell += (int64_t)(b.im - 1) * (b.jm - 1) * (b.km - 1);
-    // resg_rms_hb averages over the snapshots as well (src/cosa.f90:4620-4626)
-    const double cnt = (double)ncell * (p.harbal ? (2 * p.nharms + 1) : 1);
-    k_rms_final<<<1, 256, 0, c->s>>>(L.d_part, L.ntiles, p.npde, cnt, c->d_hist, c->d_row, c->hist_cap);
-    r = after_launch(c);
-    if (r) return r;
-  }
-  return COSA_OK;
+  if (!p.viscous) return launch_faces(c, L, A, want_rms, qin, !prim_in);
+  // primitive copy (with bprtest) shared by the viscous and convective faces;
+  // the viscous terms and, on stage 1, the viscous time step come first
+  if (!L.d_vm || !L.d_vres || !L.d_qprim || !P.vol) return COSA_ERR_ARG;
+  int64_t m3 = 0;
+  for (const DevBlock &x : L.hb) m3 = std::max<int64_t>(m3, x.P3 * S);
+  k_prim<<<dim3(grid_x(m3, L.nb), L.nb), 256, 0, c->s>>>(L.d_blocks, c->d_p, qin, L.d_qprim, c->d_status);
+  if ((r = after_launch(c)) || (r = launch_visc(c, L, compute_dt != 0, A.bx, A.by, A.bz))) return r;
+  A.vres = L.d_vres;
+  A.compute_dt = 0;
+  A.bx = A.by = A.bz = nullptr;
+  return launch_faces(c, L, A, want_rms, L.d_qprim, false);
 }
 
 // what one RK iteration of smooth() does besides the stages themselves
@@ -1202,8 +1154,17 @@ int launch_iteration(cosa_ctx *c, int nl, LevelState &L, const IterOpts &o) {
       continue;
     }
     if (p.irsop == 0) {
+      // Between the stages of an inviscid steady iteration the interior stays
+      // primitive: one conversion in the update instead of one per family and
+      // load (17.4 against 17.0 ms a cycle of the 30.7 M-cell duct).  The last
+      // stage reads conservative values again, so that the halos the call
+      // leaves behind are the BCs' on cells converted by division, as k_halo
+      // does it (16.8 ms without this).  Harmonic balance couples conservative
+      // snapshots, the viscous path makes its own copy.
+      const bool prim = !p.harbal && !p.viscous;
+      const bool prim_in = prim && irk > 1 && irk < p.nstage, prim_out = prim && irk < p.nstage - 1;
       int r = launch_stage(c, nl, L, qin, qout, qold, qcopy, irk, o.compute_dt && irk == 1, o.want_rms && irk == o.rms_stage, 1,
-                           nullptr, o.rhs, rmode);
+                           nullptr, o.rhs, rmode, prim_in, prim_out);
       if (r) return r;
     } else {
       // residual (no update) -> implicit smoothing -> update
@@ -1363,7 +1324,7 @@ int ensure_hist(cosa_ctx *c, int rows) {
 }  // namespace
 
 namespace {
-int ensure_split(cosa_ctx *c, LevelState &L);
+int ensure_faces(cosa_ctx *c, LevelState &L);
 }
 
 extern "C" {
@@ -1386,8 +1347,7 @@ int cosa_gpu_init(const cosa_params *p, int32_t nlevels, const cosa_level_desc *
   int r = 0;
   if ((r = cuda_ok(cudaStreamCreateWithFlags(&c->s, cudaStreamNonBlocking))) ||
       (r = dalloc(c, &c->d_p, 1)) || (r = dalloc(c, &c->d_bcp, COSA_MAX_LEVELS)) ||
-      (r = dalloc(c, &c->d_status, 1)) || (r = dalloc(c, &c->d_row, 1)) ||
-      (r = set_smem_attrs())) {
+      (r = dalloc(c, &c->d_status, 1)) || (r = dalloc(c, &c->d_row, 1))) {
     cosa_gpu_finalize(c);
     return r;
   }
@@ -1475,18 +1435,16 @@ int cosa_gpu_bind_level(cosa_ctx *c, int32_t nl, const cosa_level_ptrs *ptrs) {
   int r = 0;
   if (!L->d_T && (r = dalloc(c, &L->d_T, (size_t)L->n3 * c->p.npde * S))) return r;
   CK(cudaMemset(L->d_T, 0, (size_t)L->n3 * c->p.npde * S * sizeof(double)));
-  const int need = std::max(L->ntiles, 148 * 16);
+  const int need = 148 * 16;
   if (L->npart_cap < need) {
     if ((r = dalloc(c, &L->d_part, (size_t)need * 8))) return r;
     L->npart_cap = need;
   }
   drop_graphs(c);  // graphs hold the previous pointers
   L->bound = true;
+  if ((r = ensure_faces(c, *L))) return r;  // the stage's tasks and buffers with the other set-up
   if (c->p.moving) {
-    // moving grids run the face-split schedule (the tile kernel has no face speeds)
     if (!ptrs->fvi || !ptrs->fvj || !ptrs->fvk || !ptrs->xdot || !ptrs->ydot || !ptrs->zdot) return COSA_ERR_ARG;
-    if ((r = ensure_split(c, *L))) return r;
-    L->schedule = 1;
   }
   return COSA_OK;
 }
@@ -1720,6 +1678,7 @@ int cosa_gpu_smooth(cosa_ctx *c, int32_t nl, int32_t niter, int32_t mgit0, int32
     if (hist && (mgit == 1 || mgit % rms_every == 0 || mgit == last)) rows.push_back(it);
   }
   if ((r = ensure_hist(c, std::max<int>(1, (int)rows.size())))) return r;
+  if ((r = ensure_faces(c, *L))) return r;
   if ((c->p.irsop > 0 || c->p.rkimp || c->p.dualt) && (r = ensure_irs_scratch(c, *L))) return r;
   if ((c->p.rkimp || c->p.dualt) && L->npart_cap < L->nb * 64) {  // per-block norm partials (implicit HB, dual time)
     drop_graphs(c);
@@ -2298,6 +2257,7 @@ int cosa_gpu_smooth_level(cosa_ctx *c, int32_t nl, int32_t niter, int32_t from_f
   cudaSetDevice(c->device);
   const bool want = resrms && nl == 1 && niter > 0 && (mgit == 1 || mgit % rms_every == 0 || mgit == ncycle);
   if ((r = ensure_hist(c, 1))) return r;
+  if ((r = ensure_faces(c, *L))) return r;
   if ((c->p.irsop > 0 || c->p.rkimp || c->p.dualt) && (r = ensure_irs_scratch(c, *L))) return r;
   if ((c->p.rkimp || c->p.dualt) && L->npart_cap < L->nb * 64) {  // per-block norm partials (implicit HB, dual time)
     drop_graphs(c);
@@ -2332,6 +2292,7 @@ int cosa_gpu_rkuns(cosa_ctx *c, int32_t ntime, int32_t iprint, double *hist) {
   if (!P.q || !P.qold || !P.dtvol || !P.si || !P.sj || !P.sk || !P.vol) return COSA_ERR_ARG;
   if (p.viscous && !L->d_vm) return COSA_ERR_ARG;
   cudaSetDevice(c->device);
+  if ((r = ensure_faces(c, *L))) return r;
   std::vector<int> rows;
   for (int it = 0; it < ntime; ++it)
     if (hist && ((it + 1) % iprint == 0 || it + 1 == ntime)) rows.push_back(it);
@@ -2391,6 +2352,7 @@ int cosa_gpu_mg(cosa_ctx *c, int32_t mgit0, int32_t ncycles, int32_t ncycle, int
   if ((r = ensure_hist(c, std::max<int>(1, (int)rows.size())))) return r;
   for (int nl = 1; nl <= nlevel; ++nl) {
     LevelState &Lv = *level(c, nl);
+    if ((r = ensure_faces(c, Lv))) return r;
     if ((c->p.irsop > 0 || c->p.rkimp || c->p.dualt) && (r = ensure_irs_scratch(c, Lv))) return r;
     if ((c->p.rkimp || c->p.dualt) && Lv.npart_cap < Lv.nb * 64) {  // per-block norm partials (implicit HB, dual time)
       drop_graphs(c);
@@ -2448,6 +2410,7 @@ int cosa_gpu_profile(cosa_ctx *c, int32_t nl, int32_t niter, double ms[4], int64
   CK(cudaEventCreate(&t0));
   CK(cudaEventCreate(&t1));
   const int compute_dt = (1 / c->p.iupdt * c->p.iupdt == 1) ? 1 : 0;
+  if ((r = ensure_faces(c, *L))) return r;
   if (c->p.irsop > 0 && (r = ensure_irs_scratch(c, *L))) return r;
   cudaEventRecord(t0, c->s);
   IterOpts o;
@@ -3490,61 +3453,137 @@ int launch_rans_iteration(cosa_ctx *c, int nl, LevelState &L, const IterOpts &o)
 
 }  // namespace
 
-// ---- stage schedule autotuner -----------------------------------------------------------
+// ---- stage schedules: tasks, buffers, choice ---------------------------------------------
 namespace {
-// warp tasks of k_faces_line, block after block and snapshot after snapshot:
-// first every d = 1 task (rows in groups of kLineRows, 31 faces per warp),
-// then the d = 2, 3 tasks (lines of 32 lanes in segments of at most kLineSeg
-// faces, the two families of a block back to back)
-constexpr int kLineRows = 16, kLineSeg = 16;
-int build_face_tasks(cosa_ctx *c, LevelState &L) {
-  const int S = 2 * c->p.nharms + 1;
-  std::vector<FaceTask> t;
-  for (int b = 0; b < L.nb; ++b) {
-    const DevBlock &x = L.hb[b];
-    const int nj = x.jm - 1, nk = x.km - 1;
-    for (int n = 0; n < S; ++n)
-      for (int k = 1; k <= nk; ++k)
-        for (int j0 = 1; j0 <= nj; j0 += kLineRows)
-          for (int i0 = 1; i0 <= x.im; i0 += 31)
-            t.push_back(FaceTask{b, 1, n, i0, j0, k, 0, std::min(kLineRows, nj - j0 + 1)});
-  }
-  L.nftasks1 = (int)t.size();
-  for (int b = 0; b < L.nb; ++b) {
-    const DevBlock &x = L.hb[b];
-    const int ni = x.im - 1, nj = x.jm - 1, nk = x.km - 1;
-    for (int n = 0; n < S; ++n) {
-      for (int d = 2; d <= 3; ++d) {
-        const int mx = d == 2 ? x.jm : x.km, nt = d == 2 ? nk : nj;
-        const int nseg = (mx + kLineSeg - 1) / kLineSeg, len = (mx + nseg - 1) / nseg;
-        for (int tb = 1; tb <= nt; ++tb)
-          for (int f0 = 1; f0 <= mx; f0 += len)
-            for (int i0 = 1; i0 <= ni; i0 += 32)
-              t.push_back(FaceTask{b, d, n, i0, 0, tb, f0, std::min(len, mx - f0 + 1)});
-      }
-    }
-  }
+// Rows of an i task and faces (store) or cells (chain) of a marching task.
+// A segment of n costs n + 1 face evaluations and a start-up of three cells,
+// so long segments are cheaper, but a level needs enough warps: the length is
+// the largest power of two up to kLineMax that leaves kLineWaves full
+// waves of the chip's 148 x 12 resident warps.
+constexpr int kLineMax = 32, kLineWaves = 4;
+int line_len(int64_t cells) {
+  int len = kLineMax;
+  while (len > 1 && cells / (32 * (int64_t)len) < (int64_t)kLineWaves * 148 * 12) len /= 2;
+  return len;
+}
+int upload_tasks(cosa_ctx *c, const std::vector<FaceTask> &t, FaceTask **d) {
   if (t.size() >= (size_t)1 << 30) return COSA_ERR_UNSUPPORTED;
-  int r = dalloc(c, &L.d_ftasks, t.size());
+  int r = dalloc(c, d, t.size());
   if (r) return r;
-  CK(cudaMemcpy(L.d_ftasks, t.data(), t.size() * sizeof(FaceTask), cudaMemcpyHostToDevice));
-  L.nftasks = (int)t.size();
+  CK(cudaMemcpy(*d, t.data(), t.size() * sizeof(FaceTask), cudaMemcpyHostToDevice));
   return COSA_OK;
 }
-
-int ensure_split(cosa_ctx *c, LevelState &L) {
+// i tasks of a block: 31 faces (store) or 30 cells (chain) per warp
+void i_tasks(std::vector<FaceTask> &t, const DevBlock &x, int b, int S, int rows, int per, int imax) {
+  for (int n = 0; n < S; ++n)
+    for (int k = 1; k <= x.km - 1; ++k)
+      for (int j0 = 1; j0 <= x.jm - 1; j0 += rows)
+        for (int i0 = 1; i0 <= imax; i0 += per)
+          t.push_back(FaceTask{b, 1, n, i0, j0, k, 0, std::min(rows, x.jm - j0)});
+}
+// j or k tasks of a block: `items` faces (store) or cells (chain) cut into
+// equal segments of at most len; `extra` more faces close a chain's segment
+void m_tasks(std::vector<FaceTask> &t, const DevBlock &x, int b, int S, int d, int items, int len, int extra) {
+  const int nseg = (items + len - 1) / len, l = (items + nseg - 1) / nseg, nt = d == 2 ? x.km - 1 : x.jm - 1;
+  for (int n = 0; n < S; ++n)
+    for (int tb = 1; tb <= nt; ++tb)
+      for (int f0 = 1; f0 <= items; f0 += l)
+        for (int i0 = 1; i0 <= x.im - 1; i0 += 32)
+          t.push_back(FaceTask{b, d, n, i0, 0, tb, f0, std::min(l, items - f0 + 1) + extra});
+}
+int64_t level_cells(const cosa_ctx *c, const LevelState &L) {
+  int64_t n = 0;
+  for (const DevBlock &x : L.hb) n += (int64_t)(x.im - 1) * (x.jm - 1) * (x.km - 1);
+  return n * (2 * c->p.nharms + 1);
+}
+int want_parts(cosa_ctx *c, LevelState &L, int64_t rows) {
+  if (L.npart_cap >= rows) return COSA_OK;
+  drop_graphs(c);
+  const int r = dalloc(c, &L.d_part, (size_t)rows * 8);
+  if (!r) L.npart_cap = (int)rows;
+  return r;
+}
+// the fluxes of one store group: at most this many F0 cells x snapshots (or
+// the largest block), 480 MB
+constexpr int64_t kStoreCells = 4000000;
+int ensure_store(cosa_ctx *c, LevelState &L) {
+  const int S = 2 * c->p.nharms + 1;
+  if (L.groups.empty()) {
+    const int len = std::min(16, line_len(level_cells(c, L)));
+    std::vector<FaceTask> t;
+    int64_t cap = 0, n0 = 0;
+    for (int b = 0; b < L.nb; ++b) {
+      const DevBlock &x = L.hb[b];
+      const int64_t f = (int64_t)x.im * x.jm * x.km;
+      if (b == 0 || (n0 + f) * S > kStoreCells) {
+        L.groups.push_back({b, 0, (int64_t)t.size(), 0});
+        n0 = 0;
+      }
+      i_tasks(t, x, b, S, len, 31, x.im);
+      m_tasks(t, x, b, S, 2, x.jm, len, 0);
+      m_tasks(t, x, b, S, 3, x.km, len, 0);
+      n0 += f;
+      cap = std::max(cap, n0);
+      LevelState::Group &G = L.groups.back();
+      G.nb = b - G.b0 + 1;
+      G.nt = (int64_t)t.size() - G.t0;
+    }
+    int r = upload_tasks(c, t, &L.d_ftasks);
+    if (!r) r = dalloc(c, &L.d_cflux, (size_t)3 * cap * 5 * S);
+    if (r) { L.groups.clear(); return r; }
+    L.cflux_n0 = cap;
+  }
+  // k_rms_mid's rows follow when the blocks have many
+  return want_parts(c, L, (int64_t)L.nb * cells_gx(c, L) + kRmsMid);
+}
+int ensure_chain(cosa_ctx *c, LevelState &L) {
+  const int S = 2 * c->p.nharms + 1;
+  if (!L.d_div) {
+    const int len = line_len(level_cells(c, L));
+    std::vector<FaceTask> t;
+    for (int fam = 1; fam <= 3; ++fam) {
+      const size_t before = t.size();
+      for (int b = 0; b < L.nb; ++b) {
+        const DevBlock &x = L.hb[b];
+        if (fam == 1) i_tasks(t, x, b, S, len, 30, x.im - 1);
+        else m_tasks(t, x, b, S, fam, (fam == 2 ? x.jm : x.km) - 1, len, 1);
+      }
+      L.nctasks[fam - 1] = (int64_t)(t.size() - before);
+    }
+    int r = upload_tasks(c, t, &L.d_ctasks);
+    if (!r) r = dalloc(c, &L.d_div, (size_t)L.n0 * 5 * S);
+    if (r) return r;
+  }
+  return want_parts(c, L, L.nctasks[2] + kRmsMid);
+}
+// The schedule by size (cells x snapshots).  Store has one face launch of all
+// families and as many warps as faces allow; chain moves fewer bytes (464
+// against 530 B a cell-stage) but runs the families one after another.  One
+// cycle, store / chain in us: ducts of 33 k cells 85 / 110, 131 k
+// 148 / 179, 295 k 298 / 333, 590 k (one block) 509 / 495, (eight) 601 / 608,
+// 655 k 594 / 596; two-cell-thick channels of 131 k 175 / 186, 262 k 315 / 319,
+// 1.05 M 925 / 829; 30.7 M cells (24 blocks): store's fluxes no longer fit L2.
+constexpr int64_t kChainCells = 600000;
+int default_schedule(const cosa_ctx *c, const LevelState &L) {
+  return c->nseg == 0 && !c->p.moving && level_cells(c, L) >= kChainCells ? 1 : 0;
+}
+// what launch_stage needs of the level's schedule, chosen by size at first;
+// when the chain's running balance does not fit the device, store, whose
+// buffer is bounded, takes its place
+int ensure_faces(cosa_ctx *c, LevelState &L) {
+  if (routine_stage(c->p)) return COSA_OK;
   const int S = 2 * c->p.nharms + 1;
   int r = 0;
-  if (!L.d_ftasks && (r = build_face_tasks(c, L))) return r;
+  if (L.schedule < 0) L.schedule = default_schedule(c, L);
   // the primitive copy only for viscous flows (the viscous set-up allocates it)
   if (c->p.viscous && !L.d_qprim && (r = dalloc(c, &L.d_qprim, (size_t)L.n3 * 5 * S))) return r;
-  if (!L.d_cflux && (r = dalloc(c, &L.d_cflux, (size_t)3 * L.n0 * 5 * S))) return r;
-  if (L.npart_cap < L.nb * kCellsGX) {
+  if (L.schedule == 1 && !c->p.moving) {
+    if (!(r = ensure_chain(c, L))) return r;
+    cudaGetLastError();
+    L.schedule = 0;
     drop_graphs(c);
-    if ((r = dalloc(c, &L.d_part, (size_t)L.nb * kCellsGX * 8))) return r;
-    L.npart_cap = L.nb * kCellsGX;
   }
-  return COSA_OK;
+  return ensure_store(c, L);
 }
 }  // namespace
 
@@ -3560,7 +3599,6 @@ extern "C" int cosa_gpu_autotune(cosa_ctx *c, int32_t nl, int32_t niter, double 
     return COSA_OK;
   }
   cudaSetDevice(c->device);
-  if ((r = ensure_split(c, *L))) return r;
   const int S = 2 * c->p.nharms + 1;
   const size_t nq = (size_t)L->n3 * c->p.npde * S;
   double *save = nullptr;
@@ -3593,17 +3631,13 @@ extern "C" int cosa_gpu_autotune(cosa_ctx *c, int32_t nl, int32_t niter, double 
   return r ? r : cuda_ok(cudaGetLastError());
 }
 
-/* force a schedule (0 tile, 1 split) without timing */
+/* force a schedule (0 store, 1 chain) without timing */
 extern "C" int cosa_gpu_set_schedule(cosa_ctx *c, int32_t nl, int32_t schedule) {
   LevelState *L = level(c, nl);
   if (!L || schedule < 0 || schedule > 1) return COSA_ERR_ARG;
-  if (schedule == 1) {
-    int r = ensure_split(c, *L);
-    if (r) return r;
-  }
   L->schedule = schedule;
   drop_graphs(c);
-  return COSA_OK;
+  return L->bound ? ensure_faces(c, *L) : COSA_OK;
 }
 
 #include "serve.cuh"

@@ -1,29 +1,49 @@
-// Line-marching convective face kernel of the face-split stage schedule.
+// Line-marching convective kernels of the explicit RK stage.
 //
 // Every face of a line (fixed transverse cell, family d) needs the limited
 // MUSCL states of its two cells; the limiter of cell c depends only on its
 // two slopes dq(c) = q(c) - q(c-1) and dq(c+1), and gives both the state of
-// c on its lower face (dqp(c), for face c) and on its upper face (dqm(c+1),
-// for face c+1) from one sensor (limit_i/j/k, src/flux.f90:3472-3888, where
-// the two sensors of a cell are the same expression).  So a thread that
-// walks a line evaluates each cell's sensor once instead of twice and loads
-// each cell once instead of four times:
+// c on its lower face (for face c) and on its upper face (for face c+1) from
+// one sensor (limit_i/j/k, src/flux.f90:3472-3888, where the two sensors of a
+// cell are the same expression).  So a thread that walks a line evaluates each
+// cell's sensor once instead of twice and loads each cell once instead of four
+// times:
 //
 //   d = 2, 3   lanes along i (coalesced), each thread marches along j or k
-//              over a segment of faces, carrying two cells, one slope and
-//              the pending dqm;
+//              over a segment of faces, carrying a cell, a slope and the
+//              pending left state;
 //   d = 1      lanes along i as well: lane l owns cell c = i0 - 1 + l, gets
-//              the neighbouring cells through L1, and passes its dqm(c+1) to
-//              lane l + 1 with a warp shuffle; lanes 1..31 compute faces
+//              the neighbouring cells through L1, and passes its upper state
+//              to lane l + 1 with a warp shuffle; lanes 1..31 compute faces
 //              i0 .. i0 + 30.
 //
-// The stage input holds conservative interior cells and primitive halo
-// cells (k_halo); interior cells are converted on load (c2p5_nr) with the
-// positivity test of bprtest, so no primitive copy of the state is made.
-// The viscous path, which needs that copy anyway, reads it instead.
+// One warp is one CTA, so that everything a task holds (block, bases, strides,
+// loop bounds) is uniform over the CTA and the strong-boundary cases are
+// uniform branches off the loop instead of selects in it.
 //
-// FP64: the same device functions and operation order as k_faces (bit for
-// bit).  MIXED: slopes are FP64 differences rounded to FP32, the limiter
+// Two schedules use these loops (picked by size, launch_split_tail):
+//   store   one launch over all faces, fluxes to memory, then k_cells: the
+//           most parallel form, for grids that leave the chip idle;
+//   chain   i, then j, then k launches, each adding its family's flux
+//           difference to the running sum D of the cell (the reference's
+//           bresid order), the last one finishing the stage: D is 40 bytes a
+//           cell where the three families' fluxes are 120 written and read.
+// The face and cell arithmetic is shared, so both give the same bits.
+//
+// The stage input's halo cells are primitive (k_halo); its interior is
+// conservative and converted on load (CONV, c2p5_nr with the positivity test
+// of bprtest), or primitive: in the viscous path's copy, and between the
+// stages of an iteration (launch_iteration).
+//
+// What bounds them: issue and FP64 latency.  A face takes about 230 FP64
+// operations (limiter and states 17 a variable, Roe flux 129); the three
+// families of the 30.7 M-cell duct take 3.9 ms a stage, 2.5 ms of it at the
+// FP64 pipe's rate, and move 464 B/cell (2.2 ms at 6.65 TB/s).  Before: 755 to
+// 840 warp instructions a face with selects for the strong boundaries,
+// 64-bit addresses per access and register-staged prefetch, fluxes through
+// memory (530 B/cell with the cell pass): 5.3 ms.
+//
+// MIXED: slopes are FP64 differences rounded to FP32, the limiter
 // and the whole Roe flux run in FP32, and the flux enters FP64 as
 //     F = ds * ( g(q_L cell) + [ (Dg_L + Dg_R)/2 - |A| dq / 2 ] )
 // with g(q) = f(q).n the unit-normal flux of the left cell's FP64 state and
@@ -31,13 +51,13 @@
 // X, expanded so that every FP32 term is proportional to the differences:
 // the FP32 rounding error scales with the local jumps, not with the state.
 #pragma once
-#include "split.cuh"
+#include "fused.cuh"
 
 // one warp's share of a face family: d = 1: rows j = ta .. ta + nf - 1 at
 // k = tb, lanes cells i0 - 1 + lane; d = 2: lanes i = i0 + lane, k = tb, faces
 // j = f0 .. f0 + nf - 1; d = 3: lanes i = i0 + lane, j = tb, faces k = f0 ..
 // f0 + nf - 1
-struct FaceTask {
+struct __align__(16) FaceTask {
   int blk, d, n, i0, ta, tb, f0, nf;
 };
 
@@ -217,13 +237,8 @@ __device__ __forceinline__ void face_flux_mixed(const PhysPar &P, float g, float
   }
 }
 
-// per-slope doubling on strong-boundary faces (muscl_b*, src/flux.f90:1318-1406)
-__device__ __forceinline__ bool dbl_at(int s, int mx, bool slo, bool shi) {
-  return (s == 1 && slo) || (s == mx && shi);
-}
-
-// scheme constants of k_faces_line, passed by value: kernel parameters sit in
-// the constant bank, where FP64 instructions read them as operands instead
+// scheme constants of the line kernels, passed by value: kernel parameters sit
+// in the constant bank, where FP64 instructions read them as operands instead
 // of holding them in registers across the marching loop
 struct LinePar {
   PhysPar ph;
@@ -237,310 +252,494 @@ inline LinePar make_line_par(const cosa_params &P) {
   o.S = 2 * P.nharms + 1; o.S2 = 2 * P.nharms * P.hbmove + 1; o.hbmove = P.hbmove;
   return o;
 }
+// arrays of a line launch
+struct LineArgs {
+  const DevBlock *blocks;
+  const FaceTask *tasks;
+  const double *q;               // stage input or its primitive copy
+  const double *s[3];            // face metrics of the three families
+  const uint8_t *strong;
+  const StrongMap *smap;
+  int first_order;
+  int64_t n0;
+  double *cf;                    // store: fluxes of the three families; chain: D (F0 layout)
+  int *status;
+  FaceVel fv;
+};
 
-// state of cell c of a face line: conservative interior cells are converted
-// (with bprtest's positivity test), halo cells are primitive already
-template <bool CONV>
-__device__ __forceinline__ void conv_cell(bool interior, const LinePar &LP, int &st, double *v) {
-  if (CONV && interior) {
-    c2p5_nr(LP.gamma, v);
-    if (v[4] <= LP.qmin_p) st |= COSA_ERR_NEG_P;
-    else if (v[0] <= LP.qmin_rho) st |= COSA_ERR_NEG_RHO;
-  }
+// interior cells of a conservative stage input: to primitive variables, with
+// bprtest's positivity test
+__device__ __forceinline__ void to_prim(double gamma, double qmin_rho, double qmin_p, int &st, double *v) {
+  c2p5_nr(gamma, v);
+  if (v[4] <= qmin_p) st |= COSA_ERR_NEG_P;
+  else if (v[0] <= qmin_rho) st |= COSA_ERR_NEG_RHO;
 }
-__device__ __forceinline__ void raw_cell(const double *__restrict__ p, int64_t P3, double *v) {
-#pragma unroll
-  for (int m = 0; m < 5; ++m) v[m] = __ldg(p + m * P3);
+// asynchronous copies global -> shared memory, 8 and 16 bytes a lane
+__device__ __forceinline__ void cp8(double *dst, const double *src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src));
 }
-template <bool CONV>
-__device__ __forceinline__ void load_cell(const double *__restrict__ p, int64_t P3, bool interior, const LinePar &LP,
-                                          int &st, double *v) {
-  raw_cell(p, P3, v);
-  conv_cell<CONV>(interior, LP, st, v);
+__device__ __forceinline__ void cp16(double2 *dst, const double *src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src));
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;"); }
+template <int N>
+__device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+// staging of one step: what it needs comes one step ahead without holding
+// registers.  I: cells (with the two beyond the warp's) and metrics; M: the
+// next cell, the face's metrics and, in the chain, the running balance D, the
+// base state and the time step of the cell that the face closes
+struct StageI {
+  double q[2][5][34];
+  double2 met[2][2][32];
+};
+template <int OUT>
+struct StageM {
+  double q[2][5][32];
+  double2 met[2][2][32];
+  double D[2][OUT >= 1 ? 5 : 1][32];
+  double base[2][OUT == 2 ? 6 : 1][32];
+};
+// normal speed of a face from its velocity: sijk(5)*kx + sijk(6)*ky +
+// sijk(7)*kz, roflux_b's order (src/flux.f90:110-113)
+__device__ __forceinline__ double face_ubn(const double *__restrict__ v, double kx, double ky, double kz) {
+  return __fma_rn(__ldg(v + 2), kz, __fma_rn(__ldg(v + 1), ky, __dmul_rn(__ldg(v), kx)));
 }
 
-// the two FP64 face states of a face from its cells L, R and the offsets
-// dqm (of L) and dqp (of R); first order takes the cells; the strong-boundary
-// overrides (rare: the first and last face of a line) take one cell for both
-__device__ __forceinline__ void face_states64(bool fo, bool ovr_lo, bool ovr_hi, const double *qL, const double *qR,
-                                              const double *dqm, const double *dqp, double *ql, double *qr) {
+// what a cell's flux balance r goes through after the three families: viscous
+// balance, harmonic-balance source, norms, forcing, update (k_cells and the
+// last launch of the chain).  q0: the cell's base state (read when A.update)
+template <bool RMS>
+__device__ __forceinline__ void finish_cell(const StageArgs &A, const cosa_params &P, const DevBlock &b, int S, int n,
+                                            int64_t cell, double vol_omega, double dt, double *r, const double *q0,
+                                            double gamma, double qmin_rho, double qmin_p, double *acc, int &st) {
+  double qw[5];
 #pragma unroll
   for (int m = 0; m < 5; ++m) {
-    if (fo) { qr[m] = qR[m]; ql[m] = qL[m]; }
-    else { qr[m] = __dadd_rn(qR[m], dqp[m]); ql[m] = __dadd_rn(qL[m], dqm[m]); }
-  }
-  if (ovr_lo | ovr_hi) {
-#pragma unroll
-    for (int m = 0; m < 5; ++m) {
-      const double v = ovr_lo ? qL[m] : qR[m];
-      qr[m] = v; ql[m] = v;
+    const int64_t o = p3_var(b, 5, S, m + 1, n) + cell;
+    if (A.vres) r[m] = r[m] + A.vres[o];
+    if (A.vol) {
+      // src_bhb (src/src.f90:556-613)
+      double qhb = 0.0;
+      for (int nj2 = 0; nj2 < S; ++nj2)
+        qhb = __fma_rn(__dmul_rn(vol_omega, P.dhb[n * S + nj2]), A.qin[p3_var(b, 5, S, m + 1, nj2) + cell], qhb);
+      r[m] = r[m] + qhb;
     }
-  }
-}
-// the mixed path's offsets of the face states from their cells (dqL from
-// cell L, dqR from cell R) with the overrides; dlr = q_R - q_L
-__device__ __forceinline__ void face_offsets32(bool ovr_lo, bool ovr_hi, const float *dlr, const float *dqm,
-                                               const float *dqp, float *dqL, float *dqR) {
-#pragma unroll
-  for (int m = 0; m < 5; ++m) { dqL[m] = dqm[m]; dqR[m] = dqp[m]; }
-  if (ovr_lo | ovr_hi) {
-#pragma unroll
-    for (int m = 0; m < 5; ++m) {
-      if (ovr_lo) { dqL[m] = 0.0f; dqR[m] = -dlr[m]; }  // both states = cell L
-      else { dqL[m] = dlr[m]; dqR[m] = 0.0f; }          // both states = cell R
-    }
-  }
-}
-__device__ __forceinline__ void ld_met(const double *__restrict__ sp, double *m4) {
-  const double2 a = __ldg(reinterpret_cast<const double2 *>(sp));
-  const double2 c = __ldg(reinterpret_cast<const double2 *>(sp + 2));
-  m4[0] = a.x; m4[1] = a.y; m4[2] = c.x; m4[3] = c.y;
-}
-
-// Grid: one CTA of 128 threads per 4 tasks (warp w takes task 4 blockIdx.x + w).
-// q: the stage input (CONV) or its primitive copy; face fluxes of family d
-// into cf + (d-1) n0 5 S (F0 layout per family).  IFAM: the tasks are i-face
-// tasks (d = 1), else marching tasks (d = 2, 3); separate instantiations keep
-// the register allocation of each to its own code.  The next row's (IFAM) or
-// the next step's cells and face metrics are loaded one step ahead, and all
-// addresses advance by constant strides.
-// normal speed of face e (its metric record index p2_idx / 4) of family d:
-// sijk(5)*kx + sijk(6)*ky + sijk(7)*kz, roflux_b's order (src/flux.f90:110-113)
-__device__ __forceinline__ double face_ubn(const double *__restrict__ fv, int64_t rec, double kx, double ky,
-                                           double kz) {
-  const double *v = fv + rec * 3;
-  return __ldg(v) * kx + __ldg(v + 1) * ky + __ldg(v + 2) * kz;
-}
-
-#ifndef COSA_LINE_MINB64
-#define COSA_LINE_MINB64 3  // resident CTAs per SM the FP64 instantiations are compiled for
-#endif
-template <bool MIXED, bool CONV, bool IFAM, bool MV = false>
-__global__ void __launch_bounds__(128, MIXED ? 4 : COSA_LINE_MINB64)
-k_faces_line(const DevBlock *__restrict__ blocks, const FaceTask *__restrict__ tasks, int ntasks,
-             const LinePar LP, const double *__restrict__ q, const double *__restrict__ si,
-             const double *__restrict__ sj, const double *__restrict__ sk, const uint8_t *__restrict__ strong,
-             const StrongMap *__restrict__ smap, int first_order, int64_t n0, double *__restrict__ cf,
-             int *status, FaceVel FV = FaceVel{{nullptr, nullptr, nullptr}}) {
-  const int wid = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (wid >= ntasks) return;
-  const FaceTask T = tasks[wid];
-  const DevBlock b = blocks[T.blk];
-  const PhysPar &ph = LP.ph;
-  const float g32 = (float)ph.g, gg32 = (float)ph.g_gm1, eps32 = (float)ph.epslimf, rk32 = (float)ph.rkap;
-  const int S = LP.S, S2 = LP.S2;
-  const int d = T.d, n = T.n, nh = n * LP.hbmove;
-  const double *s = d == 1 ? si : (d == 2 ? sj : sk);
-  double *F0 = cf + (int64_t)(d - 1) * n0 * 5 * S;
-  const StrongMap sm = smap[T.blk];
-  const int mx = d == 1 ? b.im : (d == 2 ? b.jm : b.km);
-  const double *qv = q + p3_var(b, 5, S, 1, n);
-  const int64_t fv = (int64_t)b.im * b.jm * b.km;  // variable stride of the F0 face arrays
-  const bool fo = first_order != 0;
-  int st = 0;
-
-  if (IFAM) {
-    // lane l: cell c = i0 - 1 + l of rows j = ta .., k = tb; faces c for lanes
-    // 1..31.  Lanes past the line (c > mx) read cell mx's stencil and store nothing.
-    const int k = T.tb, c = T.i0 - 1 + lane, cl = min(c, mx);
-    const bool face = lane >= 1 && c >= 1 && c <= mx;
-    const bool in_m = cl - 1 >= 1 && cl - 1 <= mx - 1, in_0 = cl >= 1 && cl <= mx - 1,
-               in_p = cl + 1 >= 1 && cl + 1 <= mx - 1;
-    const double *pc = qv + p3_cell(b, cl, T.ta, k);
-    const double *sp = s + p2_idx(b, S2, 1, cl, T.ta, k, nh);
-    const double *vp = MV ? FV.f[0] + p2_idx(b, S2, 1, cl, T.ta, k, nh) / 4 * 3 : nullptr;
-    double *Fp = F0 + f0_idx(b, 5, S, max(cl, 1), T.ta, k, 1, n);  // lane 0 stores nothing
-    const int64_t qrow = b.I3, mrow = (int64_t)(b.im + 2) * 4, frow = b.im;
-    double A[3][5], met[4];
-    raw_cell(pc - 1, b.P3, A[0]); raw_cell(pc, b.P3, A[1]); raw_cell(pc + 1, b.P3, A[2]);
-    ld_met(sp, met);
-    for (int row = 0; row < T.nf; ++row) {
-      const int j = T.ta + row;
-      conv_cell<CONV>(in_m, LP, st, A[0]);
-      conv_cell<CONV>(in_0, LP, st, A[1]);
-      conv_cell<CONV>(in_p, LP, st, A[2]);
-      // the next row (the last row reloads itself: in bounds, unused)
-      const int64_t nx = row + 1 < T.nf ? 1 : 0;
-      double B[3][5], metn[4];
-      raw_cell(pc + nx * qrow - 1, b.P3, B[0]); raw_cell(pc + nx * qrow, b.P3, B[1]);
-      raw_cell(pc + nx * qrow + 1, b.P3, B[2]);
-      ld_met(sp + nx * mrow, metn);
-      const bool slo = strong_at(strong, sm, 0, 0, j, k), shi = strong_at(strong, sm, 0, 1, j, k);
-      const bool dlo = dbl_at(c, mx, slo, shi), dhi = dbl_at(c + 1, mx, slo, shi);
-      const bool ovr_lo = c == 1 && slo, ovr_hi = c == mx && shi;
-      double Fv[5];
-      if (!MIXED) {
-        double dqp[5], dqmn[5], dqm[5];
-#pragma unroll
-        for (int m = 0; m < 5; ++m) {
-          double a = A[1][m] - A[0][m], bb = A[2][m] - A[1][m];
-          if (dlo) a = (A[1][m] - A[0][m]) * 2;
-          if (dhi) bb = (A[2][m] - A[1][m]) * 2;
-          if (!fo) limit_cell64(ph.ilimf, ph.epslimf, ph.rkap, a, bb, dqp[m], dqmn[m]);
-          else { dqp[m] = 0.0; dqmn[m] = 0.0; }
-          dqm[m] = __shfl_up_sync(0xffffffffu, dqmn[m], 1);
-        }
-        double qr[5], ql[5];
-        face_states64(fo, ovr_lo, ovr_hi, A[0], A[1], dqm, dqp, ql, qr);
-        if (face) {
-          const double ubn = MV ? face_ubn(vp, 0, met[0], met[1], met[2]) : 0.0;
-          roe_flux_euler<MV>(ph, met[0], met[1], met[2], met[3], qr, ql, Fv, ubn);
-        }
+    if (RMS) acc[m] += r[m] * r[m];
+    if (A.rhs_mode) {
+      double *rh = A.rhs + o;
+      if (A.rhs_mode == 2) {
+        const double rn = *rh + r[m];
+        *rh = rn;
+        r[m] = r[m] - rn;
       } else {
-        float dqp[5], dqmn[5], dqm[5], b0[5], bm1[5], dlr[5];
+        r[m] = r[m] - *rh;
+      }
+    }
+    if (A.res_out) A.res_out[o] = r[m];
+    if (A.update) {
+      if (A.qold_copy) A.qold_copy[o] = q0[m];
+      qw[m] = __fma_rn(-__dmul_rn(A.ar, r[m]), dt, q0[m]);
+    }
+  }
+  if (A.update) {
+    // the next stage reads primitive variables: one conversion here for the
+    // three families' loads (and bprtest's test of that stage's input)
+    if (A.prim_out) to_prim(gamma, qmin_rho, qmin_p, st, qw);
+#pragma unroll
+    for (int m = 0; m < 5; ++m) A.qout[p3_var(b, 5, S, m + 1, n) + cell] = qw[m];
+  }
+}
+
+// i-face rows of one task.  OUT 0: fluxes stored; 1: D = F(c+1) - F(c) of the
+// 30 cells between the task's 31 faces
+template <bool MIXED, bool CONV, bool MV, bool LIM1, int OUT>
+__device__ __forceinline__ void line_i(const FaceTask &T, const LinePar &LP, const LineArgs &L, StageI &B, int lane) {
+  const DevBlock &b = L.blocks[T.blk];
+  const PhysPar &ph = LP.ph;
+  const int n = T.n, nh = n * LP.hbmove, k = T.tb, mx = b.im;
+  const bool fo = L.first_order != 0;
+  const StrongMap &sm = L.smap[T.blk];
+  const bool strong = sm.off[0][0] >= 0 || sm.off[0][1] >= 0;
+  int st = 0;
+  // lane l: cell c, column l + 1; lanes 0 and 31 also bring columns 0 and 33.
+  // Cells past the line's last halo cell repeat it, faces past the line repeat
+  // the last metrics; nothing of them is stored.
+  const int c = T.i0 - 1 + lane;
+  const bool face = lane >= 1 && c >= 1 && c <= mx, edge = lane == 0 || lane == 31;
+  const int ecol = lane == 0 ? 0 : 33, ce = lane == 0 ? c - 1 : c + 1;
+  const bool in_0 = c >= 1 && c <= mx - 1, in_e = ce >= 1 && ce <= mx - 1;
+  const unsigned P3 = (unsigned)b.P3, qrow = (unsigned)b.I3;
+  const double *qb = L.q + p3_var(b, 5, LP.S, 1, n) + p3_cell(b, 0, T.ta, k);
+  const unsigned o0 = (unsigned)min(c, mx + 1), oe = (unsigned)min(ce, mx + 1);
+  const int64_t e0 = p2_idx(b, LP.S2, 1, min(c, mx), T.ta, k, nh);
+  const double *sp = L.s[0] + e0, *vp = MV ? L.fv.f[0] + e0 / 4 * 3 : nullptr;
+  const unsigned fv = (unsigned)b.im * (unsigned)b.jm * (unsigned)b.km;  // variable stride of an F0 array
+  double *Fp = L.cf + f0_idx(b, 5, LP.S, min(max(c, 1), mx), T.ta, k, 1, n);
+  const int64_t mrow = (int64_t)(b.im + 2) * 4;
+  const int frow = b.im;
+  auto issue = [&](int slot) {
+#pragma unroll
+    for (int m = 0; m < 5; ++m) cp8(&B.q[slot][m][lane + 1], qb + (int)o0 + (int64_t)m * P3);
+    if (edge) {
+#pragma unroll
+      for (int m = 0; m < 5; ++m) cp8(&B.q[slot][m][ecol], qb + (int)oe + (int64_t)m * P3);
+    }
+    cp16(&B.met[slot][0][lane], sp);
+    cp16(&B.met[slot][1][lane], sp + 2);
+    cp_commit();
+  };
+  issue(0);
+  for (int row = 0; row < T.nf; ++row) {
+    const int slot = row & 1;
+    __syncwarp();  // every lane is done with the slot that is filled next
+    if (row + 1 < T.nf) {
+      qb += qrow;
+      sp += mrow;
+      issue(slot ^ 1);
+      cp_wait<1>();
+    } else {
+      cp_wait<0>();
+    }
+    double qm[5], q0[5], qp[5], F[5];
+#pragma unroll
+    for (int m = 0; m < 5; ++m) q0[m] = B.q[slot][m][lane + 1];
+    if (CONV) {
+      if (in_0) {
+        to_prim(LP.gamma, LP.qmin_rho, LP.qmin_p, st, q0);
+#pragma unroll
+        for (int m = 1; m < 5; ++m) B.q[slot][m][lane + 1] = q0[m];
+      }
+      if (edge && in_e) {
+        double v[5];
+#pragma unroll
+        for (int m = 0; m < 5; ++m) v[m] = B.q[slot][m][ecol];
+        to_prim(LP.gamma, LP.qmin_rho, LP.qmin_p, st, v);
+#pragma unroll
+        for (int m = 1; m < 5; ++m) B.q[slot][m][ecol] = v[m];
+      }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int m = 0; m < 5; ++m) { qm[m] = B.q[slot][m][lane]; qp[m] = B.q[slot][m][lane + 2]; }
+    const double2 ma = B.met[slot][0][lane], mb = B.met[slot][1][lane];
+    const double met[4] = {ma.x, ma.y, mb.x, mb.y};
+    bool slo = false, shi = false;
+    if (strong) {
+      slo = strong_at(L.strong, sm, 0, 0, T.ta + row, k);
+      shi = strong_at(L.strong, sm, 0, 1, T.ta + row, k);
+    }
+    if (!MIXED) {
+      double qr[5], ql[5];
+#pragma unroll
+      for (int m = 0; m < 5; ++m) {
+        double a = q0[m] - qm[m], bb = qp[m] - q0[m];
+        if (strong) {
+          // per-slope doubling on strong-boundary faces (muscl_b*, src/flux.f90:1318-1406)
+          if ((c == 1 && slo) || (c == mx && shi)) a = a * 2;
+          if ((c == 0 && slo) || (c == mx - 1 && shi)) bb = bb * 2;
+        }
+        double up;
+        if (fo) { qr[m] = q0[m]; up = q0[m]; }
+        else cell_states64<LIM1>(ph.ilimf, ph.epslimf, ph.rkap, q0[m], a, bb, qr[m], up);
+        ql[m] = __shfl_up_sync(0xffffffffu, up, 1);
+      }
+      if (strong) {
 #pragma unroll
         for (int m = 0; m < 5; ++m) {
-          const float a = (float)(A[1][m] - A[0][m]), bb = (float)(A[2][m] - A[1][m]);
-          dlr[m] = a;
-          b0[m] = (float)A[1][m];
-          bm1[m] = (float)A[0][m];
-          if (!fo) limit_cell32(ph.ilimf, eps32, rk32, dlo ? a * 2.0f : a, dhi ? bb * 2.0f : bb, dqp[m], dqmn[m]);
-          else { dqp[m] = 0.0f; dqmn[m] = 0.0f; }
-          dqm[m] = __shfl_up_sync(0xffffffffu, dqmn[m], 1);
-        }
-        float dqL[5], dqR[5];
-        face_offsets32(ovr_lo, ovr_hi, dlr, dqm, dqp, dqL, dqR);
-        if (face) {
-          const double ubn = MV ? face_ubn(vp, 0, met[0], met[1], met[2]) : 0.0;
-          face_flux_mixed<MV>(ph, g32, gg32, met, A[0], bm1, b0, dlr, dqL, dqR, Fv, ubn);
+          if (c == 1 && slo) { qr[m] = qm[m]; ql[m] = qm[m]; }
+          if (c == mx && shi) { qr[m] = q0[m]; ql[m] = q0[m]; }
         }
       }
+      const double ubn = MV ? face_ubn(vp, met[0], met[1], met[2]) : 0.0;
+      roe_flux_euler<MV>(ph, met[0], met[1], met[2], met[3], qr, ql, F, ubn);
+    } else {
+      const float eps32 = (float)ph.epslimf, rk32 = (float)ph.rkap;
+      float dqL[5], dqR[5], b0[5], bm1[5], dlr[5];
+#pragma unroll
+      for (int m = 0; m < 5; ++m) {
+        float a = (float)(q0[m] - qm[m]), bb = (float)(qp[m] - q0[m]);
+        dlr[m] = a;
+        b0[m] = (float)q0[m];
+        bm1[m] = (float)qm[m];
+        if (strong) {
+          if ((c == 1 && slo) || (c == mx && shi)) a = a * 2.0f;
+          if ((c == 0 && slo) || (c == mx - 1 && shi)) bb = bb * 2.0f;
+        }
+        float dm = 0.0f;
+        dqR[m] = 0.0f;
+        if (!fo) limit_cell32(LIM1 ? 1 : ph.ilimf, eps32, rk32, a, bb, dqR[m], dm);
+        dqL[m] = __shfl_up_sync(0xffffffffu, dm, 1);
+      }
+      if (strong) {
+#pragma unroll
+        for (int m = 0; m < 5; ++m) {
+          if (c == 1 && slo) { dqL[m] = 0.0f; dqR[m] = -dlr[m]; }  // both states = cell L
+          if (c == mx && shi) { dqL[m] = dlr[m]; dqR[m] = 0.0f; }  // both states = cell R
+        }
+      }
+      const double ubn = MV ? face_ubn(vp, met[0], met[1], met[2]) : 0.0;
+      face_flux_mixed<MV>(ph, (float)ph.g, (float)ph.g_gm1, met, qm, bm1, b0, dlr, dqL, dqR, F, ubn);
+    }
+    if (OUT == 0) {
       if (face) {
 #pragma unroll
-        for (int m = 0; m < 5; ++m) Fp[m * fv] = Fv[m];
+        for (int m = 0; m < 5; ++m) Fp[(int64_t)m * fv] = F[m];
       }
+    } else {
 #pragma unroll
-      for (int m = 0; m < 5; ++m) { A[0][m] = B[0][m]; A[1][m] = B[1][m]; A[2][m] = B[2][m]; }
+      for (int m = 0; m < 5; ++m) F[m] = __shfl_down_sync(0xffffffffu, F[m], 1) - F[m];
+      if (lane >= 1 && lane <= 30 && c <= mx - 1) {
 #pragma unroll
-      for (int m = 0; m < 4; ++m) met[m] = metn[m];
-      pc += qrow; sp += mrow; Fp += frow;
-      if (MV) vp += mrow / 4 * 3;
+        for (int m = 0; m < 5; ++m) Fp[(int64_t)m * fv] = F[m];
+      }
     }
-  } else {
-    // lanes along i; march along d over faces f0 .. f0 + nf - 1
-    const int i = T.i0 + lane;
-    if (i <= b.im - 1) {
-      const int tb = T.tb;
-      // transverse cell indices of the line for strong_at: (i, k) for d = 2, (i, j) for d = 3
-      const bool slo = strong_at(strong, sm, d - 1, 0, i, tb), shi = strong_at(strong, sm, d - 1, 1, i, tb);
-      const int64_t step = d == 2 ? (int64_t)b.I3 : (int64_t)b.I3 * b.J3;
-      const int64_t mstep = d == 2 ? (int64_t)(b.im + 2) * 4 : (int64_t)(b.im + 2) * (b.jm + 2) * 4;
-      const int64_t fstep = d == 2 ? (int64_t)b.im : (int64_t)b.im * b.jm;
-      const int f0 = T.f0, f1 = T.f0 + T.nf;
-      const double *p = qv + (d == 2 ? p3_cell(b, i, f0 - 2, tb) : p3_cell(b, i, tb, f0 - 2));
-      const double *sp = s + (d == 2 ? p2_idx(b, S2, 1, i, f0, tb, nh) : p2_idx(b, S2, 1, i, tb, f0, nh));
-      double *Fp = F0 + (d == 2 ? f0_idx(b, 5, S, i, f0, tb, 1, n) : f0_idx(b, 5, S, i, tb, f0, 1, n));
-      const double *vp = MV ? FV.f[d - 1] + (sp - s) / 4 * 3 : nullptr;  // face velocity of face f0
-      auto inner = [&](int cc) { return cc >= 1 && cc <= mx - 1; };
-      double qa[5], qb[5], qc[5];
-      load_cell<CONV>(p, b.P3, inner(f0 - 2), LP, st, qa);
-      load_cell<CONV>(p + step, b.P3, inner(f0 - 1), LP, st, qb);
-      load_cell<CONV>(p + 2 * step, b.P3, inner(f0), LP, st, qc);
-      // cell f + 1 and the metrics of face f + 1 are loaded one step ahead
-      // (the cell converted when its step comes): step f reads cell
-      // min(f + 2, mx + 1) (the last halo layer) and face f + 1 <= mx + 1
-      double qn[5], met[4];
-      raw_cell(p + 3 * step, b.P3, qn);
-      ld_met(sp, met);
-      p += 4 * step;
-      sp += mstep;
-      // carried: qb = cell f-1, qc = cell f, dqm(f) (the slopes are taken
-      // again from the cells: fewer live registers)
+    Fp += frow;
+    if (MV) vp += mrow / 4 * 3;
+  }
+  if (CONV && st && L.status) atomicOr(L.status, st);
+}
+
+// a segment of j or k faces, lanes along i.  OUT 0: fluxes stored; 1: the
+// flux differences of the segment's nf - 1 cells added to D; 2: D with them
+// added goes through finish_cell
+template <bool MIXED, bool CONV, bool MV, bool LIM1, int OUT, bool RMS>
+__device__ __forceinline__ void line_m(const FaceTask &T, const LinePar &LP, const LineArgs &L, const StageArgs &A,
+                                       const cosa_params *Pp, int part_row, StageM<OUT> &B, int lane) {
+  const DevBlock &b = L.blocks[T.blk];
+  const PhysPar &ph = LP.ph;
+  const int d = T.d, n = T.n, nh = n * LP.hbmove, tb = T.tb, f0 = T.f0, f1 = T.f0 + T.nf;
+  const bool fo = L.first_order != 0;
+  const int mx = d == 2 ? b.jm : b.km;
+  int st = 0;
+  const bool act = T.i0 + lane <= b.im - 1;
+  const int i = min(T.i0 + lane, b.im - 1);
+  bool slo, shi;
+  {
+    const StrongMap &sm = L.smap[T.blk];
+    slo = d == 2 ? strong_at(L.strong, sm, 1, 0, i, tb) : strong_at(L.strong, sm, 2, 0, i, tb);
+    shi = d == 2 ? strong_at(L.strong, sm, 1, 1, i, tb) : strong_at(L.strong, sm, 2, 1, i, tb);
+  }
+  const unsigned P3 = (unsigned)b.P3;
+  const unsigned step = d == 2 ? (unsigned)b.I3 : (unsigned)b.I3 * (unsigned)b.J3;
+  const int64_t mstep = d == 2 ? (int64_t)(b.im + 2) * 4 : (int64_t)(b.im + 2) * (b.jm + 2) * 4;
+  const unsigned fstep = d == 2 ? (unsigned)b.im : (unsigned)b.im * (unsigned)b.jm;
+  const unsigned fv = (unsigned)b.im * (unsigned)b.jm * (unsigned)b.km;
+  const int64_t cell0 = p3_var(b, 5, LP.S, 1, n) + (d == 2 ? p3_cell(b, i, f0, tb) : p3_cell(b, i, tb, f0));
+  const double *pq = L.q + cell0;  // cell f0
+  const int64_t e0 = d == 2 ? p2_idx(b, LP.S2, 1, i, f0, tb, nh) : p2_idx(b, LP.S2, 1, i, tb, f0, nh);
+  const double *sp = (d == 2 ? L.s[1] : L.s[2]) + e0;
+  const double *vp = MV ? (d == 2 ? L.fv.f[1] : L.fv.f[2]) + e0 / 4 * 3 : nullptr;
+  double *Fp = L.cf + (OUT == 0 ? (int64_t)(d - 1) * L.n0 * 5 * LP.S : 0) +
+               (d == 2 ? f0_idx(b, 5, LP.S, i, f0, tb, 1, n) : f0_idx(b, 5, LP.S, i, tb, f0, 1, n));
+  double qc[5];
+  double acc[5] = {0, 0, 0, 0, 0};
+  // the running left state: cell f - 1 on face f; FP64: ql the state, a the
+  // slope of cell f (doubled at a strong boundary); mixed: dm the FP32 offset
+  // from cell f - 1 (qb, fb), sB the undoubled slope
+  double a[5], ql[5], qb[5];
+  float dm[5], sB[5], fb[5], fc[5];
+  const float eps32 = (float)ph.epslimf, rk32 = (float)ph.rkap;
+  // step f's data: cell f + 1, the metrics of face f; the chain: D, base state
+  // and time step of cell f - 1
+  auto issue = [&](int f, int slot) {
+    const double *p = pq + (f - f0 + 1) * (int64_t)step;
+#pragma unroll
+    for (int m = 0; m < 5; ++m) cp8(&B.q[slot][m][lane], p + (int64_t)m * P3);
+    const double *s = sp + (f - f0) * mstep;
+    cp16(&B.met[slot][0][lane], s);
+    cp16(&B.met[slot][1][lane], s + 2);
+    if (OUT >= 1 && f > f0) {
+      const double *D = Fp + (int64_t)(f - 1 - f0) * fstep;
+#pragma unroll
+      for (int m = 0; m < 5; ++m) cp8(&B.D[slot][m][lane], D + (int64_t)m * fv);
+      if (OUT == 2 && A.update) {
+        const double *p0 = A.qold + cell0 + (f - 1 - f0) * (int64_t)step;
+#pragma unroll
+        for (int m = 0; m < 5; ++m) cp8(&B.base[slot][m][lane], p0 + (int64_t)m * P3);
+        cp8(&B.base[slot][OUT == 2 ? 5 : 0][lane], A.dtvol + p1_idx(b, LP.S, i, tb, f - 1, n));
+      }
+    }
+    cp_commit();
+  };
+  issue(f0, f0 & 1);
+  {
+    double qa[5], q1[5];
+#pragma unroll
+    for (int m = 0; m < 5; ++m) {
+      const double *p = pq + (int64_t)m * P3;
+      qa[m] = __ldg(p - 2 * (int64_t)step);
+      q1[m] = __ldg(p - (int64_t)step);
+      qc[m] = __ldg(p);
+    }
+    if (CONV) {
+      // interior: cells 1 .. mx - 1, tested where they are marched over
+      int skip = 0;
+      if (f0 - 2 >= 1) to_prim(LP.gamma, LP.qmin_rho, LP.qmin_p, skip, qa);
+      if (f0 - 1 >= 1) to_prim(LP.gamma, LP.qmin_rho, LP.qmin_p, skip, q1);
+      if (f0 <= mx - 1) to_prim(LP.gamma, LP.qmin_rho, LP.qmin_p, st, qc);
+    }
+    const bool dlo = f0 == 2 && slo, dmi = (f0 == 1 && slo) || (f0 == mx && shi);
+#pragma unroll
+    for (int m = 0; m < 5; ++m) {
       if (!MIXED) {
-        double dqm[5];
-#pragma unroll
-        for (int m = 0; m < 5; ++m) {
-          double a = qb[m] - qa[m], bb = qc[m] - qb[m];
-          if (dbl_at(f0 - 1, mx, slo, shi)) a = (qb[m] - qa[m]) * 2;
-          if (dbl_at(f0, mx, slo, shi)) bb = (qc[m] - qb[m]) * 2;
-          double unused;
-          if (!fo) limit_cell64(ph.ilimf, ph.epslimf, ph.rkap, a, bb, unused, dqm[m]);
-          else dqm[m] = 0.0;
-        }
-        for (int f = f0; f < f1; ++f) {
-          conv_cell<CONV>(inner(f + 1), LP, st, qn);
-          double qx[5], metn[4];
-          raw_cell(f + 2 <= mx + 1 ? p : p - step, b.P3, qx);
-          ld_met(sp, metn);
-          p += step;
-          sp += mstep;
-          const bool dl = dbl_at(f, mx, slo, shi), dh = dbl_at(f + 1, mx, slo, shi);
-          const bool ovr_lo = f == 1 && slo, ovr_hi = f == mx && shi;
-          double dqp[5], dqmn[5];
-#pragma unroll
-          for (int m = 0; m < 5; ++m) {
-            double a = qc[m] - qb[m], bb = qn[m] - qc[m];
-            if (dl) a = (qc[m] - qb[m]) * 2;
-            if (dh) bb = (qn[m] - qc[m]) * 2;
-            if (!fo) limit_cell64(ph.ilimf, ph.epslimf, ph.rkap, a, bb, dqp[m], dqmn[m]);
-            else { dqp[m] = 0.0; dqmn[m] = 0.0; }
-          }
-          double qr[5], ql[5], Fv[5];
-          face_states64(fo, ovr_lo, ovr_hi, qb, qc, dqm, dqp, ql, qr);
-          const double ubn = MV ? face_ubn(vp, 0, met[0], met[1], met[2]) : 0.0;
-          roe_flux_euler<MV>(ph, met[0], met[1], met[2], met[3], qr, ql, Fv, ubn);
-          if (MV) vp += mstep / 4 * 3;
-#pragma unroll
-          for (int m = 0; m < 5; ++m) Fp[m * fv] = Fv[m];
-          Fp += fstep;
-#pragma unroll
-          for (int m = 0; m < 5; ++m) { qb[m] = qc[m]; qc[m] = qn[m]; qn[m] = qx[m]; dqm[m] = dqmn[m]; }
-#pragma unroll
-          for (int m = 0; m < 4; ++m) met[m] = metn[m];
-        }
+        double a0 = q1[m] - qa[m];
+        a[m] = qc[m] - q1[m];
+        if (dlo) a0 = a0 * 2;
+        if (dmi) a[m] = a[m] * 2;
+        double lo_;
+        if (fo) ql[m] = q1[m];
+        else cell_states64<LIM1>(ph.ilimf, ph.epslimf, ph.rkap, q1[m], a0, a[m], lo_, ql[m]);
+        if (f0 == 1 && slo) ql[m] = q1[m];  // strong lower boundary: both states of face 1 are cell 0
       } else {
-        float sB[5], dqm[5], fb[5], fc[5];
-#pragma unroll
-        for (int m = 0; m < 5; ++m) {
-          const float a = (float)(qb[m] - qa[m]), bb = (float)(qc[m] - qb[m]);
-          sB[m] = bb;
-          fb[m] = (float)qb[m]; fc[m] = (float)qc[m];
-          float unused;
-          if (!fo)
-            limit_cell32(ph.ilimf, eps32, rk32, dbl_at(f0 - 1, mx, slo, shi) ? a * 2.0f : a,
-                         dbl_at(f0, mx, slo, shi) ? bb * 2.0f : bb, unused, dqm[m]);
-          else dqm[m] = 0.0f;
-        }
-        for (int f = f0; f < f1; ++f) {
-          conv_cell<CONV>(inner(f + 1), LP, st, qn);
-          double qx[5], metn[4];
-          raw_cell(f + 2 <= mx + 1 ? p : p - step, b.P3, qx);
-          ld_met(sp, metn);
-          p += step;
-          sp += mstep;
-          const bool dl = dbl_at(f, mx, slo, shi), dh = dbl_at(f + 1, mx, slo, shi);
-          const bool ovr_lo = f == 1 && slo, ovr_hi = f == mx && shi;
-          float dqp[5], dqmn[5], bbv[5];
-#pragma unroll
-          for (int m = 0; m < 5; ++m) {
-            const float bb = (float)(qn[m] - qc[m]);
-            bbv[m] = bb;
-            if (!fo) limit_cell32(ph.ilimf, eps32, rk32, dl ? sB[m] * 2.0f : sB[m], dh ? bb * 2.0f : bb, dqp[m],
-                                  dqmn[m]);
-            else { dqp[m] = 0.0f; dqmn[m] = 0.0f; }
-          }
-          // sB = (float)(q(f) - q(f-1)), undoubled
-          float dqL[5], dqR[5];
-          face_offsets32(ovr_lo, ovr_hi, sB, dqm, dqp, dqL, dqR);
-          double Fv[5];
-          const double ubn = MV ? face_ubn(vp, 0, met[0], met[1], met[2]) : 0.0;
-          face_flux_mixed<MV>(ph, g32, gg32, met, qb, fb, fc, sB, dqL, dqR, Fv, ubn);
-          if (MV) vp += mstep / 4 * 3;
-#pragma unroll
-          for (int m = 0; m < 5; ++m) Fp[m * fv] = Fv[m];
-          Fp += fstep;
-#pragma unroll
-          for (int m = 0; m < 5; ++m) {
-            qb[m] = qc[m]; qc[m] = qn[m]; qn[m] = qx[m];
-            fb[m] = fc[m]; fc[m] = (float)qc[m];
-            sB[m] = bbv[m];
-            dqm[m] = dqmn[m];
-          }
-#pragma unroll
-          for (int m = 0; m < 4; ++m) met[m] = metn[m];
-        }
+        const float a0 = (float)(q1[m] - qa[m]);
+        sB[m] = (float)(qc[m] - q1[m]);
+        qb[m] = q1[m];
+        fb[m] = (float)q1[m];
+        fc[m] = (float)qc[m];
+        float lo_;
+        dm[m] = 0.0f;
+        if (!fo) limit_cell32(LIM1 ? 1 : ph.ilimf, eps32, rk32, dlo ? a0 * 2.0f : a0, dmi ? sB[m] * 2.0f : sB[m], lo_, dm[m]);
+        if (f0 == 1 && slo) dm[m] = 0.0f;
       }
     }
   }
-  if (st && status) atomicOr(status, st);
+  double Fprev[5];
+  for (int f = f0; f < f1; ++f) {
+    const int slot = f & 1;
+    if (f + 1 < f1) {
+      issue(f + 1, slot ^ 1);
+      cp_wait<1>();
+    } else {
+      cp_wait<0>();
+    }
+    double qn[5], F[5];
+#pragma unroll
+    for (int m = 0; m < 5; ++m) qn[m] = B.q[slot][m][lane];
+    if (CONV && f + 1 <= mx - 1) to_prim(LP.gamma, LP.qmin_rho, LP.qmin_p, st, qn);
+    if (!MIXED) {
+      double qr[5], up[5];
+#pragma unroll
+      for (int m = 0; m < 5; ++m) {
+        double bb = qn[m] - qc[m];
+        if (f + 1 == mx && shi) bb = bb * 2;
+        if (fo) { qr[m] = qc[m]; up[m] = qc[m]; }
+        else cell_states64<LIM1>(ph.ilimf, ph.epslimf, ph.rkap, qc[m], a[m], bb, qr[m], up[m]);
+        a[m] = bb;
+      }
+      if (f == 1 && slo) {
+#pragma unroll
+        for (int m = 0; m < 5; ++m) qr[m] = ql[m];
+      }
+      if (f == mx && shi) {
+#pragma unroll
+        for (int m = 0; m < 5; ++m) { qr[m] = qc[m]; ql[m] = qc[m]; }
+      }
+#pragma unroll
+      for (int m = 0; m < 5; ++m) qc[m] = qn[m];
+      const double2 ma = B.met[slot][0][lane], mb = B.met[slot][1][lane];
+      const double ubn = MV ? face_ubn(vp, ma.x, ma.y, mb.x) : 0.0;
+      roe_flux_euler<MV>(ph, ma.x, ma.y, mb.x, mb.y, qr, ql, F, ubn);
+#pragma unroll
+      for (int m = 0; m < 5; ++m) ql[m] = up[m];
+    } else {
+      float dqL[5], dqR[5], bbv[5], up[5];
+#pragma unroll
+      for (int m = 0; m < 5; ++m) {
+        bbv[m] = (float)(qn[m] - qc[m]);
+        const float al = (f == 1 && slo) || (f == mx && shi) ? sB[m] * 2.0f : sB[m];
+        dqL[m] = dm[m];
+        dqR[m] = 0.0f;
+        up[m] = 0.0f;
+        if (!fo) limit_cell32(LIM1 ? 1 : ph.ilimf, eps32, rk32, al, f + 1 == mx && shi ? bbv[m] * 2.0f : bbv[m], dqR[m], up[m]);
+        if (f == 1 && slo) dqR[m] = -sB[m];
+        if (f == mx && shi) { dqL[m] = sB[m]; dqR[m] = 0.0f; }
+      }
+      const double2 ma = B.met[slot][0][lane], mb = B.met[slot][1][lane];
+      const double met[4] = {ma.x, ma.y, mb.x, mb.y};
+      const double ubn = MV ? face_ubn(vp, met[0], met[1], met[2]) : 0.0;
+      face_flux_mixed<MV>(ph, (float)ph.g, (float)ph.g_gm1, met, qb, fb, fc, sB, dqL, dqR, F, ubn);
+#pragma unroll
+      for (int m = 0; m < 5; ++m) {
+        qb[m] = qc[m];
+        qc[m] = qn[m];
+        fb[m] = fc[m];
+        fc[m] = (float)qn[m];
+        sB[m] = bbv[m];
+        dm[m] = up[m];
+      }
+    }
+    if (OUT == 0) {
+      if (act) {
+#pragma unroll
+        for (int m = 0; m < 5; ++m) Fp[(int64_t)m * fv] = F[m];
+      }
+      Fp += fstep;
+    } else {
+      if (f > f0 && act) {
+        // bresid order: i, then j, then k (src/cosa.f90:1800-1876)
+        double D[5];
+#pragma unroll
+        for (int m = 0; m < 5; ++m) D[m] = B.D[slot][m][lane] + F[m] - Fprev[m];
+        if (OUT == 1) {
+          double *Dp = Fp + (int64_t)(f - 1 - f0) * fstep;
+#pragma unroll
+          for (int m = 0; m < 5; ++m) Dp[(int64_t)m * fv] = D[m];
+        } else {
+          double q0[5];
+#pragma unroll
+          for (int m = 0; m < 5; ++m) q0[m] = B.base[slot][OUT == 2 ? m : 0][lane];
+          const double ov = A.vol ? Pp->omega * A.vol[p1_idx(b, 1, i, tb, f - 1, 0)] : 0.0;
+          finish_cell<RMS>(A, *Pp, b, LP.S, n, p3_cell(b, i, tb, f - 1), ov, B.base[slot][OUT == 2 ? 5 : 0][lane], D, q0,
+                           LP.gamma, LP.qmin_rho, LP.qmin_p, acc, st);
+        }
+      }
+#pragma unroll
+      for (int m = 0; m < 5; ++m) Fprev[m] = F[m];
+    }
+    if (MV) vp += mstep / 4 * 3;
+  }
+  if (OUT == 2 && RMS) {
+#pragma unroll
+    for (int m = 0; m < 5; ++m) {
+      double x = acc[m];
+      for (int w = 16; w > 0; w >>= 1) x += __shfl_down_sync(0xffffffffu, x, w);
+      if (lane == 0) A.part[(int64_t)part_row * 8 + m] = x;
+    }
+  }
+  if (st && L.status) atomicOr(L.status, st);
+}
+
+// Resident warps per SM that the line kernels are compiled for.  FP64 i lines
+// and the store kernel at 16 (128 registers, a few words spilled), the marching
+// chain kernels at 12 (168 registers).  Measured, one cycle of the 30.7 M-cell
+// duct: i lines at 12 / 16 / 18 warps 16.95 / 16.84 / - ms; marching at 11 /
+// 12 / 14 warps 17.3 / 16.8 / 18.9 ms (spills).  Five cycles of the pitching
+// aerofoil (store) at 10 / 14 / 16 warps 1.59 / 1.55 / 1.49 ms.  Mixed
+// precision fits 16 everywhere (18: 6.2 against 5.2 ms on the 4.2 M-cell duct).
+constexpr int kWarpsStore = 16, kWarpsI = 16, kWarpsM = 12, kWarpsMixed = 16;
+
+// store schedule: all faces, the task's family picks the loop
+template <bool MIXED, bool CONV, bool MV, bool LIM1>
+__global__ void __launch_bounds__(32, MIXED ? kWarpsMixed : kWarpsStore)
+k_line_store(const LinePar LP, const LineArgs L) {
+  __shared__ union {
+    StageI i;
+    StageM<0> m;
+  } B;
+  const FaceTask T = L.tasks[blockIdx.x];
+  if (T.d == 1) line_i<MIXED, CONV, MV, LIM1, 0>(T, LP, L, B.i, threadIdx.x);
+  else line_m<MIXED, CONV, MV, LIM1, 0, false>(T, LP, L, StageArgs{}, nullptr, 0, B.m, threadIdx.x);
+}
+// chain schedule: family FAM; FAM 3 finishes the stage
+template <int FAM, bool MIXED, bool CONV, bool LIM1, bool RMS>
+__global__ void __launch_bounds__(32, MIXED ? kWarpsMixed : FAM == 1 ? kWarpsI : kWarpsM)
+k_line_chain(const LinePar LP, const LineArgs L, const StageArgs A, const cosa_params *__restrict__ Pp) {
+  const FaceTask T = L.tasks[blockIdx.x];
+  if constexpr (FAM == 1) {
+    __shared__ StageI B;
+    line_i<MIXED, CONV, false, LIM1, 1>(T, LP, L, B, threadIdx.x);
+  } else {
+    __shared__ StageM<FAM - 1> B;
+    line_m<MIXED, CONV, false, LIM1, FAM - 1, RMS>(T, LP, L, A, Pp, blockIdx.x, B, threadIdx.x);
+  }
 }

@@ -1,30 +1,18 @@
-// Fused RK stage for sm_100a: halo fill + tiled residual/update kernel.
+// Fused RK stage for sm_100a: halo fill, stage arguments, norm reduction.
 //
 // One RK stage of smooth() (src/cosa.f90:1719-2016) for the explicit Euler
 // path is cons2prim -> bc -> cutman_q -> prtest -> [lambda, deltat] ->
 // muscl/roflux/resid x3 -> prim2cons -> [resg_rms] -> update: about 25
-// full-array sweeps.  Here it is two kernels:
+// full-array sweeps.  Here it is k_halo, then the line kernels of faces.cuh:
 //
-//  k_halo        one thread per boundary/cut face cell and snapshot: reads
-//                the conservative interior next to the face, converts it to
-//                primitive form, applies the BC (or the cut copy) and writes
-//                the primitive halo values into the halo slots of the same
-//                state array.  Halo cells written twice in the reference keep
-//                the reference's last writer (mask computed on the host).
-//  k_stage_tile  a CTA owns a TI x TJ column of cells of one block and
-//                marches along k.  Planes of the state are staged in a 4-deep
-//                shared-memory ring (interior cells converted cons->prim on
-//                the way in, halo cells taken as written by k_halo); every
-//                i-, j- and k-face of the tile is reconstructed (MUSCL +
-//                limiter) and Roe-fluxed once per tile, the k-face flux is
-//                carried in registers between planes, the flux divergence is
-//                summed in the reference order, and the stage update
-//                q = qold - alpha dt/V R is written directly.  On stage 1 it
-//                also computes the local time step (lambda/deltat) and the
-//                per-tile residual sums of squares for resg_rms.
+//  k_halo        two threads per boundary/cut face cell and snapshot: read
+//                the interior next to the face, convert it to primitive form
+//                (first stage; later stages hold primitive values), apply the
+//                BC (or the cut copy) and write the primitive halo values
+//                into the halo slots of the same state array.  Halo cells
+//                written twice in the reference keep the reference's last
+//                writer (mask computed on the host).
 #pragma once
-#include <cuda_pipeline.h>
-
 #include "physics.cuh"
 #include "kernels_ref.cuh"
 
@@ -42,10 +30,6 @@ struct __align__(16) HaloItem {
   signed char sgn;  // sign applied to the face normal
   signed char nl;   // multigrid level of the item's block (the low-speed cut-off epsp(nl))
   int pad[2];
-};
-
-struct Tile {
-  int blk, n, i0, j0, k0, k1;  // first cell (i0,j0), planes k0..k1 (inclusive)
 };
 
 // strong-boundary flags of one block: for each direction d and side s
@@ -71,11 +55,8 @@ struct FaceVel {
 
 // the boundary values of every flow-condition slot and level (make_bcpar:
 // sines, cosines and a power), once per upload of the parameters instead of
-// once per halo cell and stage.  With them inside k_halo took 19.7 us on the
-// 128 x 64 x 2 channel and 92 us on the 4.2 M-cell duct (463 k items); with
-// this, 48-byte items and one snapshot per grid row twenty channel cycles
-// went from 3.34 to 2.90 ms, a cycle of the 30.7 M-cell duct from 21.8 to
-// 21.3 ms, five of the pitching aerofoil (S = 5) from 2.71 to 2.24 ms
+// once per halo cell: k_halo on the 24-block duct of 4.2 M cells (463 k items)
+// took 92 us with them inside, on the 128 x 64 x 2 channel 19.7 us
 __global__ void k_bcpar(const cosa_params *__restrict__ Pp, int nslots, BcPar *__restrict__ out) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t < nslots * COSA_MAX_LEVELS) out[t] = make_bcpar(Pp[t / COSA_MAX_LEVELS], t % COSA_MAX_LEVELS + 1);
@@ -83,11 +64,12 @@ __global__ void k_bcpar(const cosa_params *__restrict__ Pp, int nslots, BcPar *_
 
 // scalars of k_halo, passed by value
 struct HaloPar {
-  int S, S2, hbmove;
+  int S, S2, hbmove, test;  // test: bprtest of the i halos (fused stages)
   double gamma, qmin_rho, qmin_p;
 };
-inline HaloPar make_halo_par(const cosa_params &P) {
+inline HaloPar make_halo_par(const cosa_params &P, int test) {
   HaloPar h;
+  h.test = test;
   h.S = 2 * P.nharms + 1; h.S2 = 2 * P.nharms * P.hbmove + 1; h.hbmove = P.hbmove;
   h.gamma = P.gamma; h.qmin_rho = P.qmin[0]; h.qmin_p = P.qmin[4];
   return h;
@@ -205,22 +187,22 @@ k_halo(const DevBlock *__restrict__ blocks, const HaloItem *__restrict__ items, 
     if (write & 1) qd[v * dP3 + it.h1] = h1[v];
     if (write & 2) qd[v * dP3 + it.h2] = h2[v];
   }
-  if (CONS && it.idir == 1) {  // bprtest also checks the i halos of the state (src/cosa.f90:1000)
+  if (H.test && it.idir == 1) {  // bprtest also checks the i halos of the state (src/cosa.f90:1000)
     if (write & 1) { if (h1[4] <= H.qmin_p) st |= COSA_ERR_NEG_P; else if (h1[0] <= H.qmin_rho) st |= COSA_ERR_NEG_RHO; }
     if (write & 2) { if (h2[4] <= H.qmin_p) st |= COSA_ERR_NEG_P; else if (h2[0] <= H.qmin_rho) st |= COSA_ERR_NEG_RHO; }
   }
   if (st) atomicOr(status, st);
 }
 
-// ---- k_stage_tile ------------------------------------------------------------------
+// ---- stage arguments ------------------------------------------------------------------
 struct StageArgs {
-  const double *qin;     // stage input: interior conservative, halos primitive
+  const double *qin;     // stage input
   double *qout;          // stage output (interior written)
   const double *qold;    // RK base state q^n
   double *qold_copy;     // if set, q^n interior is copied here (stage 1)
-  double *dtvol;         // Delta t / V, written when compute_dt, read otherwise
+  double *dtvol;         // Delta t / V
   const double *si, *sj, *sk;
-  double *part;          // per-tile residual sums of squares (npde) or null
+  double *part;          // residual sums of squares (8 doubles per row) or null
   double *rhs;           // multigrid forcing term of a coarse level, or null
   int rhs_mode;          // 1: r -= rhs; 2: rhs += r first (forcing), then r -= rhs
   double *res_out;       // if set, the residual is stored here (P3 layout)
@@ -234,312 +216,31 @@ struct StageArgs {
   int compute_dt;
   int first_order;
   int update;            // 0: residual only (restriction pass)
+  int prim_out;          // 1: the output's interior is stored primitive (the next stage reads it so)
   const double *cfl_blk; // per-block CFL number (serving: each solve's own), or null for P.cfl
 };
 
-// Thread layout: TJ main warps, warp w holds row j0+w of the tile (lane =
-// i - i0) and computes that cell's left i-face, left j-face and upper k-face
-// of every plane, then updates the cell; one extra warp computes the tile's
-// boundary faces (the j-faces above the last row and the i-faces right of the
-// last column), so every warp does a balanced share of the Roe fluxes.
-template <int TI, int TJ, bool MIXED, bool RMS>
-__global__ void __launch_bounds__(TI *TJ + 32, 2)
-k_stage_tile(const DevBlock *__restrict__ blocks, const Tile *__restrict__ tiles, const cosa_params *__restrict__ Pp,
-             StageArgs A) {
-  static_assert(TI == 32, "a main warp is one row of the tile");
-  constexpr int NM = TI * TJ;                             // main threads (one per cell)
-  constexpr int NT = NM + 32;                             // + the boundary-face warp
-  constexpr int PI = TI + 4, PJ = TJ + 4, PL = PI * PJ;  // padded plane
-  constexpr int NSLOT = 5;                                // planes k-1..k+2 + the one in flight
-  constexpr int CPT = (PL + NT - 1) / NT;                 // plane cells per thread
-  extern __shared__ double smem[];
-  double *ring = smem;                        // [NSLOT][5][PJ][PI]
-  double *fi = ring + NSLOT * 5 * PL;         // [5][TJ][TI+1]
-  double *fj = fi + 5 * TJ * (TI + 1);        // [5][TJ+1][TI]
-  double *red = fj + 5 * (TJ + 1) * TI;       // [5][TJ]
-
-  const cosa_params &P = *Pp;
-  const Tile T = tiles[blockIdx.x];
-  const DevBlock b = blocks[T.blk];
-  const int npde = 5, S = 2 * P.nharms + 1, S2 = 2 * P.nharms * P.hbmove + 1;
-  const int n = T.n, nh = n * P.hbmove;
-  const PhysPar ph = make_phys(P);
-  const double g = P.gamma;
-  const int tid = threadIdx.x;
-  const bool main_warp = tid < NM;
-  const int ti = tid % TI, tj = main_warp ? tid / TI : 0;
-  const int ci = T.i0 + ti, cj = T.j0 + tj;          // this thread's cell column
-  const bool cvalid = main_warp && ci <= b.im - 1 && cj <= b.jm - 1;
-  const int64_t vstride = b.P3;
-  const double *qin = A.qin + p3_var(b, npde, S, 1, n);
-  const StrongMap sm = A.smap[T.blk];
-  // metric plane strides (fixed grid per snapshot)
-  const int64_t I2 = b.im + 2, J2 = b.jm + 2;
-  const int64_t mbase = (b.op2 * S2 + (int64_t)nh * I2 * J2 * (b.km + 2)) * 4;
-  int st = 0;
-
-  auto slot = [](int k) { return ((k % NSLOT) + NSLOT) % NSLOT; };
-
-  auto cell_kind = [&](int c, int k, int64_t &gcell) -> int {
-    if (c >= PL) return 0;
-    const int pi = c % PI, pj = c / PI;
-    const int i = T.i0 - 2 + pi, j = T.j0 - 2 + pj;
-    const bool iin = i >= 1 && i <= b.im - 1, jin = j >= 1 && j <= b.jm - 1, kin = k >= 1 && k <= b.km - 1;
-    const int nout = (!iin) + (!jin) + (!kin);
-    if (nout > 1 || i > b.im + 1 || j > b.jm + 1) return 0;  // corners, edges, outside
-    gcell = p3_cell(b, i, j, k);
-    return nout == 0 ? 1 : 2;
-  };
-  auto prefetch = [&](int k) {
-    double *dst = ring + slot(k) * 5 * PL;
-#pragma unroll
-    for (int r = 0; r < CPT; ++r) {
-      const int c = tid + r * NT;
-      int64_t gc;
-      if (!cell_kind(c, k, gc)) continue;
-#pragma unroll
-      for (int m = 0; m < 5; ++m) __pipeline_memcpy_async(dst + m * PL + c, qin + m * vstride + gc, sizeof(double));
-    }
-    __pipeline_commit();
-  };
-  auto convert = [&](int k) {
-    double *dst = ring + slot(k) * 5 * PL;
-#pragma unroll
-    for (int r = 0; r < CPT; ++r) {
-      const int c = tid + r * NT;
-      int64_t gc;
-      if (cell_kind(c, k, gc) != 1) continue;
-      double v[5];
-#pragma unroll
-      for (int m = 0; m < 5; ++m) v[m] = dst[m * PL + c];
-      c2p5_nr(g, v);
-      if (v[4] <= P.qmin[4]) st |= COSA_ERR_NEG_P;
-      else if (v[0] <= P.qmin[0]) st |= COSA_ERR_NEG_RHO;
-#pragma unroll
-      for (int m = 0; m < 5; ++m) dst[m * PL + c] = v[m];
-    }
-  };
-
-  // MUSCL + limiter + Roe flux of face f along a line: w0..w3 = cells f-2..f+1
-  auto face = [&](const double *w0p, const double *w1p, const double *w2p, const double *w3p, int f, int mx,
-                  bool slo, bool shi, const double *met, double *F) {
-    double qr[5], ql[5];
-    const bool ovr_lo = (f == 1 && slo), ovr_hi = (f == mx && shi);
-    const bool d_lo = (f - 1 == 1 && slo) || (f - 1 == mx && shi);
-    const bool d_mid = (f == 1 && slo) || (f == mx && shi);
-    const bool d_hi = (f + 1 == 1 && slo) || (f + 1 == mx && shi);
-#pragma unroll
-    for (int m = 0; m < 5; ++m) {
-      const double a0 = w0p[m * PL], a1 = w1p[m * PL], a2 = w2p[m * PL], a3 = w3p[m * PL];
-      if (A.first_order) {
-        qr[m] = a2; ql[m] = a1;
-      } else {
-        double dlo = a1 - a0, dmid = a2 - a1, dhi = a3 - a2;
-        if (d_lo) dlo = (a1 - a0) * 2;
-        if (d_mid) dmid = (a2 - a1) * 2;
-        if (d_hi) dhi = (a3 - a2) * 2;
-        if (MIXED) {
-          float dp, dm;
-          limit_face_fast(ph.ilimf, (float)ph.epslimf, (float)ph.rkap, (float)dlo, (float)dmid, (float)dhi, dp, dm);
-          qr[m] = a2 + (double)dp; ql[m] = a1 + (double)dm;
-        } else {
-          double dp, dm;
-          limit_face_nr(ph.ilimf, ph.epslimf, ph.rkap, dlo, dmid, dhi, dp, dm);
-          qr[m] = __dadd_rn(a2, dp); ql[m] = __dadd_rn(a1, dm);
-        }
-      }
-      if (ovr_lo) { qr[m] = a1; ql[m] = a1; }
-      if (ovr_hi) { qr[m] = a2; ql[m] = a2; }
-    }
-    if (MIXED) roe_flux_mixed(ph, met[0], met[1], met[2], met[3], qr, ql, F);
-    else roe_flux_euler(ph, met[0], met[1], met[2], met[3], qr, ql, F);
-  };
-
-  auto load_metric = [&](const double *s, int i, int j, int k, double *m4) {
-    const int64_t e = mbase + (i + I2 * (j + J2 * (int64_t)k)) * 4;
-    const double2 a = __ldg(reinterpret_cast<const double2 *>(s + e));
-    const double2 c = __ldg(reinterpret_cast<const double2 *>(s + e + 2));
-    m4[0] = a.x; m4[1] = a.y; m4[2] = c.x; m4[3] = c.y;
-  };
-
-  // k-face flux at face kf (between planes kf-1 and kf) of this column
-  auto kface = [&](int kf, double *F) {
-    const int pc = (tj + 2) * PI + (ti + 2);
-    double m4[4];
-    load_metric(A.sk, ci, cj, kf, m4);
-    const bool slo = (kf <= 2) && strong_at(A.strong, sm, 2, 0, ci, cj);
-    const bool shi = (kf >= b.km - 1) && strong_at(A.strong, sm, 2, 1, ci, cj);
-    face(ring + slot(kf - 2) * 5 * PL + pc, ring + slot(kf - 1) * 5 * PL + pc, ring + slot(kf) * 5 * PL + pc,
-         ring + slot(kf + 1) * 5 * PL + pc, kf, b.km, slo, shi, m4, F);
-  };
-
-  // the (up to) two in-plane faces of this thread: task t = 0, 1
-  //   main warps: t = 0 i-face (ci, cj), t = 1 j-face (ci, cj)
-  //   extra warp: t = 0 j-face (i0+lane, j0+TJ), t = 1 i-face (i0+TI, j0+lane) for lane < TJ
-  struct InTask { int dir, i, j; bool valid; };
-  auto task = [&](int t) -> InTask {
-    InTask r;
-    if (main_warp) {
-      r.dir = t; r.i = ci; r.j = cj;
-      r.valid = t == 0 ? (ci <= b.im && cj <= b.jm - 1) : (ci <= b.im - 1 && cj <= b.jm);
-    } else if (t == 0) {
-      r.dir = 1; r.i = T.i0 + ti; r.j = T.j0 + TJ;
-      r.valid = r.i <= b.im - 1 && r.j <= b.jm;
-    } else {
-      r.dir = 0; r.i = T.i0 + TI; r.j = T.j0 + ti;
-      r.valid = ti < TJ && r.i <= b.im && r.j <= b.jm - 1;
-    }
-    return r;
-  };
-
-  double acc[5] = {0, 0, 0, 0, 0};
-  for (int k = T.k0 - 2; k <= T.k0 + 2; ++k) prefetch(k);
-  __pipeline_wait_prior(0);
-  for (int k = T.k0 - 2; k <= T.k0 + 2; ++k) convert(k);
+// ---- deterministic reduction of partial rows -> resrms ------------------
+// many rows (the chain's last launch has one per warp) are first summed to
+// gridDim.x rows, row p of `part` into row p % gridDim.x
+__global__ void k_rms_mid(const double *__restrict__ part, int nparts, int npde, double *__restrict__ out) {
+  __shared__ double red[8][8];
+  double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  for (int64_t p = blockIdx.x + (int64_t)gridDim.x * threadIdx.x; p < nparts; p += (int64_t)gridDim.x * blockDim.x)
+    for (int v = 0; v < npde; ++v) acc[v] += part[p * 8 + v];
+  for (int v = 0; v < npde; ++v) {
+    double x = acc[v];
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+    if ((threadIdx.x & 31) == 0) red[v][threadIdx.x >> 5] = x;
+  }
   __syncthreads();
-  double fk_lo[5];
-  if (cvalid) kface(T.k0, fk_lo);
-
-  for (int k = T.k0; k <= T.k1; ++k) {
-    if (k > T.k0) {
-      __pipeline_wait_prior(0);  // plane k+2, issued during the previous face phase
-      convert(k + 2);
-    }
-    __syncthreads();
-    // the slot of plane k+3 held plane k-2, last read before the barrier above
-    if (k + 3 <= T.k1 + 2) prefetch(k + 3);
-    const double *pl = ring + slot(k) * 5 * PL;
-    {
-      InTask tk = task(0);
-      double mcur[4], mnext[4];
-      if (tk.valid) load_metric(tk.dir == 0 ? A.si : A.sj, tk.i, tk.j, k, mcur);
-#pragma unroll
-      for (int t = 0; t < 2; ++t) {
-        const InTask tn = task(1);
-        if (t == 0 && tn.valid) load_metric(tn.dir == 0 ? A.si : A.sj, tn.i, tn.j, k, mnext);
-        if (tk.valid) {
-          const int pc = (tk.j - T.j0 + 2) * PI + (tk.i - T.i0 + 2);
-          const int stride = tk.dir == 0 ? 1 : PI;
-          const int f = tk.dir == 0 ? tk.i : tk.j, mx = tk.dir == 0 ? b.im : b.jm;
-          const int t2 = tk.dir == 0 ? tk.j : tk.i;
-          const bool slo = (f <= 2) && strong_at(A.strong, sm, tk.dir, 0, t2, k);
-          const bool shi = (f >= mx - 1) && strong_at(A.strong, sm, tk.dir, 1, t2, k);
-          double F[5];
-          face(pl + pc - 2 * stride, pl + pc - stride, pl + pc, pl + pc + stride, f, mx, slo, shi, mcur, F);
-          if (tk.dir == 0) {
-            const int a = tk.i - T.i0, r = tk.j - T.j0;
-#pragma unroll
-            for (int m = 0; m < 5; ++m) fi[(m * TJ + r) * (TI + 1) + a] = F[m];
-          } else {
-            const int a = tk.i - T.i0, r = tk.j - T.j0;
-#pragma unroll
-            for (int m = 0; m < 5; ++m) fj[(m * (TJ + 1) + r) * TI + a] = F[m];
-          }
-        }
-        tk = tn;
-#pragma unroll
-        for (int m = 0; m < 4; ++m) mcur[m] = mnext[m];
-      }
-    }
-    double fk_hi[5];
-    if (cvalid) kface(k + 1, fk_hi);
-    __syncthreads();
-    if (cvalid) {
-      const int64_t cell = p3_cell(b, ci, cj, k);
-      const int64_t o1 = p1_idx(b, S, ci, cj, k, n);
-      double dt;
-      if (A.compute_dt) {
-        // lambdab + bdeltat (src/cosa.f90:1293-1323, 4860-4870)
-        double qc[5], sim[4], sip[4], sjm[4], sjp[4], skm[4], skp[4];
-        const int pc = (tj + 2) * PI + (ti + 2);
-#pragma unroll
-        for (int m = 0; m < 5; ++m) qc[m] = pl[m * PL + pc];
-        load_metric(A.si, ci, cj, k, sim); load_metric(A.si, ci + 1, cj, k, sip);
-        load_metric(A.sj, ci, cj, k, sjm); load_metric(A.sj, ci, cj + 1, k, sjp);
-        load_metric(A.sk, ci, cj, k, skm); load_metric(A.sk, ci, cj, k + 1, skp);
-        double li, lj, lk;
-        eig_eul(g, qc, sim, sip, sjm, sjp, skm, skp, li, lj, lk);
-        dt = (A.cfl_blk ? A.cfl_blk[T.blk] : P.cfl) / (li + lj + lk);
-        A.dtvol[o1] = dt;
-        if (A.bx) {
-          double ba, bb_, bc;
-          irs_beta(P.irsop, P.rat, P.psirs, li, lj, lk, ba, bb_, bc);
-          A.bx[o1] = ba; A.by[o1] = bb_; A.bz[o1] = bc;
-        }
-      } else {
-        dt = A.dtvol[o1];
-      }
-      const double *qo = A.qold + p3_var(b, npde, S, 1, n);
-      double *qw = A.qout + p3_var(b, npde, S, 1, n);
-#pragma unroll
-      for (int m = 0; m < 5; ++m) {
-        // bresid order: i, then j, then k (src/cosa.f90:1800-1876)
-        double r = fi[(m * TJ + tj) * (TI + 1) + ti + 1] - fi[(m * TJ + tj) * (TI + 1) + ti];
-        r = r + fj[(m * (TJ + 1) + tj + 1) * TI + ti] - fj[(m * (TJ + 1) + tj) * TI + ti];
-        r = r + fk_hi[m] - fk_lo[m];
-        // viscous terms (q_face/q_der/vflux/resid, src/cosa.f90:1809-1876)
-        if (A.vres) r = r + A.vres[p3_var(b, npde, S, m + 1, n) + cell];
-        if (A.vol) {
-          // src_bhb (src/src.f90:556-613): harmonic-balance coupling of the snapshots
-          const double ov = P.omega * A.vol[p1_idx(b, 1, ci, cj, k, 0)];
-          double qhb = 0.0;
-          for (int nj2 = 0; nj2 < S; ++nj2)
-            qhb = qhb + ov * P.dhb[n * S + nj2] * A.qin[p3_var(b, npde, S, m + 1, nj2) + cell];
-          r = r + qhb;
-        }
-        // resg_rms of the fine level, where rhs is zero (src/cosa.f90:1925-1936)
-        if (RMS) acc[m] += r * r;
-        if (A.rhs_mode) {
-          // multigrid forcing on coarse levels (src/cosa.f90:1950-1960)
-          double *rh = A.rhs + p3_var(b, npde, S, m + 1, n) + cell;
-          if (A.rhs_mode == 2) {
-            const double rn = *rh + r;
-            *rh = rn;
-            r = r - rn;
-          } else {
-            r = r - *rh;
-          }
-        }
-        if (A.res_out) A.res_out[p3_var(b, npde, S, m + 1, n) + cell] = r;
-        if (A.update) {
-          const double q0 = qo[m * vstride + cell];
-          if (A.qold_copy) A.qold_copy[p3_var(b, npde, S, m + 1, n) + cell] = q0;
-          qw[m * vstride + cell] = q0 - A.ar * r * dt;
-        }
-      }
-#pragma unroll
-      for (int m = 0; m < 5; ++m) fk_lo[m] = fk_hi[m];
-    }
+  if (threadIdx.x < npde) {
+    double x = 0;
+    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) x += red[threadIdx.x][w];
+    out[(int64_t)blockIdx.x * 8 + threadIdx.x] = x;
   }
-  if (RMS) {
-    __syncthreads();
-    // deterministic per-tile sums: warp shuffle then fixed-order warp sums
-    if (main_warp) {
-#pragma unroll
-      for (int m = 0; m < 5; ++m) {
-        double x = acc[m];
-        for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-        if ((tid & 31) == 0) red[m * TJ + (tid >> 5)] = x;
-      }
-    }
-    __syncthreads();
-    if (tid < 5) {
-      double x = 0;
-      for (int w = 0; w < TJ; ++w) x += red[tid * TJ + w];
-      A.part[(int64_t)blockIdx.x * 8 + tid] = x;
-    }
-  }
-  if (st) atomicOr(A.status, st);
 }
 
-template <int TI, int TJ>
-constexpr size_t stage_smem_bytes() {
-  return sizeof(double) * (5 * 5 * (TI + 4) * (TJ + 4) + 5 * TJ * (TI + 1) + 5 * (TJ + 1) * TI + 5 * TJ);
-}
-template <int TI, int TJ>
-constexpr int stage_threads() { return TI * TJ + 32; }
-
-// ---- deterministic reduction of per-tile / per-CTA partials -> resrms ------------------
 // resg_rms (src/cosa.f90:4458-4501): sqrt(sum/ncell), total sqrt(sum/ncell/npde)
 __global__ void k_rms_final(const double *__restrict__ part, int nparts, int npde, double ncell,
                             double *__restrict__ out, int *row_counter, int nrows_max) {
@@ -570,7 +271,7 @@ __global__ void k_rms_final(const double *__restrict__ part, int nparts, int npd
   }
 }
 
-// per-segment version of k_rms_final: CTA s reduces tiles [seg[2s], +seg[2s+1])
+// per-segment version of k_rms_final: CTA s reduces rows [seg[2s], +seg[2s+1])
 // in the same fixed order into out[s * (npde + 1) ...]
 __global__ void k_rms_seg(const double *__restrict__ part, const int *__restrict__ seg,
                           const double *__restrict__ seg_ncell, int npde, double *__restrict__ out) {

@@ -3,7 +3,7 @@
 // Every function restates a Fortran routine (cited) with the same operation
 // order and parenthesisation, so an FP64 build differs from the reference
 // only by FMA contraction.  The variants used by the fused stage kernel
-// (limit_face_nr, roe_flux_euler, c2p5_nr) take the reciprocals and
+// (cell_states64, roe_flux_euler, c2p5_nr) take the reciprocals and
 // reciprocal square roots on their dependency chains from rcp_nr / rsqrt_nr
 // below: results differ from the IEEE division and square root by at most a
 // couple of ulp, far inside the parity bound, and each chain gets shorter.
@@ -34,29 +34,28 @@ __host__ __device__ __forceinline__ PhysPar make_phys(const cosa_params &P) {
   return q;
 }
 
-// ---- Newton-Raphson reciprocal and reciprocal square root -------------------------
+// ---- reciprocal and reciprocal square root by a third-order step -------------------
 // Seeds from the PTX approximations rcp.approx.ftz.f64 / rsqrt.approx.ftz.f64
-// (relative error around 2^-22), then two Newton-Raphson steps each:
-//   1/x:        r <- r + r (1 - x r)              (error e -> e^2)
-//   1/sqrt(x):  y <- y (3/2 - (x/2) y^2)          (error e -> 3 e^2 / 2)
-// which leaves only the rounding of the last operations (a few ulp at most).
-// Inputs are positive normal numbers here (densities, speeds of sound squared,
-// sums of squares plus a positive epsilon); no zero, denormal or infinity
-// handling is needed or done.
+// (relative error below 2^-19), then one step of Householder's third-order
+// iteration, the residual's power series cut after its second term:
+//   1/x:        e = 1 - x r,    r <- r + r (e + e^2)           (error e^3)
+//   1/sqrt(x):  e = 1 - x y^2,  y <- y + y e (1/2 + 3/8 e)     (error 5/16 e^3)
+// 3 and 5 operations in place of the 4 and 7 of two Newton steps, and a
+// shorter chain; what is left is the rounding of the last operations (a few
+// ulp at most).  Inputs are positive normal numbers here (densities, speeds of
+// sound squared, sums of squares plus a positive epsilon); no zero, denormal
+// or infinity handling is needed or done.
 __device__ __forceinline__ double rcp_nr(double x) {
   double r;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-  double e = fma(-x, r, 1.0);
-  r = fma(r, e, r);
-  e = fma(-x, r, 1.0);
-  return fma(r, e, r);
+  const double e = __fma_rn(-x, r, 1.0);
+  return __fma_rn(r, __fma_rn(e, e, e), r);
 }
 __device__ __forceinline__ double rsqrt_nr(double x) {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double h = 0.5 * x;
-  y = y * fma(-h * y, y, 1.5);
-  return y * fma(-h * y, y, 1.5);
+  const double e = __fma_rn(-__dmul_rn(x, y), y, 1.0);
+  return __fma_rn(__dmul_rn(y, e), __fma_rn(0.375, e, 0.5), y);
 }
 
 // ---- cons2prim_b / prim2cons_b cell formulas (src/update.f90:2135-2188, 1875-2084)
@@ -151,9 +150,8 @@ __device__ __forceinline__ void limit_face(int ilim, T eps, T rkap, T dlo, T dmi
 // dhi = b), and dqm(c+1), the offset to its upper face (limit_face's dqm with
 // dlo = a, dmid = b), in FP64 for the fused stage kernels.  The sensor's
 // division is a Newton-Raphson reciprocal; every rounding is pinned with
-// explicit intrinsics (fixed contraction), so the tile kernel (two cells per
-// face) and the line-marching face kernel (one cell at a time) give the same
-// bits.  ilim 1, 2 and 4 share their sensor between dqp and dqm, as the
+// explicit intrinsics (fixed contraction), so every kernel that inlines it
+// gives the same bits.  ilim 1, 2 and 4 share their sensor between dqp and dqm, as the
 // reference's two expressions coincide (src/flux.f90:3561-3604).
 __device__ __forceinline__ double lim3_nr(double x, double y, double epsq) {
   // (x (y^2 + 2 e) + y (2 x^2 + e)) / (2 x^2 - x y + 2 y^2 + 3 e), limit_i ilim 3
@@ -197,13 +195,27 @@ __device__ __forceinline__ void limit_cell64(int ilim, double eps, double rkap, 
   }
 }
 
-// limit_face on the fused stage kernels' arithmetic: the two cells' halves
-// of limit_cell64 (dqp from cell f, dqm from cell f-1)
-__device__ __forceinline__ void limit_face_nr(int ilim, double eps, double rkap, double dlo, double dmid, double dhi,
-                                              double &dqp, double &dqm) {
-  double unused;
-  limit_cell64(ilim, eps, rkap, dmid, dhi, dqp, unused);
-  limit_cell64(ilim, eps, rkap, dlo, dmid, unused, dqm);
+// The two limited face states of a cell from its value q and its two slopes
+// a = q(c) - q(c-1), b = q(c+1) - q(c): lo on its lower face (q + dqp), up on
+// its upper face (q + dqm).  ilim 1 with the sensor s and t = s/4:
+//   (1 -+ k s) a + (1 +- k s) b = (a + b) +- k s (b - a),
+// 17 FP64 operations with the states, 22 as limit_cell64 and two additions.
+template <bool LIM1>
+__device__ __forceinline__ void cell_states64(int ilim, double eps, double rkap, double q, double a, double b,
+                                              double &lo, double &up) {
+  if (LIM1) {
+    const double den = __fma_rn(b, b, __fma_rn(a, a, eps));
+    const double s = __dmul_rn(__fma_rn(__dadd_rn(a, a), b, eps), rcp_nr(den));
+    const double t = __dmul_rn(0.25, s), ks = __dmul_rn(rkap, s);
+    const double p = __dadd_rn(a, b), d = __dsub_rn(b, a);
+    lo = __fma_rn(-t, __fma_rn(-ks, d, p), q);
+    up = __fma_rn(t, __fma_rn(ks, d, p), q);
+  } else {
+    double dqp, dqm;
+    limit_cell64(ilim, eps, rkap, a, b, dqp, dqm);
+    lo = __dadd_rn(q, dqp);
+    up = __dadd_rn(q, dqm);
+  }
 }
 
 // FP32 limiter of the mixed path: limit_face's algebra with fast division
@@ -287,141 +299,78 @@ __device__ __forceinline__ void roe_flux_fp64(const PhysPar &P, double kx, doubl
 }
 
 // Euler face flux for the fused stage: roflux_b's algebra with the TKE terms
-// (zero for Euler) dropped; sqrt(rho), 1/rho, the Roe-average weights, the
-// speed of sound and its inverse come from rsqrt_nr / rcp_nr instead of
-// separate square roots and divisions (last-bit differences).  MV: moving
-// face with normal grid speed ubn (src/flux.f90:110-113, 122-189): the normal
-// velocities relative to the face, the energy flux's p ubn and the shifted
-// eigenvalues; the fixed-grid instantiation has none of these terms.
+// (zero for Euler) dropped and its sums collected (129 FP64 operations, 162 as
+// the reference writes them): the Roe averages as x_L + w (x_R - x_L), the
+// dissipation through df1 = al1 + al3 + al4 and
+// c2 = a (al3 - al4) - al2 dun, the total enthalpies through E = rho h0.
+// Every rounding is pinned, so each kernel that inlines it gives the same
+// bits; the terms that are ready first are summed first, to shorten the chain
+// behind the speed of sound.  MV: moving face with normal grid speed ubn
+// (src/flux.f90:110-113, 122-189): the normal velocities relative to the
+// face, the energy flux's p ubn and the shifted eigenvalues; the fixed-grid
+// instantiation has none of these terms.
 template <bool MV = false>
 __device__ __forceinline__ void roe_flux_euler(const PhysPar &P, double kx, double ky, double kz, double ds,
                                                const double *qr, const double *ql, double *flux,
                                                double ubn = 0.0) {
-  const double g_gm1 = P.g_gm1, gm1 = P.gm1;
+  auto mul = [](double a, double b) { return __dmul_rn(a, b); };
+  auto add = [](double a, double b) { return __dadd_rn(a, b); };
+  auto sub = [](double a, double b) { return __dsub_rn(a, b); };
+  auto mad = [](double a, double b, double c) { return __fma_rn(a, b, c); };
   const double rhor = qr[0], ur = qr[1], vr = qr[2], wr = qr[3], pr = qr[4];
-  const double unr = MV ? ur * kx + vr * ky + wr * kz - ubn : ur * kx + vr * ky + wr * kz;
-  const double q2r = ur * ur + vr * vr + wr * wr;
-  const double rsr = rsqrt_nr(rhor);  // 1/sqrt(rho_R): sqrt(rho_R) and 1/rho_R from it
-  const double h0r = g_gm1 * pr * (rsr * rsr) + q2r / 2;
   const double rhol = ql[0], ul = ql[1], vl = ql[2], wl = ql[3], pl = ql[4];
-  const double unl = MV ? ul * kx + vl * ky + wl * kz - ubn : ul * kx + vl * ky + wl * kz;
-  const double q2l = ul * ul + vl * vl + wl * wl;
-  const double rsl = rsqrt_nr(rhol);
-  const double h0l = g_gm1 * pl * (rsl * rsl) + q2l / 2;
-  const double drho = rhor - rhol, dp = pr - pl, du = ur - ul, dv = vr - vl, dw = wr - wl;
-  const double dun = unr - unl;
-  const double rhols = rhol * rsl, rhors = rhor * rsr;
-  const double rho = rhols * rhors;
-  const double rden = rcp_nr(rhols + rhors);
-  const double u = (rhols * ul + rhors * ur) * rden;
-  const double v = (rhols * vl + rhors * vr) * rden;
-  const double w = (rhols * wl + rhors * wr) * rden;
-  const double un = u * kx + v * ky + w * kz;
-  const double h0 = (rhols * h0l + rhors * h0r) * rden;
-  const double q2 = u * u + v * v + w * w;
-  const double a2 = gm1 * (h0 - q2 / 2);
-  const double ra = rsqrt_nr(a2);  // 1/a
-  const double a = a2 * ra;
-  double rm123 = MV ? fabs(un - ubn) : fabs(un), rm4 = MV ? fabs(un + a - ubn) : fabs(un + a);
-  double rm5 = MV ? fabs(un - a - ubn) : fabs(un - a);
+  const double rsr = rsqrt_nr(rhor), rsl = rsqrt_nr(rhol);
+  double unr = mad(wr, kz, mad(vr, ky, mul(ur, kx))), unl = mad(wl, kz, mad(vl, ky, mul(ul, kx)));
+  if (MV) { unr = sub(unr, ubn); unl = sub(unl, ubn); }
+  const double er = mad(mul(0.5, rhor), mad(wr, wr, mad(vr, vr, mul(ur, ur))), mul(P.g_gm1, pr));
+  const double el = mad(mul(0.5, rhol), mad(wl, wl, mad(vl, vl, mul(ul, ul))), mul(P.g_gm1, pl));
+  const double du = sub(ur, ul), dv = sub(vr, vl), dw = sub(wr, wl), dun = sub(unr, unl);
+  const double srr = mul(rhor, rsr), srl = mul(rhol, rsl);  // sqrt(rho)
+  const double rden = rcp_nr(add(srl, srr));
+  const double wgt = mul(srr, rden);
+  const double u = mad(wgt, du, ul), v = mad(wgt, dv, vl), w = mad(wgt, dw, wl), un = mad(wgt, dun, unl);
+  const double h0 = mul(mad(er, rsr, mul(el, rsl)), rden);
+  const double q2h = mul(0.5, mad(w, w, mad(v, v, mul(u, u))));
+  const double a2 = mul(P.gm1, sub(h0, q2h));
+  const double ra = rsqrt_nr(a2), a = mul(a2, ra);
+  double rm1 = fabs(un), rm4 = fabs(add(un, a)), rm5 = fabs(sub(un, a));
   if (P.efx_setup_f) {
-    double rdelta = P.cntrpy_f * (P.w1 * P.entfxctf_f + P.w2 * (sqrt(q2) + a) +
-                                  P.w3 * 0.2 * (MV ? fabs(un) + a + fabs(ubn) : fabs(un) + a));
+    double rdelta = P.cntrpy_f * (P.w1 * P.entfxctf_f + P.w2 * (sqrt(2 * q2h) + a) +
+                                  P.w3 * 0.2 * (MV ? fabs(un + ubn) + a + fabs(ubn) : fabs(un) + a));
     rdelta = fmax(rdelta, 1.0e-12);
-    if (rm123 <= rdelta && P.efx_all_f) rm123 = 0.5 * (rm123 * rm123 + rdelta * rdelta) / rdelta;
+    if (rm1 <= rdelta && P.efx_all_f) rm1 = 0.5 * (rm1 * rm1 + rdelta * rdelta) / rdelta;
     if (rm4 <= rdelta) rm4 = 0.5 * (rm4 * rm4 + rdelta * rdelta) / rdelta;
     if (rm5 <= rdelta) rm5 = 0.5 * (rm5 * rm5 + rdelta * rdelta) / rdelta;
   }
   if (P.eig_limit_f) {
-    if (rm123 <= P.eig_cutoff_f) rm123 = P.eig_cutoff_f;
+    if (rm1 <= P.eig_cutoff_f) rm1 = P.eig_cutoff_f;
     if (P.eig_lim_all_f && rm4 <= P.eig_cutoff_f) rm4 = P.eig_cutoff_f;
     if (P.eig_lim_all_f && rm5 <= P.eig_cutoff_f) rm5 = P.eig_cutoff_f;
   }
-  const double dpa2 = dp * (ra * ra), rdua = rho * dun * ra;
-  const double al1 = rm123 * (drho - dpa2);
-  const double al2 = rm123 * rho;
-  const double al3 = rm4 * (dpa2 + rdua) / 2;
-  const double al4 = rm5 * (dpa2 - rdua) / 2;
-  const double df1 = al1 + al3 + al4;
-  const double df2 = al1 * u + al2 * (du - dun * kx) + al3 * (u + a * kx) + al4 * (u - a * kx);
-  const double df3 = al1 * v + al2 * (dv - dun * ky) + al3 * (v + a * ky) + al4 * (v - a * ky);
-  const double df4 = al1 * w + al2 * (dw - dun * kz) + al3 * (w + a * kz) + al4 * (w - a * kz);
-  const double df5 = al1 * (q2 / 2) + al2 * (u * du + v * dv + w * dw - un * dun) + al3 * (h0 + a * un) +
-                     al4 * (h0 - a * un);
-  const double hds = ds / 2;
-  flux[0] = (rhor * unr + rhol * unl - df1) * hds;
-  flux[1] = ((rhor * ur * unr + pr * kx) + (rhol * ul * unl + pl * kx) - df2) * hds;
-  flux[2] = ((rhor * vr * unr + pr * ky) + (rhol * vl * unl + pl * ky) - df3) * hds;
-  flux[3] = ((rhor * wr * unr + pr * kz) + (rhol * wl * unl + pl * kz) - df4) * hds;
-  if (MV) flux[4] = ((rhor * h0r * unr + pr * ubn) + (rhol * h0l * unl + pl * ubn) - df5) * hds;
-  else flux[4] = (rhor * h0r * unr + rhol * h0l * unl - df5) * hds;
-}
-
-// Mixed precision: the central part (fr + fl) in FP64 from the FP64 face
-// states, the Roe dissipation df in FP32 from FP32 copies of the states and
-// of their FP64 differences.  Same algebra as roe_flux_fp64.
-__device__ __forceinline__ void roe_flux_mixed(const PhysPar &P, double kx, double ky, double kz, double ds,
-                                               const double *qr, const double *ql, double *flux) {
-  const double g = P.g;
-  const double rhor = qr[0], ur = qr[1], vr = qr[2], wr = qr[3], pr = qr[4];
-  const double rhol = ql[0], ul = ql[1], vl = ql[2], wl = ql[3], pl = ql[4];
-  const double unr = ur * kx + vr * ky + wr * kz;
-  const double unl = ul * kx + vl * ky + wl * kz;
-  const double q2r = ur * ur + vr * vr + wr * wr;
-  const double q2l = ul * ul + vl * vl + wl * wl;
-  const double h0r = P.g_gm1 * pr * rcp_nr(rhor) + q2r / 2;
-  const double h0l = P.g_gm1 * pl * rcp_nr(rhol) + q2l / 2;
-  // FP32 dissipation on FP64 differences
-  const float fkx = (float)kx, fky = (float)ky, fkz = (float)kz;
-  const float drho = (float)(rhor - rhol), dp = (float)(pr - pl);
-  const float du = (float)(ur - ul), dv = (float)(vr - vl), dw = (float)(wr - wl);
-  const float dun = (float)(unr - unl);
-  const float frl = (float)rhol, frr = (float)rhor;
-  const float rhols = frl * rsqrtf(frl), rhors = frr * rsqrtf(frr);
-  const float rho = rhols * rhors;
-  const float rden = __fdividef(1.0f, rhols + rhors);
-  const float u = (rhols * (float)ul + rhors * (float)ur) * rden;
-  const float v = (rhols * (float)vl + rhors * (float)vr) * rden;
-  const float w = (rhols * (float)wl + rhors * (float)wr) * rden;
-  const float un = u * fkx + v * fky + w * fkz;
-  const float h0 = (rhols * (float)h0l + rhors * (float)h0r) * rden;
-  const float q2 = u * u + v * v + w * w;
-  const float a2 = (float)(g - 1) * (h0 - q2 * 0.5f);
-  const float ria = rsqrtf(a2);
-  const float a = a2 * ria;
-  float rm123 = fabsf(un), rm4 = fabsf(un + a), rm5 = fabsf(un - a);
-  if (P.efx_setup_f) {
-    float rdelta = (float)P.cntrpy_f * ((float)P.w1 * (float)P.entfxctf_f + (float)P.w2 * (sqrtf(q2) + a) +
-                                        (float)P.w3 * 0.2f * (fabsf(un) + a));
-    rdelta = fmaxf(rdelta, 1.0e-12f);
-    if (rm123 <= rdelta && P.efx_all_f) rm123 = 0.5f * (rm123 * rm123 + rdelta * rdelta) / rdelta;
-    if (rm4 <= rdelta) rm4 = 0.5f * (rm4 * rm4 + rdelta * rdelta) / rdelta;
-    if (rm5 <= rdelta) rm5 = 0.5f * (rm5 * rm5 + rdelta * rdelta) / rdelta;
-  }
-  if (P.eig_limit_f) {
-    const float c = (float)P.eig_cutoff_f;
-    if (rm123 <= c) rm123 = c;
-    if (P.eig_lim_all_f && rm4 <= c) rm4 = c;
-    if (P.eig_lim_all_f && rm5 <= c) rm5 = c;
-  }
-  const float ia2 = ria * ria;
-  const float dpa2 = dp * ia2, rdua = rho * dun * ria;
-  const float al1 = rm123 * (drho - dpa2);
-  const float al2 = rm123 * rho;
-  const float al3 = rm4 * (dpa2 + rdua) * 0.5f;
-  const float al4 = rm5 * (dpa2 - rdua) * 0.5f;
-  const float df1 = al1 + al3 + al4;
-  const float df2 = al1 * u + al2 * (du - dun * fkx) + al3 * (u + a * fkx) + al4 * (u - a * fkx);
-  const float df3 = al1 * v + al2 * (dv - dun * fky) + al3 * (v + a * fky) + al4 * (v - a * fky);
-  const float df4 = al1 * w + al2 * (dw - dun * fkz) + al3 * (w + a * fkz) + al4 * (w - a * fkz);
-  const float df5 = al1 * (q2 * 0.5f) + al2 * (u * du + v * dv + w * dw - un * dun) + al3 * (h0 + a * un) +
-                    al4 * (h0 - a * un);
-  const double hds = 0.5 * ds;
-  flux[0] = (rhor * unr + rhol * unl - (double)df1) * hds;
-  flux[1] = ((rhor * ur * unr + pr * kx) + (rhol * ul * unl + pl * kx) - (double)df2) * hds;
-  flux[2] = ((rhor * vr * unr + pr * ky) + (rhol * vl * unl + pl * ky) - (double)df3) * hds;
-  flux[3] = ((rhor * wr * unr + pr * kz) + (rhol * wl * unl + pl * kz) - (double)df4) * hds;
-  flux[4] = (rhor * h0r * unr + rhol * h0l * unl - (double)df5) * hds;
+  const double dpa2 = mul(sub(pr, pl), mul(ra, ra)), rdua = mul(mul(mul(srl, srr), dun), ra);
+  const double al1 = mul(rm1, sub(sub(rhor, rhol), dpa2)), al2 = mul(rm1, mul(srl, srr));
+  const double al3 = mul(mul(0.5, rm4), add(dpa2, rdua)), al4 = mul(mul(0.5, rm5), sub(dpa2, rdua));
+  const double a34 = add(al3, al4), df1 = add(al1, a34);
+  const double c2 = mad(-al2, dun, mul(a, sub(al3, al4)));
+  const double mr = mul(rhor, unr), ml = mul(rhol, unl);
+  const double hds = mul(0.5, ds);
+  // the momentum rows keep the reference's sums of the large terms (each
+  // side's convective and pressure flux, then both, then the dissipation):
+  // with the pressures added first their common rounding costs a fifth more
+  // error, and five times more difference to the reference on thin cells
+  auto mom = [&](double xr, double xl, double xa, double dx, double k) {
+    const double f = add(mad(mr, xr, mul(pr, k)), mad(ml, xl, mul(pl, k)));
+    return mul(sub(f, mad(df1, xa, mad(al2, dx, mul(c2, k)))), hds);
+  };
+  flux[0] = mul(sub(add(mr, ml), df1), hds);
+  flux[1] = mom(ur, ul, u, du, kx);
+  flux[2] = mom(vr, vl, v, dv, ky);
+  flux[3] = mom(wr, wl, w, dw, kz);
+  const double udu = mad(w, dw, mad(v, dv, mul(u, du)));
+  double fe = mad(er, unr, mul(el, unl));
+  if (MV) fe = mad(add(pr, pl), ubn, fe);
+  const double una = MV ? add(un, ubn) : un;
+  flux[4] = mul(mad(-c2, una, mad(-a34, h0, mad(-al1, q2h, mad(-al2, udu, fe)))), hds);
 }
 
 // roflux_b's mean-flow flux with the turbulent kinetic energy terms

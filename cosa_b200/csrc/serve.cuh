@@ -7,13 +7,13 @@
 // n3 slots in every pool (its P2 and P1 arrays are smaller than its P3 one,
 // so they fit the same range).  The active solves' blocks, placed at their
 // pool offsets, form one merged level of the engine's context: one k_halo and
-// one k_stage_tile launch per RK stage cover every tile of every solve.
+// one face and one cell launch per RK stage cover every solve.
 // Flow conditions (free stream, inlet total state, outlet pressure) differ
 // per solve and reach k_halo through a per-item parameter slot; the scheme
 // (gamma, limiter, CFL, RK coefficients) is the engine's.
 //
 // Each solve's arithmetic touches only its own cells, its residual norm is
-// reduced over its own tiles in a fixed order, and it is checked for
+// reduced over its own blocks' rows in a fixed order, and it is checked for
 // convergence every check_every of its own iterations: a solve gives the
 // same result alone and among others.  The convergence test is the
 // residual drop rms / rms(first iteration) < tol on the total norm.
@@ -36,7 +36,6 @@ struct ServeSolve {
   int max_iter = 0;
   int64_t n3 = 0, n2 = 0, n1 = 0, off = -1, ncell = 0;
   std::vector<int64_t> lop;         // per block: local P3, P2, P1 offsets
-  int64_t ntiles = 0;
   int iters = 0;
   double rms0 = 0, rms = 0;
   double t_submit = 0, t_admit = 0, t_done = 0;
@@ -129,7 +128,8 @@ void pool_free(cosa_serve *e, int64_t off, int64_t n) {
 
 // the device tables of a level built by build_level, released before a rebuild
 void free_level_tables(cosa_ctx *c, LevelState &L) {
-  void *owned[] = {L.d_blocks, L.d_bct, L.d_items, L.d_strong, L.d_smap, L.d_tiles};
+  void *owned[] = {L.d_blocks, L.d_bct, L.d_items, L.d_strong, L.d_smap, L.d_walls,
+                   L.d_cutx, L.d_cutv, L.d_ftasks, L.d_cflux};
   for (void *v : owned) {
     if (!v) continue;
     cudaFree(v);
@@ -140,11 +140,6 @@ void free_level_tables(cosa_ctx *c, LevelState &L) {
   L = LevelState{};
   L.d_part = part;
   L.npart_cap = cap;
-}
-
-int64_t tiles_of(const int32_t *d) {
-  const int64_t ni = d[0] - 1, nj = d[1] - 1, nk = d[2] - 1;
-  return ((nk + 31) / 32) * ((nj + kTJ - 1) / kTJ) * ((ni + kTI - 1) / kTI);
 }
 
 // merged level of the active solves at their pool offsets
@@ -162,7 +157,6 @@ int serve_rebuild(cosa_serve *e) {
   std::vector<int> seg;
   std::vector<double> segn, cflb;
   int nb = 0;
-  int64_t tile0 = 0;
   for (int a = 0; a < na; ++a) {
     const ServeSolve &s = e->solves[(size_t)e->active[a]];
     dims.insert(dims.end(), s.dims.begin(), s.dims.end());
@@ -182,16 +176,14 @@ int serve_rebuild(cosa_serve *e) {
       bps.push_back(a);
       cflb.push_back(s.flow.cfl > 0 ? s.flow.cfl : c->p.cfl);
     }
-    seg.push_back((int)tile0);
-    seg.push_back((int)s.ntiles);
+    seg.push_back(nb * kCellsGX);
+    seg.push_back(s.nb * kCellsGX);
     segn.push_back((double)s.ncell);
-    tile0 += s.ntiles;
     nb += s.nb;
   }
   cosa_level_desc d{nb, dims.data(), nbcs.data(), bct.data(), (int32_t)(cut.size() / 21), cut.data()};
   int r = build_level(c, L, d, offs.data(), bps.data());
   if (r) return r;
-  if (L.ntiles != tile0) return COSA_ERR_ARG;
   // per-solve flow conditions on the scheme's parameters
   if (e->ps_cap < na) {
     if (e->d_ps) { cudaFree(e->d_ps); e->d_ps = nullptr; }
@@ -219,12 +211,17 @@ int serve_rebuild(cosa_serve *e) {
   CK(cudaMemcpyAsync(c->d_seg, seg.data(), seg.size() * sizeof(int), cudaMemcpyHostToDevice, c->s));
   CK(cudaMemcpyAsync(c->d_seg_ncell, segn.data(), segn.size() * sizeof(double), cudaMemcpyHostToDevice, c->s));
   c->nseg = na;
-  if (L.npart_cap < L.ntiles) {
+  const int rows = nb * kCellsGX + kRmsMid;
+  if (L.npart_cap < rows) {
     if (L.d_part) cudaFree(L.d_part);
     L.d_part = nullptr;
-    CK(cudaMalloc(&L.d_part, (size_t)L.ntiles * 8 * sizeof(double)));
-    L.npart_cap = L.ntiles;
+    CK(cudaMalloc(&L.d_part, (size_t)rows * 8 * sizeof(double)));
+    L.npart_cap = rows;
   }
+  // the store schedule for every active set: its norms' partial rows belong
+  // to one block each, so a solve's do not depend on the others
+  L.schedule = 0;
+  if ((r = ensure_faces(c, L))) return r;
   L.ptrs = cosa_level_ptrs{};
   L.ptrs.q = e->Q; L.ptrs.qold = e->QO; L.ptrs.dtvol = e->DT;
   L.ptrs.si = e->SI; L.ptrs.sj = e->SJ; L.ptrs.sk = e->SK; L.ptrs.vol = e->VOL;
@@ -398,7 +395,6 @@ int cosa_serve_submit(cosa_serve *e, const cosa_level_desc *grid, const double *
     s.n2 += (im + 2) * (jm + 2) * (km + 2);
     s.n1 += (im + 1) * (jm + 1) * (km + 1);
     s.ncell += (im - 1) * (jm - 1) * (km - 1);
-    s.ntiles += tiles_of(s.dims.data() + 3 * b);
   }
   if (s.n3 > e->cap) return COSA_ERR_ARG;  // can never be admitted
   s.x.assign(x, x + s.n2);

@@ -320,8 +320,8 @@ class Context:
         return list(ms), list(cnt)
 
     def autotune(self, nl=1, niter=5):
-        """Time the fused-tile and face-split stage schedules on level nl and
-        keep the faster; returns (ms_tile, ms_split, choice)."""
+        """Time the store (0) and chain (1) stage schedules on level nl and
+        keep the faster; returns (ms_store, ms_chain, choice)."""
         ms = (C.c_double * 2)()
         ch = C.c_int32()
         self._check(load().cosa_gpu_autotune(self.h, nl, niter, ms, C.byref(ch)), "autotune")

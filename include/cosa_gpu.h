@@ -550,16 +550,18 @@ int cosa_gpu_smooth_level(cosa_ctx *ctx, int32_t nl, int32_t niter, int32_t from
 int cosa_gpu_mg(cosa_ctx *ctx, int32_t mgit0, int32_t ncycles, int32_t ncycle,
                 int32_t rms_every, double *hist);
 /* stage-schedule autotuner (no reference counterpart): times niter
-   iterations of level nl with the fused tile kernel (schedule 0) and with
-   the face-split schedule (1: face fluxes through HBM, then a cell pass),
-   keeps the faster for the level and returns the ms per iteration of each;
-   the level's state is restored afterwards.  set_schedule forces one. */
+   iterations of level nl with the store schedule (0: all face fluxes in one
+   launch and to memory, then a cell pass) and with the chain schedule (1: the
+   three families one after another, each adding its flux differences to the
+   cell's running balance), ms[0] and ms[1] per iteration, and keeps the
+   faster (*choice); the level's state is restored afterwards.  Without it a
+   level takes store or chain by its size.  set_schedule forces one. */
 int cosa_gpu_autotune(cosa_ctx *ctx, int32_t nl, int32_t niter, double ms[2], int32_t *choice);
 int cosa_gpu_set_schedule(cosa_ctx *ctx, int32_t nl, int32_t schedule);
 /* niter fused iterations without graphs, with CUDA events around every
    kernel: ms[0] = mean halo-kernel time, ms[1] = mean time of the main
-   kernel (k_stage_tile, or k_faces under the split schedule), ms[2] = mean
-   iteration time, ms[3] = mean k_cells time (split schedule);
+   kernels (of one stage), ms[2] = mean iteration time, ms[3] = mean k_cells
+   time (store schedule);
    counts = launches timed */
 int cosa_gpu_profile(cosa_ctx *ctx, int32_t nl, int32_t niter, double ms[4],
                      int64_t counts[4]);
@@ -608,7 +610,7 @@ int cosa_gpu_resg_rms_noalloc(int32_t nblocks, const int32_t *dims, int32_t npde
  * tables, node coordinates in the P2 layout, initial P3 state, flow
  * conditions) wait in a first-come queue, are admitted when their arrays fit
  * in the pools, are advanced together (every RK stage of every active solve
- * in the same halo and tile launches) and retire when their total residual
+ * in the same halo, face and cell launches) and retire when their total residual
  * norm falls below tol times its first-iteration value (checked every
  * check_every of their own iterations) or after max_iter iterations.  The
  * scheme (gamma, limiter, RK coefficients, and the CFL number unless the

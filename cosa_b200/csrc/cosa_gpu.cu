@@ -21,6 +21,7 @@
 #include "split.cuh"
 #include "moving.cuh"
 #include "force.cuh"
+#include "irs.cuh"
 #include "unsteady.cuh"
 #include "lsp.cuh"
 
@@ -57,7 +58,7 @@ struct LevelState {
   double *d_part = nullptr;   // partial sums of the norms (8 doubles each)
   double *d_res = nullptr;    // residual of the IRS path (P3, zero halos)
   double *d_ores = nullptr;   // right-hand side copy of the cut-aware IRS
-  double *d_irs_scr = nullptr;  // tridiagonal pivots, 2 doubles per P3 cell and snapshot
+  double *d_irs_scr = nullptr;  // lines too long for shared memory: their pivots, 2 doubles per P3 cell and snapshot
   double *d_beta[3] = {nullptr, nullptr, nullptr};  // IRS coefficients when not bound
   int npart_cap = 0;
   cudaGraphExec_t graph[2] = {nullptr, nullptr};  // iteration without / with rms
@@ -134,6 +135,9 @@ struct cosa_ctx {
   cudaStream_t s = nullptr;
   int nlevels = 0;
   LevelState L[COSA_MAX_LEVELS];
+  double2 *d_piv = nullptr;  // IRS with a constant coefficient: pivots (k_irs_pivots) of piv_n rows for piv_eps
+  int piv_n = 0;
+  double piv_eps = 0.0;
   int *d_status = nullptr;
   int *d_row = nullptr;
   double *d_hist = nullptr;
@@ -636,11 +640,57 @@ int check_thin_blocks(const cosa_ctx *c, int nl) {
   return COSA_OK;
 }
 
+// shared memory that k_irs_tri may take; lines that do not fit it eight at a
+// time (of more than some 1000 to 3000 cells) are swept through global memory
+// by k_irs_line
+constexpr int kIrsSmem = 200 * 1024;
+int irs_max_line(const LevelState &L) {
+  int n = 1;
+  for (const DevBlock &x : L.hb) n = std::max({n, x.im - 1, x.jm - 1, x.km - 1});
+  return n;
+}
+// lines per warp that fit (0: none)
+int irs_group(int nmax, bool const_eps, bool scaled) {
+  for (int gw = 32; gw >= 8; gw /= 2)
+    if (irs_warp_doubles(nmax, gw, const_eps, scaled) * (int)sizeof(double) <= kIrsSmem) return gw;
+  return 0;
+}
+bool irs_fits(const LevelState &L, bool const_eps) { return irs_group(irs_max_line(L), const_eps, true) > 0; }
+double irs_eps(const cosa_params &p) { return 0.25 * (p.rat * p.rat - 1.0); }
+
+// once per process; contexts driven from several host threads (the serving
+// engine's context lane) may reach it together
+int irs_smem_attrs() {
+  static std::mutex mu;
+  static bool done = false;
+  std::lock_guard<std::mutex> lock(mu);
+  if (done) return COSA_OK;
+  for (auto k : {k_irs_tri<1, true>, k_irs_tri<2, true>, k_irs_tri<3, true>, k_irs_tri<1, false>, k_irs_tri<2, false>,
+                 k_irs_tri<3, false>})
+    CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kIrsSmem));
+  done = true;
+  return COSA_OK;
+}
+
+void drop_graphs(cosa_ctx *c);
 int ensure_irs_scratch(cosa_ctx *c, LevelState &L) {
   const int S = 2 * c->p.nharms + 1;
   const size_t n = (size_t)L.n3 * c->p.npde * S;
-  int r = 0;
-  if (!L.d_irs_scr && (r = dalloc(c, &L.d_irs_scr, (size_t)L.n3 * S * 2))) return r;
+  int r = irs_smem_attrs();
+  if (r) return r;
+  const int len = irs_max_line(L);
+  if (c->piv_n < len) {
+    drop_graphs(c);
+    if ((r = dalloc(c, &c->d_piv, (size_t)len))) return r;
+    c->piv_n = len;
+    c->piv_eps = -1.0;
+  }
+  if (c->piv_eps != irs_eps(c->p)) {
+    c->piv_eps = irs_eps(c->p);
+    k_irs_pivots<<<1, 32, 0, c->s>>>(c->piv_n, c->piv_eps, c->d_piv);
+    if ((r = after_launch(c))) return r;
+  }
+  if (!irs_fits(L, false) && !L.d_irs_scr && (r = dalloc(c, &L.d_irs_scr, (size_t)L.n3 * S * 2))) return r;
   if (!L.d_res) {
     if ((r = dalloc(c, &L.d_res, n))) return r;
     CK(cudaMemset(L.d_res, 0, n * sizeof(double)));
@@ -651,85 +701,61 @@ int ensure_irs_scratch(cosa_ctx *c, LevelState &L) {
   return COSA_OK;
 }
 
-// lines of kPcrMinLen..kPcrMaxLen cells are solved by cyclic reduction in
-// shared memory (at most kPcrSmemBytes per CTA, within the 48 KB default);
-// shorter lines (a warp per line would idle) and longer ones by the Thomas
-// sweeps, one thread per line
-constexpr int kPcrSmemBytes = 48 * 1024;
-constexpr int kPcrMaxLen = kPcrSmemBytes / 64;
-constexpr int kPcrMinLen = 16;
-
-// the three line sweeps of cirs_b / ccirs_b on `res` for variables vs..ve
-int irs_sweeps(cosa_ctx *c, LevelState &L, double *res, const double *ores, const double *const beta[3], double eps,
-               int vs, int ve, int with_halo) {
+// the three line sweeps of cirs_b / ccirs_b on `res` for variables vs..ve;
+// beta null: the constant coefficient irs_eps.  fin / fint: dt/V (mean flow /
+// turbulence) multiplied in by the first direction and divided out by the
+// last (only where irs_fits), or null
+int irs_sweeps(cosa_ctx *c, LevelState &L, double *res, const double *ores, const double *const beta[3],
+               int vs, int ve, int with_halo, const double *f = nullptr, const double *ft = nullptr) {
   // blocks are independent here (each sweep writes its own block's interior,
-  // halos were filled before), so a direction can run for all blocks at once
+  // halos were filled before), so a direction runs for all blocks at once
   const int S = 2 * c->p.nharms + 1, npde = c->p.npde, nv = ve - vs + 1;
+  const double eps = irs_eps(c->p);
+  const bool tri = irs_fits(L, !beta);
+  const BlockList bl{L.d_blocks};
   for (int d = 1; d <= 3; ++d) {
     const double *bt = beta ? beta[d - 1] : nullptr;
     const double *src = d == 1 ? ores : nullptr;
-    auto len_of = [&](const DevBlock &x) { return d == 1 ? x.im - 1 : (d == 2 ? x.jm - 1 : x.km - 1); };
-    auto lines_of = [&](const DevBlock &x) {
-      return d == 1 ? (int64_t)(x.jm - 1) * (x.km - 1)
-                    : (d == 2 ? (int64_t)(x.im - 1) * (x.km - 1) : (int64_t)(x.im - 1) * (x.jm - 1));
-    };
-    bool all_pcr = true;
-    int nmax = 1;
-    int64_t wmax = 1;
-    for (const DevBlock &x : L.hb) {
-      const int len = len_of(x);
-      all_pcr &= len >= kPcrMinLen && len <= kPcrMaxLen;
-      nmax = std::max(nmax, len);
-      wmax = std::max<int64_t>(wmax, lines_of(x) * S * nv);
-    }
-    if (all_pcr) {
-      // parallel cyclic reduction, one warp per line and variable, all blocks
-      const int wpc = std::max(1, std::min(4, kPcrSmemBytes / (64 * nmax)));
-      const dim3 g((unsigned)grid_x(wmax * 32, L.nb) * 256 / (32 * wpc) + 1, L.nb);
-      const size_t sm = (size_t)wpc * 8 * nmax * sizeof(double);
-      const BlockList bl{L.d_blocks};
-      if (d == 1) k_irs_pcr<1><<<g, 32 * wpc, sm, c->s>>>(bl, npde, S, res, src, bt, eps, vs, ve, with_halo, nmax);
-      else if (d == 2) k_irs_pcr<2><<<g, 32 * wpc, sm, c->s>>>(bl, npde, S, res, src, bt, eps, vs, ve, with_halo, nmax);
-      else k_irs_pcr<3><<<g, 32 * wpc, sm, c->s>>>(bl, npde, S, res, src, bt, eps, vs, ve, with_halo, nmax);
-      const int r = after_launch(c);
-      if (r) return r;
-      continue;
-    }
-    bool all_thomas = true;
-    for (const DevBlock &x : L.hb) all_thomas &= !(len_of(x) >= kPcrMinLen && len_of(x) <= kPcrMaxLen);
-    if (all_thomas) {
-      // Thomas sweeps, one thread per line, all blocks in one launch
-      int64_t lmax = 1;
-      for (const DevBlock &x : L.hb) lmax = std::max<int64_t>(lmax, lines_of(x) * S);
-      const dim3 g(grid_x(lmax, L.nb) * 2, L.nb);  // 128-thread CTAs
-      const BlockList bl{L.d_blocks};
-      if (d == 1) k_irs_line<1><<<g, 128, 0, c->s>>>(bl, npde, S, res, src, bt, eps, vs, ve, with_halo, L.d_irs_scr);
-      else if (d == 2) k_irs_line<2><<<g, 128, 0, c->s>>>(bl, npde, S, res, src, bt, eps, vs, ve, with_halo, L.d_irs_scr);
-      else k_irs_line<3><<<g, 128, 0, c->s>>>(bl, npde, S, res, src, bt, eps, vs, ve, with_halo, L.d_irs_scr);
-      const int r = after_launch(c);
-      if (r) return r;
-      continue;
-    }
-    for (const DevBlock &x : L.hb) {
-      const int len = len_of(x);
-      const int64_t nl = lines_of(x);
-      if (len >= kPcrMinLen && len <= kPcrMaxLen) {
-        const int nm = std::max(len, 1);
-        const int wpc = std::max(1, std::min(4, kPcrSmemBytes / (64 * nm)));
-        const int g = grid_for(nl * S * nv * 32, 32 * wpc);  // one warp per line and variable
-        const size_t sm = (size_t)wpc * 8 * nm * sizeof(double);
-        if (d == 1) k_irs_pcr<1><<<g, 32 * wpc, sm, c->s>>>(x, npde, S, res, src, bt, eps, vs, ve, with_halo, nm);
-        else if (d == 2) k_irs_pcr<2><<<g, 32 * wpc, sm, c->s>>>(x, npde, S, res, src, bt, eps, vs, ve, with_halo, nm);
-        else k_irs_pcr<3><<<g, 32 * wpc, sm, c->s>>>(x, npde, S, res, src, bt, eps, vs, ve, with_halo, nm);
-      } else {
-        const int g = grid_for(nl * S, 128);
-        if (d == 1) k_irs_line<1><<<g, 128, 0, c->s>>>(x, npde, S, res, src, bt, eps, vs, ve, with_halo, L.d_irs_scr);
-        else if (d == 2) k_irs_line<2><<<g, 128, 0, c->s>>>(x, npde, S, res, src, bt, eps, vs, ve, with_halo, L.d_irs_scr);
-        else k_irs_line<3><<<g, 128, 0, c->s>>>(x, npde, S, res, src, bt, eps, vs, ve, with_halo, L.d_irs_scr);
+    if (tri) {
+      int nmax = 1;
+      int64_t wmax = 1;
+      for (const DevBlock &x : L.hb) {
+        nmax = std::max(nmax, (d == 1 ? x.im : d == 2 ? x.jm : x.km) - 1);
       }
-      const int r = after_launch(c);
-      if (r) return r;
+      // narrower groups while the launch has fewer than eight warps per SM
+      int gw = irs_group(nmax, !bt, d == 1 && f);
+      for (;; gw /= 2) {
+        int64_t all = 0;
+        wmax = 1;
+        for (const DevBlock &x : L.hb) {
+          const int64_t g = d == 1 ? ((int64_t)(x.jm - 1) * (x.km - 1) + gw - 1) / gw
+                                   : (int64_t)((x.im + gw - 2) / gw) * ((d == 2 ? x.km : x.jm) - 1);
+          wmax = std::max<int64_t>(wmax, g * S * nv);
+          all += g * S * nv;
+        }
+        if (gw <= 8 || all >= 148 * 8) break;
+      }
+      // warps per CTA: up to 4 within 24 KB, so that short lines do not make
+      // thousands of one-warp CTAs
+      const int per = irs_warp_doubles(nmax, gw, !bt, d == 1 && f) * (int)sizeof(double);
+      const int wpc = std::max(1, std::min(4, 24 * 1024 / per));
+      const dim3 g((unsigned)std::min<int64_t>((wmax + wpc - 1) / wpc, 148 * 64), L.nb);
+      auto k = bt ? (d == 1 ? k_irs_tri<1, false> : d == 2 ? k_irs_tri<2, false> : k_irs_tri<3, false>)
+                  : (d == 1 ? k_irs_tri<1, true> : d == 2 ? k_irs_tri<2, true> : k_irs_tri<3, true>);
+      k<<<g, 32 * wpc, (size_t)per * wpc, c->s>>>(bl, npde, S, res, src, bt, c->d_piv, eps, vs, ve, with_halo, nmax, gw,
+                                                  d == 1 ? f : nullptr, d == 1 ? ft : nullptr, d == 3 ? f : nullptr,
+                                                  d == 3 ? ft : nullptr);
+    } else {
+      // Thomas sweeps through global memory, one thread per line
+      int64_t lmax = 1;
+      for (const DevBlock &x : L.hb)
+        lmax = std::max<int64_t>(lmax, (int64_t)(d == 1 ? x.jm : x.im) * (d == 3 ? x.jm : x.km) * S);
+      const dim3 g(grid_x(lmax, L.nb) * 2, L.nb);  // 128-thread CTAs
+      auto k = d == 1 ? k_irs_line<1> : d == 2 ? k_irs_line<2> : k_irs_line<3>;
+      k<<<g, 128, 0, c->s>>>(bl, npde, S, res, src, bt, eps, vs, ve, with_halo, L.d_irs_scr);
     }
+    const int r = after_launch(c);
+    if (r) return r;
   }
   return COSA_OK;
 }
@@ -748,20 +774,21 @@ int irs_scale(cosa_ctx *c, LevelState &L, double *res, const double *dtv, const 
 int irs_apply(cosa_ctx *c, LevelState &L, double *res, double *ores, const double *dtv, const double *const beta[3],
               const double *dtvt = nullptr, const double *const tbeta[3] = nullptr) {
   const cosa_params &p = c->p;
-  const double eps = 0.25 * (p.rat * p.rat - 1.0);
   const bool const_eps = p.irsop == 1;
   const bool kom = p.npde > 5;
   const int S = 2 * p.nharms + 1;
-  auto sweeps = [&](const double *src, int with_halo) -> int {
-    if (const_eps) return irs_sweeps(c, L, res, src, nullptr, eps, 1, p.npde, with_halo);
-    int r2 = irs_sweeps(c, L, res, src, beta, eps, 1, 5, with_halo);
-    if (!r2 && kom) r2 = irs_sweeps(c, L, res, src, tbeta, 0.0, 6, p.npde, with_halo);
+  auto sweeps = [&](const double *src, int with_halo, const double *f, const double *ft) -> int {
+    if (const_eps) return irs_sweeps(c, L, res, src, nullptr, 1, p.npde, with_halo, f, ft);
+    int r2 = irs_sweeps(c, L, res, src, beta, 1, 5, with_halo, f, ft);
+    if (!r2 && kom) r2 = irs_sweeps(c, L, res, src, tbeta, 6, p.npde, with_halo, f, ft);
     return r2;
   };
-  int r = irs_scale(c, L, res, dtv, kom ? dtvt : nullptr, 1);
-  if (r) return r;
+  int r = 0;
+  // one pass over the directions: they scale on the way in and out
+  if (p.cutcirs == 0 && irs_fits(L, const_eps)) return sweeps(nullptr, 0, dtv, kom ? dtvt : nullptr);
+  if ((r = irs_scale(c, L, res, dtv, kom ? dtvt : nullptr, 1))) return r;
   if (p.cutcirs == 0) {
-    if ((r = sweeps(nullptr, 0))) return r;
+    if ((r = sweeps(nullptr, 0, nullptr, nullptr))) return r;
   } else {
     CK(cudaMemcpyAsync(ores, res, (size_t)L.n3 * p.npde * S * sizeof(double), cudaMemcpyDeviceToDevice, c->s));
     const int ncut = (int)L.items.size() - L.n_bc_items;
@@ -770,7 +797,7 @@ int irs_apply(cosa_ctx *c, LevelState &L, double *res, double *ores, const doubl
         if ((r = launch_halo<false>(c, L, L.d_items + L.n_bc_items, ncut, res, nullptr, nullptr, nullptr, nullptr, kNoFaceVel)))
           return r;
       }
-      if ((r = sweeps(ores, 1))) return r;
+      if ((r = sweeps(ores, 1, nullptr, nullptr))) return r;
     }
   }
   return irs_scale(c, L, res, dtv, kom ? dtvt : nullptr, 0);
@@ -1078,12 +1105,9 @@ int launch_iteration(cosa_ctx *c, int nl, LevelState &L, const IterOpts &o) {
                                              ar, sir);
         });
       } else {
-        for (int b = 0; b < L.nb && !r; ++b) {
-          const DevBlock &x = L.hb[b];
-          k_update_stage<<<grid_for((int64_t)(x.im - 1) * (x.jm - 1) * (x.km - 1)), 256, 0, c->s>>>(
-              x, p.npde, 1, L.d_res, qold, qout, qcopy, L.ptrs.dtvol, ar);
-          r = after_launch(c);
-        }
+        r = for_blocks(c, L, cnt_cells, [&](auto b, dim3 g) {
+          k_update_stage<<<g, 256, 0, c->s>>>(b, p.npde, 1, L.d_res, qold, qout, qcopy, L.ptrs.dtvol, ar);
+        });
       }
       if (r) return r;
     }
@@ -1175,12 +1199,10 @@ int launch_iteration(cosa_ctx *c, int nl, LevelState &L, const IterOpts &o) {
                                L.ptrs.betaeta ? L.ptrs.betaeta : L.d_beta[1],
                                L.ptrs.betazeta ? L.ptrs.betazeta : L.d_beta[2]};
       if ((r = irs_apply(c, L, L.d_res, L.d_ores, L.ptrs.dtvol, beta))) return r;
-      for (int b = 0; b < L.nb; ++b) {
-        const DevBlock &x = L.hb[b];
-        k_update_stage<<<grid_for((int64_t)(x.im - 1) * (x.jm - 1) * (x.km - 1) * S), 256, 0, c->s>>>(
-            x, p.npde, S, L.d_res, qold, qout, qcopy, L.ptrs.dtvol, p.alphas[irk - 1]);
-        if ((r = after_launch(c))) return r;
-      }
+      r = for_blocks(c, L, cnt_cells, [&](auto b, dim3 g) {
+        k_update_stage<<<g, 256, 0, c->s>>>(b, p.npde, S, L.d_res, qold, qout, qcopy, L.ptrs.dtvol, p.alphas[irk - 1]);
+      });
+      if (r) return r;
     }
   }
   if (p.nstage % 2 == 1) {
@@ -1772,9 +1794,8 @@ int cosa_gpu_cirs(cosa_ctx *c, int32_t nl, double *res, const double *dtvol, con
   if (r) return r;
   const double *beta[3] = {betaxi, betaeta, betazeta};
   if (c->p.irsop >= 2 && (!betaxi || !betaeta || !betazeta)) return COSA_ERR_ARG;
-  const double eps = 0.25 * (c->p.rat * c->p.rat - 1.0);
   if ((r = irs_scale(c, *L, res, dtvol, nullptr, 1))) return r;
-  if ((r = irs_sweeps(c, *L, res, nullptr, c->p.irsop == 1 ? nullptr : beta, eps, 1, 5, 0))) return r;
+  if ((r = irs_sweeps(c, *L, res, nullptr, c->p.irsop == 1 ? nullptr : beta, 1, 5, 0))) return r;
   return irs_scale(c, *L, res, dtvol, nullptr, 0);
 }
 
@@ -1787,8 +1808,7 @@ int cosa_gpu_ccirs(cosa_ctx *c, int32_t nl, double *res, const double *ores, con
   if (r) return r;
   const double *beta[3] = {betaxi, betaeta, betazeta};
   if (c->p.irsop >= 2 && (!betaxi || !betaeta || !betazeta)) return COSA_ERR_ARG;
-  const double eps = 0.25 * (c->p.rat * c->p.rat - 1.0);
-  return irs_sweeps(c, *L, res, ores, c->p.irsop == 1 ? nullptr : beta, eps, 1, 5, 1);
+  return irs_sweeps(c, *L, res, ores, c->p.irsop == 1 ? nullptr : beta, 1, 5, 1);
 }
 
 int cosa_gpu_imetrix(cosa_ctx *c, int32_t nl, const double *x, const double *y, const double *z, double *si,

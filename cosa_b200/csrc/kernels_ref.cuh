@@ -599,8 +599,8 @@ __global__ void k_irs_scale(BS bs_, int npde, int S, double *__restrict__ res, c
 // so they are computed once into `scr` (2 doubles per cell) and reused for
 // each variable.  ores (if set) is the right-hand side of the i sweep of the
 // cut variant; with_halo adds eps * res(halo) on the first and last rows.
-template <int D, class BS>
-__global__ void k_irs_line(BS bs_, int npde, int S, double *__restrict__ res, const double *__restrict__ ores,
+template <int D>
+__global__ void k_irs_line(BlockList bs_, int npde, int S, double *__restrict__ res, const double *__restrict__ ores,
                            const double *__restrict__ beta, double eps, int vs, int ve, int with_halo,
                            double *__restrict__ scr) {
   const DevBlock b = bs_.get();
@@ -674,95 +674,12 @@ __global__ void k_irs_line(BS bs_, int npde, int S, double *__restrict__ res, co
   }
 }
 
-// The same line solves by parallel cyclic reduction: one warp per (line,
-// snapshot, variable), the line's four diagonals/right-hand side in shared
-// memory (ping-pong, 8 * nmax doubles per warp).  Row m of the system is
-// -e_m x_{m-1} + (1 + 2 e_m) x_m - e_m x_{m+1} = r_m (first and last rows
-// without the outer term), as in the Thomas sweeps above; step s eliminates
-// x_{m-s} and x_{m+s} from row m, so after ceil(log2 len) steps x_m = r_m /
-// b_m.  The chain of dependent steps is log2(len) instead of 2 len; the
-// result differs from the Thomas sweeps by rounding only (the matrix is
-// strictly diagonally dominant).
-template <int D, class BS>
-__global__ void __launch_bounds__(128) k_irs_pcr(BS bs_, int npde, int S, double *__restrict__ res,
-                                                 const double *__restrict__ ores, const double *__restrict__ beta,
-                                                 double eps, int vs, int ve, int with_halo, int nmax) {
-  const DevBlock b = bs_.get();
-  extern __shared__ double irs_sm[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  const int im = b.im - 1, jm = b.jm - 1, km = b.km - 1;
-  const int len = D == 1 ? im : (D == 2 ? jm : km);
-  const int n2 = D == 1 ? jm : im, n3 = D == 3 ? jm : km;
-  const int nv = ve - vs + 1;
-  const int64_t nwork = (int64_t)n2 * n3 * S * nv;
-  double *buf = irs_sm + (size_t)warp * 8 * nmax;
-  for (int64_t w = blockIdx.x * (int64_t)nw + warp; w < nwork; w += (int64_t)gridDim.x * nw) {
-    int64_t r_ = w;
-    const int t2 = (int)(r_ % n2) + 1; r_ /= n2;
-    const int t3 = (int)(r_ % n3) + 1; r_ /= n3;
-    const int s = (int)(r_ % S); r_ /= S;
-    const int v = vs + (int)r_;
-    auto cell = [&](int m) {
-      if (D == 1) return p3_cell(b, m, t2, t3);
-      if (D == 2) return p3_cell(b, t2, m, t3);
-      return p3_cell(b, t2, t3, m);
-    };
-    auto coef = [&](int m) {
-      if (!beta) return eps;
-      if (D == 1) return beta[p1_idx(b, S, m, t2, t3, s)];
-      if (D == 2) return beta[p1_idx(b, S, t2, m, t3, s)];
-      return beta[p1_idx(b, S, t2, t3, m, s)];
-    };
-    const int64_t base = p3_var(b, npde, S, v, s);
-    const double *src = ores ? ores + base : res + base;
-    double *x = res + base;
-    double *a0 = buf, *b0 = buf + nmax, *c0 = buf + 2 * nmax, *r0 = buf + 3 * nmax;
-    double *a1 = buf + 4 * nmax, *b1 = buf + 5 * nmax, *c1 = buf + 6 * nmax, *r1 = buf + 7 * nmax;
-    for (int m = lane + 1; m <= len; m += 32) {
-      const double e = coef(m);
-      double rhs = src[cell(m)];
-      if (with_halo && (m == 1 || m == len)) rhs = src[cell(m)] + e * x[cell(m == len ? len + 1 : 0)];
-      a0[m - 1] = m == 1 ? 0.0 : -e;
-      b0[m - 1] = 1 + 2 * e;
-      c0[m - 1] = m == len ? 0.0 : -e;
-      r0[m - 1] = rhs;
-    }
-    __syncwarp();
-    for (int st = 1; st < len; st <<= 1) {
-      for (int m = lane; m < len; m += 32) {
-        double am = a0[m], bm = b0[m], cm = c0[m], rm = r0[m];
-        double an = 0.0, cn = 0.0;
-        if (m - st >= 0) {
-          const double al = -am / b0[m - st];
-          an = al * a0[m - st];
-          bm += al * c0[m - st];
-          rm += al * r0[m - st];
-        }
-        if (m + st < len) {
-          const double ga = -cm / b0[m + st];
-          cn = ga * c0[m + st];
-          bm += ga * a0[m + st];
-          rm += ga * r0[m + st];
-        }
-        a1[m] = an; b1[m] = bm; c1[m] = cn; r1[m] = rm;
-      }
-      __syncwarp();
-      double *t;
-      t = a0; a0 = a1; a1 = t;
-      t = b0; b0 = b1; b1 = t;
-      t = c0; c0 = c1; c1 = t;
-      t = r0; r0 = r1; r1 = t;
-    }
-    for (int m = lane + 1; m <= len; m += 32) x[cell(m)] = r0[m - 1] / b0[m - 1];
-    __syncwarp();
-  }
-}
-
 // RK update of the stage from a stored residual (IRS path):
 // q_out = q^n - alpha dt/V R, optional copy of q^n (stage 1)
-__global__ void k_update_stage(DevBlock b, int npde, int S, const double *__restrict__ res,
+__global__ void k_update_stage(BlockList bs_, int npde, int S, const double *__restrict__ res,
                                const double *__restrict__ qold, double *__restrict__ qout, double *__restrict__ qcopy,
                                const double *__restrict__ dtv, double ar) {
+  const DevBlock b = bs_.get();
   const int ni = b.im - 1, nj = b.jm - 1, nk = b.km - 1;
   const int64_t n = (int64_t)ni * nj * nk * S;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x) {

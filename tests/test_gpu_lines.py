@@ -67,3 +67,46 @@ def test_store_schedule_in_groups_equals_chain():
         out.append(q.download())
     ctx.close()
     assert np.array_equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("irsop", [1, 3])
+@pytest.mark.parametrize("ni", [3, 31, 33, 450, 900, 1700, 3300])
+def test_irs_line_lengths(oracle_mod, ni, irsop):
+    """Residual smoothing of lines that fit shared memory 32, 16 or 8 at a time
+    and (1700 varying, 3300) do not: cirs against the oracle, and one fused
+    cycle, which scales in the sweeps where it can."""
+    case = cases.bump_channel(ni, 6, 2)
+    p = case.params
+    p.irsop, p.psirs, p.rat = irsop, 0.125, float(np.sqrt(1 + 4 * 0.6))
+    O = oracle_mod.OracleLevel(case.tables, p)
+    si, sj, sk, _ = O.metrics(case.x, case.y, case.z)
+    q = cases.perturbed_state(case, amp=0.01, seed=ni)
+    res, dt, _ = O.residual(q.copy(), si, sj, sk)
+    lam, qp = O.p3(), q.copy()
+    O.cons2prim(qp)
+    O.lambda_(qp, si, sj, sk, lam)
+    beta = [O.p1() for _ in range(3)]
+    O.deltat(dt, lam, *beta)
+    ctx = gpu.Context([case.tables], p)
+    rg = ctx.alloc_p3().upload(res)
+    ctx.cirs(1, rg, ctx.alloc_p1().upload(dt), *(ctx.alloc_p1().upload(a) for a in beta))
+    oracle_mod.irs(O, res, dt, *beta)
+
+    def off(a, b):
+        a, b = (casekit.interior_cells(case, x, 5) for x in (a, b))
+        sc = np.abs(b).reshape(-1, 5).max(axis=0)
+        sc[1:4] = sc[1:4].max()
+        return (np.abs(a - b) / sc[None, :, None]).max()
+
+    assert off(rg.download(), res) <= 1e-12
+    qo = q.copy()
+    _, st, _, _ = oracle_mod.smooth_irs(O, qo, si, sj, sk, 1, rms_every=1)
+    assert st == 0
+    m = [ctx.alloc_p2().upload(a) for a in (si, sj, sk)]
+    d = ctx.alloc_p3().upload(q)
+    ctx.bind_level(1, q=d, qold=ctx.alloc_p3(), dtvol=ctx.alloc_p1(), si=m[0], sj=m[1], sk=m[2],
+                   betaxi=ctx.alloc_p1(), betaeta=ctx.alloc_p1(), betazeta=ctx.alloc_p1())
+    _, st = ctx.smooth(1, 1, 1, 1)
+    assert st == 0
+    assert off(d.download(), qo) <= 1e-12
+    ctx.close()

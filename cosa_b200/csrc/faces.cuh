@@ -307,21 +307,23 @@ __device__ __forceinline__ double face_ubn(const double *__restrict__ v, double 
 
 // what a cell's flux balance r goes through after the three families: viscous
 // balance, harmonic-balance source, norms, forcing, update (k_cells and the
-// last launch of the chain).  q0: the cell's base state (read when A.update)
+// last launch of the chain).  co: the cell in the state arrays (variable 1 of
+// snapshot n), P3 their variable stride; q0: the cell's base state (read when
+// A.update)
 template <bool RMS>
-__device__ __forceinline__ void finish_cell(const StageArgs &A, const cosa_params &P, const DevBlock &b, int S, int n,
-                                            int64_t cell, double vol_omega, double dt, double *r, const double *q0,
+__device__ __forceinline__ void finish_cell(const StageArgs &A, const cosa_params &P, int S, int n, int64_t co,
+                                            int64_t P3, double vol_omega, double dt, double *r, const double *q0,
                                             double gamma, double qmin_rho, double qmin_p, double *acc, int &st) {
   double qw[5];
 #pragma unroll
   for (int m = 0; m < 5; ++m) {
-    const int64_t o = p3_var(b, 5, S, m + 1, n) + cell;
+    const int64_t o = co + m * P3;
     if (A.vres) r[m] = r[m] + A.vres[o];
     if (A.vol) {
       // src_bhb (src/src.f90:556-613)
       double qhb = 0.0;
       for (int nj2 = 0; nj2 < S; ++nj2)
-        qhb = __fma_rn(__dmul_rn(vol_omega, P.dhb[n * S + nj2]), A.qin[p3_var(b, 5, S, m + 1, nj2) + cell], qhb);
+        qhb = __fma_rn(__dmul_rn(vol_omega, P.dhb[n * S + nj2]), A.qin[o + (nj2 - n) * 5 * P3], qhb);
       r[m] = r[m] + qhb;
     }
     if (RMS) acc[m] += r[m] * r[m];
@@ -346,7 +348,7 @@ __device__ __forceinline__ void finish_cell(const StageArgs &A, const cosa_param
     // three families' loads (and bprtest's test of that stage's input)
     if (A.prim_out) to_prim(gamma, qmin_rho, qmin_p, st, qw);
 #pragma unroll
-    for (int m = 0; m < 5; ++m) A.qout[p3_var(b, 5, S, m + 1, n) + cell] = qw[m];
+    for (int m = 0; m < 5; ++m) A.qout[co + m * P3] = qw[m];
   }
 }
 
@@ -540,28 +542,38 @@ __device__ __forceinline__ void line_m(const FaceTask &T, const LinePar &LP, con
   float dm[5], sB[5], fb[5], fc[5];
   const float eps32 = (float)ph.epslimf, rk32 = (float)ph.rkap;
   // step f's data: cell f + 1, the metrics of face f; the chain: D, base state
-  // and time step of cell f - 1
-  auto issue = [&](int f, int slot) {
-    const double *p = pq + (f - f0 + 1) * (int64_t)step;
+  // and time step of cell f - 1.  All addresses advance by constant strides
+  // (computed afresh, 420 instructions a cell in the last launch, a cycle of the
+  // 30.7 M-cell duct took 17.0 ms, now 16.0)
+  const double *nq = pq + step, *ns = sp, *nD = Fp, *nb = nullptr, *nt = nullptr;
+  int64_t co = cell0;
+  if (OUT == 2) {
+    nb = A.qold + cell0;
+    nt = A.dtvol + (d == 2 ? p1_idx(b, LP.S, i, f0, tb, n) : p1_idx(b, LP.S, i, tb, f0, n));
+  }
+  const int64_t tstep = d == 2 ? (int64_t)(b.im + 1) : (int64_t)(b.im + 1) * (b.jm + 1);
+  auto issue = [&](bool first, int slot) {
 #pragma unroll
-    for (int m = 0; m < 5; ++m) cp8(&B.q[slot][m][lane], p + (int64_t)m * P3);
-    const double *s = sp + (f - f0) * mstep;
-    cp16(&B.met[slot][0][lane], s);
-    cp16(&B.met[slot][1][lane], s + 2);
-    if (OUT >= 1 && f > f0) {
-      const double *D = Fp + (int64_t)(f - 1 - f0) * fstep;
+    for (int m = 0; m < 5; ++m) cp8(&B.q[slot][m][lane], nq + (int64_t)m * P3);
+    nq += step;
+    cp16(&B.met[slot][0][lane], ns);
+    cp16(&B.met[slot][1][lane], ns + 2);
+    ns += mstep;
+    if (OUT >= 1 && !first) {
 #pragma unroll
-      for (int m = 0; m < 5; ++m) cp8(&B.D[slot][m][lane], D + (int64_t)m * fv);
+      for (int m = 0; m < 5; ++m) cp8(&B.D[slot][m][lane], nD + (int64_t)m * fv);
+      nD += fstep;
       if (OUT == 2 && A.update) {
-        const double *p0 = A.qold + cell0 + (f - 1 - f0) * (int64_t)step;
 #pragma unroll
-        for (int m = 0; m < 5; ++m) cp8(&B.base[slot][m][lane], p0 + (int64_t)m * P3);
-        cp8(&B.base[slot][OUT == 2 ? 5 : 0][lane], A.dtvol + p1_idx(b, LP.S, i, tb, f - 1, n));
+        for (int m = 0; m < 5; ++m) cp8(&B.base[slot][m][lane], nb + (int64_t)m * P3);
+        nb += step;
+        cp8(&B.base[slot][OUT == 2 ? 5 : 0][lane], nt);
+        nt += tstep;
       }
     }
     cp_commit();
   };
-  issue(f0, f0 & 1);
+  issue(true, f0 & 1);
   {
     double qa[5], q1[5];
 #pragma unroll
@@ -607,7 +619,7 @@ __device__ __forceinline__ void line_m(const FaceTask &T, const LinePar &LP, con
   for (int f = f0; f < f1; ++f) {
     const int slot = f & 1;
     if (f + 1 < f1) {
-      issue(f + 1, slot ^ 1);
+      issue(false, slot ^ 1);
       cp_wait<1>();
     } else {
       cp_wait<0>();
@@ -681,18 +693,18 @@ __device__ __forceinline__ void line_m(const FaceTask &T, const LinePar &LP, con
 #pragma unroll
         for (int m = 0; m < 5; ++m) D[m] = B.D[slot][m][lane] + F[m] - Fprev[m];
         if (OUT == 1) {
-          double *Dp = Fp + (int64_t)(f - 1 - f0) * fstep;
 #pragma unroll
-          for (int m = 0; m < 5; ++m) Dp[(int64_t)m * fv] = D[m];
+          for (int m = 0; m < 5; ++m) Fp[(int64_t)m * fv] = D[m];
         } else {
           double q0[5];
 #pragma unroll
           for (int m = 0; m < 5; ++m) q0[m] = B.base[slot][OUT == 2 ? m : 0][lane];
           const double ov = A.vol ? Pp->omega * A.vol[p1_idx(b, 1, i, tb, f - 1, 0)] : 0.0;
-          finish_cell<RMS>(A, *Pp, b, LP.S, n, p3_cell(b, i, tb, f - 1), ov, B.base[slot][OUT == 2 ? 5 : 0][lane], D, q0,
+          finish_cell<RMS>(A, *Pp, LP.S, n, co, (int64_t)P3, ov, B.base[slot][OUT == 2 ? 5 : 0][lane], D, q0,
                            LP.gamma, LP.qmin_rho, LP.qmin_p, acc, st);
         }
       }
+      if (f > f0) { Fp += fstep; co += step; }
 #pragma unroll
       for (int m = 0; m < 5; ++m) Fprev[m] = F[m];
     }

@@ -112,7 +112,7 @@ k_cells(const DevBlock *__restrict__ blocks, const cosa_params *__restrict__ Pp,
       r[m] = r[m] + fl[m][4] - fl[m][5];
     }
     const double ov = A.vol ? P.omega * A.vol[p1_idx(b, 1, i, j, k, 0)] : 0.0;
-    finish_cell<RMS>(A, P, b, S, n, cell, ov, dt, r, q0, P.gamma, P.qmin[0], P.qmin[4], acc, st);
+    finish_cell<RMS>(A, P, S, n, p3_var(b, npde, S, 1, n) + cell, b.P3, ov, dt, r, q0, P.gamma, P.qmin[0], P.qmin[4], acc, st);
   }
   if (RMS) {
     // deterministic per-CTA sums: warp shuffle, then fixed-order warp sums

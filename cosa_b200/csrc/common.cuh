@@ -53,6 +53,32 @@ __host__ __device__ __forceinline__ int64_t f0_idx(const DevBlock &b, int npde, 
   return b.of0 * npde * S + ((int64_t)n * npde + (v - 1)) * I * J * K + (i - 1) + I * ((j - 1) + J * (int64_t)(k - 1));
 }
 
+// the 4 components of a face metric record, two 16-byte loads
+__device__ __forceinline__ void ld_met(const double *__restrict__ sp, double *m4) {
+  const double2 a = __ldg(reinterpret_cast<const double2 *>(sp));
+  const double2 c = __ldg(reinterpret_cast<const double2 *>(sp + 2));
+  m4[0] = a.x; m4[1] = a.y; m4[2] = c.x; m4[3] = c.y;
+}
+
+// A linear index being taken apart into (i, j, k, snapshot): 32-bit division
+// while it fits (a third of the 64-bit one's instructions), 64-bit above.
+struct Dec {
+  uint64_t v;
+  __device__ __forceinline__ explicit Dec(int64_t t) : v((uint64_t)t) {}
+  __device__ __forceinline__ int operator%(int n) const {
+    return (v >> 32) ? (int)(v % (uint64_t)n) : (int)((unsigned)v % (unsigned)n);
+  }
+  __device__ __forceinline__ int64_t operator/(int n) const {
+    return (v >> 32) ? (int64_t)(v / (uint64_t)n) : (int64_t)((unsigned)v / (unsigned)n);
+  }
+  __device__ __forceinline__ Dec &operator/=(int n) {
+    v = (uint64_t)(*this / n);
+    return *this;
+  }
+  __device__ __forceinline__ explicit operator int() const { return (int)v; }
+  __device__ __forceinline__ operator int64_t() const { return (int64_t)v; }
+};
+
 // cyc(idir,m) of input() (src/input.f90:2409), 1-based
 __host__ __device__ __forceinline__ int cyc3(int idir, int m) {
   int r = idir + m - 1;

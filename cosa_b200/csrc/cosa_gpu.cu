@@ -829,6 +829,7 @@ int launch_visc(cosa_ctx *c, LevelState &L, bool dt, double *bx, double *by, dou
   int r = 0;
   if ((r = launch_edges(c, L, L.d_qprim, nullptr))) return r;
   const cosa_level_ptrs &P = L.ptrs;
+  const VisK vk = make_visk(p);
   if (dt) {
     const bool mv = c->p.moving;
     k_dt_ns<<<dim3(grid_x(mc, L.nb), L.nb), 256, 0, c->s>>>(L.d_blocks, c->d_p, L.d_qprim, P.si, P.sj, P.sk, P.vol,
@@ -837,12 +838,12 @@ int launch_visc(cosa_ctx *c, LevelState &L, bool dt, double *bx, double *by, dou
     if ((r = after_launch(c))) return r;
   }
   k_vface<<<dim3(grid_x(mf, L.nb), L.nb, 3), 256, 0, c->s>>>(L.d_blocks, c->d_p, L.d_qprim, P.si, P.sj, P.sk, L.d_vm,
-                                                             L.n0, L.d_vflux);
+                                                             L.n0, vk, L.d_vflux);
   if ((r = after_launch(c))) return r;
   if (!L.walls.empty()) {
     const int nw = (int)L.walls.size();
     k_vwall<<<grid_for((int64_t)nw * S), 256, 0, c->s>>>(L.d_blocks, L.d_walls, nw, c->d_p, L.d_qprim, P.si, P.sj,
-                                                         P.sk, L.d_vm, L.n0, L.d_vflux);
+                                                         P.sk, L.d_vm, L.n0, vk, L.d_vflux);
     if ((r = after_launch(c))) return r;
   }
   k_vdiv<<<dim3(grid_x(mc, L.nb), L.nb), 256, 0, c->s>>>(L.d_blocks, c->d_p, L.d_vflux, L.n0, L.d_vres);
@@ -1031,14 +1032,18 @@ int launch_rans_iteration(cosa_ctx *c, int nl, LevelState &L, const IterOpts &o)
 int launch_norm(cosa_ctx *c, LevelState &L, const double *res, const double *rhs, const double *q_imp) {
   int r = 0;
   int64_t ncell = 0;
+  if (!q_imp) {
+    k_rms_partial<<<dim3(64, L.nb), 256, 0, c->s>>>(BlockList{L.d_blocks}, c->d_p, res, rhs, L.d_part);
+    if ((r = after_launch(c))) return r;
+  }
   for (int b = 0; b < L.nb; ++b) {
     const DevBlock &x = L.hb[b];
     double *part = L.d_part + (int64_t)b * 64 * 8;
-    if (q_imp && c->p.harbal) k_rms_bhb_partial<<<64, 256, 0, c->s>>>(x, c->d_p, res, q_imp, L.ptrs.vol, part);
-    else if (q_imp) k_rms_dualimp<<<64, 256, 0, c->s>>>(x, c->d_p, res, rhs, q_imp, L.ptrs.vol, part);
-    else k_rms_partial<<<64, 256, 0, c->s>>>(x, c->d_p, res, rhs, part);
-    if ((r = after_launch(c))) return r;
     ncell += (int64_t)(x.im - 1) * (x.jm - 1) * (x.km - 1);
+    if (!q_imp) continue;
+    if (c->p.harbal) k_rms_bhb_partial<<<64, 256, 0, c->s>>>(x, c->d_p, res, q_imp, L.ptrs.vol, part);
+    else k_rms_dualimp<<<64, 256, 0, c->s>>>(x, c->d_p, res, rhs, q_imp, L.ptrs.vol, part);
+    if ((r = after_launch(c))) return r;
   }
   const double cnt = (double)ncell * (c->p.harbal ? 2 * c->p.nharms + 1 : 1);
   k_rms_final<<<1, 256, 0, c->s>>>(L.d_part, L.nb * 64, c->p.npde, cnt, c->d_hist, c->d_row, c->hist_cap);
@@ -1661,10 +1666,8 @@ int cosa_gpu_resg_rms(cosa_ctx *c, int32_t nl, const double *res, const double *
     if ((r = dalloc(c, &L->d_part, (size_t)L->nb * 64 * 8))) return r;
     L->npart_cap = L->nb * 64;
   }
-  for (int b = 0; b < L->nb; ++b) {
-    k_rms_partial<<<64, 256, 0, c->s>>>(L->hb[b], c->d_p, res, rhs, L->d_part + (int64_t)b * 64 * 8);
-    if ((r = after_launch(c))) return r;
-  }
+  k_rms_partial<<<dim3(64, L->nb), 256, 0, c->s>>>(BlockList{L->d_blocks}, c->d_p, res, rhs, L->d_part);
+  if ((r = after_launch(c))) return r;
   if ((r = ensure_hist(c, 1))) return r;
   int64_t ncell = 0;
   for (auto &b : L->hb) ncell += (int64_t)(b.im - 1) * (b.jm - 1) * (b.km - 1);
@@ -3146,9 +3149,9 @@ int rans_face_state(cosa_ctx *c, LevelState &L, int d, const double *q, double *
   return after_launch(c);
 }
 
-// one RK stage of the k-omega path, routine by routine as smooth() runs it
-// (src/cosa.f90:1719-2016): every kernel is a full-array pass with the
-// reference's arrays, captured with the rest of the iteration in a graph
+// one RK stage of the k-omega path in smooth()'s order (src/cosa.f90:1719-2016):
+// vertex gradients, convective and viscous face fluxes, one pass over the
+// cells, the update; captured with the rest of the iteration in a graph
 int launch_rans_stage(cosa_ctx *c, int nl, LevelState &L, int irk, const IterOpts &o) {
   const bool compute_dt = o.compute_dt && irk == 1, want_rms = o.want_rms && irk == o.rms_stage, copy_qold = o.copy_qold;
   const cosa_params &p = c->p;
@@ -3156,16 +3159,24 @@ int launch_rans_stage(cosa_ctx *c, int nl, LevelState &L, int irk, const IterOpt
   const cosa_level_ptrs &P = L.ptrs;
   double *q = P.q;
   int r = 0;
-  if (irk == 1 && copy_qold &&
-      (r = for_blocks(c, L, cnt_interior,
-                      [&](auto b, dim3 g) { k_copy_interior<<<g, 256, 0, c->s>>>(b, npde * S, q, P.qold); })))
+  // between the stages of an explicit iteration the interior of q stays
+  // primitive: the update stores it so (the point-implicit update needs k and
+  // omega themselves), the last stage's in conservative form.  The dual-time
+  // and implicit updates work on conservative values: q is converted at every
+  // stage there
+  const bool keep = !p.dualt && !p.rkimp;
+  const int *bct = L.d_bct;
+  const BlockList bl{L.d_blocks};
+  const VisK vk = make_visk(p);
+  const bool mixed = p.precision == COSA_PREC_MIXED;
+  if ((!keep || irk == 1) && (r = for_blocks(c, L, cnt_cells, [&](auto b, dim3 g) {
+         k_rans_prim<<<g, 256, 0, c->s>>>(b, c->d_p, q, irk == 1 && copy_qold ? P.qold : nullptr, c->d_status);
+       })))
     return r;
-  if ((r = cosa_gpu_cons2prim(c, nl, 0, q))) return r;
-  if (!L.items.empty()) {
-    // BC patches then cuts, last writers as in the reference
-    if ((r = launch_halo<false>(c, L, L.d_items, (int)L.items.size(), q, P.si, P.sj, P.sk, P.dist, face_vel_of(c, L))))
-      return r;
-  }
+  // BC patches then cuts, last writers as in the reference (bprtest of the i halos)
+  if (!L.items.empty() && (r = launch_halo<false>(c, L, L.d_items, (int)L.items.size(), q, P.si, P.sj, P.sk, P.dist,
+                                                  face_vel_of(c, L), 1)))
+    return r;
   if (o.first_cycle && o.force && irk == 1 && !p.prd_all_lvls) {
     // coarse-level mut from the restricted (primitive) state at the first
     // stage of the first cycle's visit (src/cosa.f90:1727-1760); SST takes
@@ -3188,8 +3199,6 @@ int launch_rans_stage(cosa_ctx *c, int nl, LevelState &L, int irk, const IterOpt
     }
     if ((r = cosa_gpu_cutman_mut(c, nl, P.mut))) return r;
   }
-  if ((r = for_blocks(c, L, cnt_all, [&](auto b, dim3 g) { k_prtest<<<g, 256, 0, c->s>>>(b, c->d_p, q, c->d_status); })))
-    return r;
   if (compute_dt) {
     if ((r = for_blocks(c, L, cnt_cells, [&](auto b, dim3 g) {
            const bool mv = p.moving;
@@ -3206,56 +3215,54 @@ int launch_rans_stage(cosa_ctx *c, int nl, LevelState &L, int irk, const IterOpt
          })))
       return r;
   }
-  if ((r = cosa_gpu_zero(c, nl, P.res))) return r;
-  if ((r = launch_edges(c, L, q, P.mut))) return r;
-  const bool mixed = p.precision == COSA_PREC_MIXED;
-  const int *bct = L.d_bct;
-  const BlockList bl{L.d_blocks};
-  const int ntr = L.nb * 3 * S;
-  if (mixed) k_rans_h0<true><<<grid_for(ntr, 64), 64, 0, c->s>>>(L.d_blocks, L.nb, c->d_p, bct, q, nl, L.d_h0);
-  else k_rans_h0<false><<<grid_for(ntr, 64), 64, 0, c->s>>>(L.d_blocks, L.nb, c->d_p, bct, q, nl, L.d_h0);
-  if ((r = after_launch(c))) return r;
-  // muscl + roflux and q_face / q_der / rtst / vflux of the three families in
-  // one launch, then resid of their sums (src/cosa.f90:1797-1824)
+  // the residual's halos are read only by the cut-aware smoothing and the
+  // transfers: zeroed there, as the reference leaves them
+  if ((p.cutcirs || p.nlevel > 1 || !keep) && (r = cosa_gpu_zero(c, nl, P.res))) return r;
+  {
+    int per = 1;
+    for (const DevBlock &x : L.hb) per = std::max(per, 4 * (x.im + x.jm + x.km - 3));
+    const dim3 g(1 + (unsigned)std::max<int64_t>(1, ((int64_t)per * (npde + 1) * S + 127) / 128), L.nb);
+    auto k = mixed ? k_rans_pre<true> : k_rans_pre<false>;
+    k<<<g, 128, 0, c->s>>>(bl, c->d_p, bct, nl, q, irk == 1 ? P.mut : nullptr, L.d_h0);
+    if ((r = after_launch(c))) return r;
+  }
+  // muscl + roflux, then q_face / q_der / rtst / vflux added, of the three
+  // families (src/cosa.f90:1797-1824)
   if ((r = for_blocks(c, L, cnt_faces, [&](auto b, dim3 g) {
          (void)b;
-         const dim3 g6(g.x * 2, g.y, 6);
-         const double *fd = blend(p) ? L.d_fdist : nullptr;
-         if (mixed)
-           k_rans_faces<true><<<g6, 128, 0, c->s>>>(bl, c->d_p, bct, q, nl, P.si, P.sj, P.sk, L.d_h0, P.mut, L.d_vm,
-                                                    L.n0, fd, L.d_rflux, face_vel_of(c, L));
-         else
-           k_rans_faces<false><<<g6, 128, 0, c->s>>>(bl, c->d_p, bct, q, nl, P.si, P.sj, P.sk, L.d_h0, P.mut, L.d_vm,
-                                                     L.n0, fd, L.d_rflux, face_vel_of(c, L));
+         const dim3 g3(g.x * 2, g.y, 3);
+         auto k = mixed ? k_rans_conv<true> : k_rans_conv<false>;
+         k<<<g3, 128, 0, c->s>>>(bl, c->d_p, make_phys(p), bct, q, nl, P.si, P.sj, P.sk, L.d_h0, L.n0, L.d_rflux,
+                                 face_vel_of(c, L));
        })) ||
-      (r = for_blocks(c, L, cnt_cells, [&](auto b, dim3 g) {
+      (r = for_blocks(c, L, cnt_faces, [&](auto b, dim3 g) {
          (void)b;
-         k_rans_resid<<<g, 256, 0, c->s>>>(bl, c->d_p, L.n0, L.d_rflux, P.res);
+         k_rans_visc<<<dim3(g.x * 2, g.y, 3), 128, 0, c->s>>>(bl, c->d_p, vk, bct, q, P.si, P.sj, P.sk, P.mut, L.d_vm,
+                                                              L.n0, blend(p) ? L.d_fdist : nullptr, L.d_rflux);
        })))
     return r;
-  // cell-centred velocity gradients, production, BSL/SST blending and the
-  // sources in one pass over the cells (src/cosa.f90:1878-1901)
-  if ((r = for_blocks(c, L, cnt_cells, [&](auto b, dim3 g) {
-         (void)b;
-         if (blend(p))
-           k_rans_cellsrc<true><<<g, 256, 0, c->s>>>(bl, c->d_p, nl, bct, q, P.qp, P.qm, P.dqm, L.d_vm, L.n0, P.mut,
-                                                    P.dist, P.vol, L.d_prd, L.d_divvel, L.d_delpls, L.d_ttrm, P.res);
-         else
-           k_rans_cellsrc<false><<<g, 256, 0, c->s>>>(bl, c->d_p, nl, bct, q, P.qp, P.qm, P.dqm, L.d_vm, L.n0, P.mut,
-                                                     P.dist, P.vol, L.d_prd, L.d_divvel, L.d_delpls, nullptr, P.res);
-       })))
-    return r;
-  if ((r = cosa_gpu_prim2cons(c, nl, q))) return r;
+  // flux balance, velocity gradients, production, BSL/SST blending, sources
+  // and the time-spectral source in one pass over the cells
+  // (src/cosa.f90:1878-1922).  SST's eddy viscosity reads the last stage's
+  // differences; src_hb is skipped under rkimp without IRS on one level
+  const bool hb_sir = p.harbal && (!p.rkimp || p.irsop > 0 || p.nlevel > 1);
+  {
+    const bool diff = p.kom_sst && irk == p.nstage;
+    double *dx = diff ? P.qp : nullptr, *dy = diff ? P.qm : nullptr, *dz = diff ? P.dqm : nullptr;
+    if ((r = for_blocks(c, L, cnt_cells, [&](auto b, dim3 g) {
+           (void)b;
+           auto k = blend(p) ? k_rans_cell<true> : k_rans_cell<false>;
+           k<<<dim3(g.x * 2, g.y), 128, 0, c->s>>>(bl, c->d_p, vk, nl, bct, q, L.d_rflux, dx, dy, dz, L.d_vm, L.n0, P.mut,
+                                                   P.dist, P.vol, L.d_prd, L.d_divvel, L.d_delpls,
+                                                   blend(p) ? L.d_ttrm : nullptr, P.res, hb_sir ? 1 : 0);
+         })))
+      return r;
+  }
+  if ((!keep || o.res_only) && (r = cosa_gpu_prim2cons(c, nl, q))) return r;
   // dual time: src_uns, the norm with rhs_uns, res -= rhs_uns on the fine
   // level (src/cosa.f90:1908-1941)
   if (dual_src_in_res(p) &&
       (r = for_blocks(c, L, cnt_cells, [&](auto b, dim3 g) { k_src_uns<<<g, 256, 0, c->s>>>(b, c->d_p, q, P.vol, P.res); })))
-    return r;
-  // harmonic balance: src_hb unless rkimp without IRS on one level
-  // (src/cosa.f90:1918-1922)
-  const bool hb_sir = p.harbal && (!p.rkimp || p.irsop > 0 || p.nlevel > 1);
-  if (hb_sir &&
-      (r = for_blocks(c, L, cnt_cells, [&](auto b, dim3 g) { k_src_hb<<<g, 256, 0, c->s>>>(b, c->d_p, q, P.vol, P.res); })))
     return r;
   const bool imp_norm = p.rkimp && ((p.dualt && !dual_src_in_res(p)) || (p.harbal && !hb_sir));
   if (want_rms && (r = launch_norm(c, L, P.res, p.dualt ? P.rhs : nullptr, imp_norm ? q : nullptr))) return r;
@@ -3327,11 +3334,15 @@ int launch_rans_stage(cosa_ctx *c, int nl, LevelState &L, int irk, const IterOpt
     // point-implicit k / omega, the mean-flow update and fixq in one pass
     const double ar = p.alphas[irk - 1];
     const double *tt = blend(p) ? L.d_ttrm : nullptr;
+    const bool last = irk == p.nstage;
     if ((r = for_blocks(c, L, cnt_cells, [&](auto b, dim3 g) {
-           k_update_rans<<<g, 256, 0, c->s>>>(b, c->d_p, P.res, q, P.qold, P.vol, P.dtvolt, P.dtvol, L.d_delpls,
-                                              L.d_prd, ar, tt);
+           auto k = !keep ? k_update_rans<false, false> : last ? k_update_rans<true, false> : k_update_rans<true, true>;
+           k<<<g, 256, 0, c->s>>>(b, c->d_p, P.res, q, P.qold, P.vol, P.dtvolt, P.dtvol, L.d_delpls, L.d_prd, ar, tt,
+                                  c->d_status);
          })))
       return r;
+    // the face halos of the state that the iteration leaves
+    if (keep && last && !L.items.empty() && (r = launch_halo_p2c(c, L, q, q))) return r;
   }
   // k_update_rans applies fixq itself
   if (p.ifixq && p.rkimp && (p.dualt || p.harbal) && (r = cosa_gpu_fixq(c, nl, q))) return r;
@@ -3415,7 +3426,7 @@ int launch_lsp_stage(cosa_ctx *c, int nl, LevelState &L, int irk, const IterOpts
          (void)b;
          const dim3 gz(g.x * 2, g.y, p.viscous ? 6 : 3);
          k_lsp_faces<<<gz, 128, 0, c->s>>>(bl, c->d_p, bct, q, nl, P.si, P.sj, P.sk, L.d_cut_pgr, L.d_cut_vis, L.d_vm,
-                                           L.n0, L.d_rflux);
+                                           L.n0, make_visk(p), L.d_rflux);
        })) ||
       (r = for_blocks(c, L, cnt_cells, [&](auto b, dim3 g) {
          (void)b;

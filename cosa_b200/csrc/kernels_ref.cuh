@@ -441,8 +441,9 @@ __device__ __forceinline__ void rms_accumulate(const DevBlock &b, int npde, int 
   }
 }
 
-__global__ void k_rms_partial(DevBlock b, const cosa_params *__restrict__ Pp, const double *__restrict__ res,
+__global__ void k_rms_partial(BlockList bs_, const cosa_params *__restrict__ Pp, const double *__restrict__ res,
                               const double *__restrict__ rhs, double *__restrict__ part) {
+  const DevBlock b = bs_.get();
   const cosa_params &P = *Pp;
   const int npde = P.npde, S = 2 * P.nharms + 1;
   double acc[7] = {0, 0, 0, 0, 0, 0, 0};
@@ -459,7 +460,7 @@ __global__ void k_rms_partial(DevBlock b, const cosa_params *__restrict__ Pp, co
     for (int v = 0; v < npde; ++v) {
       double x = threadIdx.x < nw ? red[v][threadIdx.x] : 0.0;
       for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-      if (threadIdx.x == 0) part[(int64_t)blockIdx.x * 8 + v] = x;
+      if (threadIdx.x == 0) part[((int64_t)blockIdx.y * gridDim.x + blockIdx.x) * 8 + v] = x;
     }
   }
 }

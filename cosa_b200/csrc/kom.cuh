@@ -25,6 +25,14 @@
 // is given, Wilcox's constants otherwise.
 #pragma once
 #include "visc.cuh"
+#include "faces.cuh"
+#include "mg.cuh"
+
+// Resident CTAs of 128 per SM that the k-omega stage's face and cell kernels
+// are compiled for: 128 registers, 16 warps.  Five cycles on the 512 x 128 x 2
+// aerofoil grid at 3 / 4 / 5 (cells 3 / 4 / 6): 5.2 / 4.7 / 4.9 ms; three of the
+// pitching one (S = 3): 1.84 / 1.72 / 1.76 ms.
+constexpr int kRansCtas = 4;
 
 // ---- per-routine kernels ---------------------------------------------------------------
 // one thread per face (i,j,k) of family D and snapshot
@@ -33,7 +41,7 @@
   const int64_t total = (int64_t)ni * nj * nk * S;                                                          \
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;                              \
        t += (int64_t)gridDim.x * blockDim.x) {                                                              \
-    int64_t r_ = t;                                                                                         \
+    Dec r_(t);                                                                                         \
     const int i = (int)(r_ % ni) + 1; r_ /= ni;                                                             \
     const int j = (int)(r_ % nj) + 1; r_ /= nj;                                                             \
     const int k = (int)(r_ % nk) + 1;                                                                       \
@@ -44,7 +52,7 @@
   const int64_t total = (int64_t)ni * nj * nk * S;                                                          \
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;                              \
        t += (int64_t)gridDim.x * blockDim.x) {                                                              \
-    int64_t r_ = t;                                                                                         \
+    Dec r_(t);                                                                                         \
     const int i = (int)(r_ % ni) + 1; r_ /= ni;                                                             \
     const int j = (int)(r_ % nj) + 1; r_ /= nj;                                                             \
     const int k = (int)(r_ % nk) + 1;                                                                       \
@@ -397,7 +405,7 @@ __global__ void k_rest4(DevBlock b1, DevBlock b2, int S, const double *__restric
   const int ni = b2.im - 1, nj = b2.jm - 1, nk = b2.km - 1;
   const int64_t total = (int64_t)ni * nj * nk * S;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-    int64_t r = t;
+    Dec r(t);
     const int i2 = (int)(r % ni) + 1; r /= ni;
     const int j2 = (int)(r % nj) + 1; r /= nj;
     const int k2 = (int)(r % nk) + 1; r /= nk;
@@ -479,7 +487,7 @@ __global__ void k_add_interior(BS bs_, int nvs, double *__restrict__ v1, const d
   const int64_t total = (int64_t)ni * nj * nk * nvs;
   const int64_t base = b.op3 * nvs;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-    int64_t r = t;
+    Dec r(t);
     const int i = (int)(r % ni) + 1; r /= ni;
     const int j = (int)(r % nj) + 1; r /= nj;
     const int k = (int)(r % nk) + 1; r /= nk;
@@ -684,7 +692,7 @@ __device__ __forceinline__ void rans_face_recon(const DevBlock &b, const cosa_pa
     const int64_t base = p3_var(b, npde, S, v, n);
     const double qm2 = q[base + cm2], qm = q[base + cm], q0 = q[base + c0], qp = q[base + cp];
     const bool fo = first_all || (P.foturb && v >= 6);
-    double a_ = 0.0, b_ = 0.0;
+    double vp = q0, vm = qm;
     if (!fo) {
       double dlo = qm - qm2, dmid = q0 - qm, dhi = qp - q0;
       if (dlo2) dlo = dlo * 2;
@@ -695,12 +703,18 @@ __device__ __forceinline__ void rans_face_recon(const DevBlock &b, const cosa_pa
       if (MIXED) {
         float fa, fb;
         limit_face_fast(ilim, (float)eps, (float)P.rkap, (float)dlo, (float)dmid, (float)dhi, fa, fb);
-        a_ = fa; b_ = fb;
+        vp = q0 + fa; vm = qm + fb;
       } else {
-        limit_face<double>(ilim, eps, P.rkap, dlo, dmid, dhi, a_, b_);
+        double unused;
+        if (ilim == 1) {
+          cell_states64<true>(1, eps, P.rkap, q0, dmid, dhi, vp, unused);
+          cell_states64<true>(1, eps, P.rkap, qm, dlo, dmid, unused, vm);
+        } else {
+          cell_states64<false>(ilim, eps, P.rkap, q0, dmid, dhi, vp, unused);
+          cell_states64<false>(ilim, eps, P.rkap, qm, dlo, dmid, unused, vm);
+        }
       }
     }
-    double vp = fo ? q0 : q0 + a_, vm = fo ? qm : qm + b_;
     if (side) vp = vm = side == 1 ? qm : q0;  // q(0) at the min face, q(mx) at the max face
     vr[v - 1] = vp;
     vl[v - 1] = vm;
@@ -712,47 +726,64 @@ __device__ __forceinline__ void rans_face_recon(const DevBlock &b, const cosa_pa
 // family (and its j, k counterparts) per block, family and snapshot, into
 // h0[((block * 3 + d - 1) * S + n) * 2 + side]
 template <bool MIXED>
-__global__ void k_rans_h0(const DevBlock *__restrict__ blocks, int nb, const cosa_params *__restrict__ Pp,
-                          const int *__restrict__ bct, const double *__restrict__ q, int nl, double *__restrict__ h0) {
-  const cosa_params &P = *Pp;
+__device__ __forceinline__ void rans_h0(const DevBlock &b, int ib, const cosa_params &P, const int *__restrict__ bct,
+                                        const double *__restrict__ q, int nl, int d, int n, double *__restrict__ h0) {
   const int S = 2 * P.nharms + 1;
-  const int64_t total = (int64_t)nb * 3 * S;
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-    const int n = (int)(t % S), d = (int)((t / S) % 3) + 1, ib = (int)(t / (3 * S));
-    const DevBlock b = blocks[ib];
-    const int ic = d == 1 ? b.im : b.im - 1, jc = d == 2 ? b.jm : b.jm - 1, kc = d == 3 ? b.km : b.km - 1;
-    double a7[7], b7[7];
-    rans_face_recon<MIXED>(b, P, bct, q, d, nl, ic, jc, kc, n, 6, a7, b7);
-    h0[t * 2] = face_h0(P.gamma, a7);
-    h0[t * 2 + 1] = face_h0(P.gamma, b7);
+  const int ic = d == 1 ? b.im : b.im - 1, jc = d == 2 ? b.jm : b.jm - 1, kc = d == 3 ? b.km : b.km - 1;
+  double a7[7], b7[7];
+  rans_face_recon<MIXED>(b, P, bct, q, d, nl, ic, jc, kc, n, 6, a7, b7);
+  const int64_t t = ((int64_t)ib * 3 + (d - 1)) * S + n;
+  h0[t * 2] = face_h0(P.gamma, a7);
+  h0[t * 2 + 1] = face_h0(P.gamma, b7);
+}
+// what the face launch needs beside the halos, in one launch of grid (x,
+// block): q_edges of the primitive state (and, on an iteration's first stage,
+// of mut, which changes only at its end) and, in CTA 0's first threads, h0 of
+// each family's last face (no edge cell enters it)
+template <bool MIXED>
+__global__ void k_rans_pre(BlockList bs_, const cosa_params *__restrict__ Pp, const int *__restrict__ bct, int nl,
+                           double *__restrict__ q, double *__restrict__ mut, double *__restrict__ h0) {
+  const DevBlock b = bs_.get();
+  const cosa_params &P = *Pp;
+  const int npde = P.npde, S = 2 * P.nharms + 1;
+  if (blockIdx.x == 0) {
+    for (int t = threadIdx.x; t < 3 * S; t += blockDim.x)
+      rans_h0<MIXED>(b, blockIdx.y, P, bct, q, nl, t % 3 + 1, t / 3, h0);
+    return;
+  }
+  const int per = 4 * ((b.km - 1) + (b.jm - 1) + (b.im - 1));
+  const int nv = npde + (mut ? 1 : 0);
+  const int64_t total = (int64_t)per * nv * S;
+  for (int64_t t = (blockIdx.x - 1) * (int64_t)blockDim.x + threadIdx.x; t < total;
+       t += (int64_t)(gridDim.x - 1) * blockDim.x) {
+    const Dec d(t);
+    const int vn = (int)(d / per), v = vn % nv, n = vn / nv;
+    edge_cell(b, d % per, v < npde ? q + p3_var(b, npde, S, v + 1, n) : mut + b.op3 * S + (int64_t)n * b.P3);
   }
 }
 
 // muscl + roflux_b of the faces of family D of block b: the reconstructed
 // states stay in registers, the seven convective face fluxes go to F
 template <int D, bool MIXED>
-__device__ __forceinline__ void rans_conv_faces(const DevBlock &b, const cosa_params &P, const int *__restrict__ bct,
+__device__ __forceinline__ void rans_conv_faces(const DevBlock &b, const cosa_params &P, const PhysPar &ph,
+                                                const int *__restrict__ bct,
                                                 const double *__restrict__ q, int nl, const double *__restrict__ s,
                                                 const double *__restrict__ h0b, double *__restrict__ F,
                                                 const double *__restrict__ fv = nullptr) {
-  const PhysPar ph = make_phys(P);
   const int npde = P.npde, S = 2 * P.nharms + 1, S2 = 2 * P.nharms * P.hbmove + 1;
   KOM_FACE_LOOP(D)
-    double vr[7], vl[7], f[5];
+    double vr[7], vl[7], f[7];
     rans_face_recon<MIXED>(b, P, bct, q, D, nl, i, j, k, n, npde, vr, vl);
     const int nh = n * P.hbmove;
     const int64_t e4 = p2_idx(b, S2, 1, i, j, k, nh);
-    const double kx = s[e4], ky = s[e4 + 1], kz = s[e4 + 2], ds = s[e4 + 3];
+    double met[4];
+    ld_met(s + e4, met);
     // the face speed of a moving grid (roflux_b, src/flux.f90:110-113, 262-264)
-    const double ubn = fv ? fv[(e4 >> 2) * 3] * kx + fv[(e4 >> 2) * 3 + 1] * ky + fv[(e4 >> 2) * 3 + 2] * kz : 0.0;
-    if (MIXED) roe_flux_mixed_tke(ph, kx, ky, kz, ds, vr, vl, vr[5], vl[5], f, ubn);
-    else roe_flux_fp64(ph, kx, ky, kz, ds, vr, vl, vr[5], vl[5], f, ubn);
+    const double ubn = fv ? face_ubn(fv + (e4 >> 2) * 3, met[0], met[1], met[2]) : 0.0;
+    roe_flux_rans(ph, P, met[0], met[1], met[2], met[3], vr, vl, h0b[2 * n], h0b[2 * n + 1], ubn, f);
+    const int64_t o = f0_idx(b, npde, S, i, j, k, 1, n), st = (int64_t)b.im * b.jm * b.km;
 #pragma unroll
-    for (int m = 0; m < 5; ++m) F[f0_idx(b, npde, S, i, j, k, m + 1, n)] = f[m];
-    double fk, fw;
-    roe_turb(P, kx, ky, kz, ds, vr, vl, h0b[2 * n], h0b[2 * n + 1], fk, fw, ubn);
-    F[f0_idx(b, npde, S, i, j, k, 6, n)] = fk;
-    F[f0_idx(b, npde, S, i, j, k, 7, n)] = fw;
+    for (int m = 0; m < 7; ++m) F[o + m * st] = f[m];
   }
 }
 
@@ -761,14 +792,15 @@ __device__ __forceinline__ void rans_conv_faces(const DevBlock &b, const cosa_pa
 // faces the one-sided wall formulas with the halo mut (src/flux.f90:1848-1962,
 // 2846-2946, 947-1180); the NV viscous face fluxes go to F.  NV = 7: k-omega
 // (Reynolds stresses, k and omega diffusion); NV = 5: laminar flow (mut null)
-template <int D, int NV = 7>
+// ADD: onto the convective flux already there
+template <int D, int NV = 7, bool ADD = false>
 __device__ __forceinline__ void rans_visc_faces(const DevBlock &b, int ib, const cosa_params &P,
                                                 const int *__restrict__ bct, const double *__restrict__ q,
                                                 const double *__restrict__ mut, const double *__restrict__ vm,
                                                 int64_t n0, const double *__restrict__ s,
-                                                const double *__restrict__ fdist, double *__restrict__ F) {
+                                                const double *__restrict__ fdist, const VisK &V,
+                                                double *__restrict__ F) {
   const int npde = P.npde, S = 2 * P.nharms + 1;
-  const ViscPar V = make_visc(P);
   constexpr int di = D == 1, dj = D == 2, dk = D == 3;
   const int mx = D == 1 ? b.im : (D == 2 ? b.jm : b.km);
   KOM_FACE_LOOP(D)
@@ -793,57 +825,57 @@ __device__ __forceinline__ void rans_visc_faces(const DevBlock &b, int ib, const
     double vmf[9];
     load_vm(vm + (int64_t)(n * P.hbmove) * 27 * n0, b, n0, D, i, j, k, vmf);
     const int64_t e4 = p2_idx(b, 2 * P.nharms * P.hbmove + 1, 1, i, j, k, n * P.hbmove);
-    double Fv[NV];
-    if constexpr (NV == 7) {
-      double gr[3][3], t6[6];
+    double Fv[NV], met[4];
+    ld_met(s + e4, met);
+    visc_flux<NV>(V, qf, g, vmf, met[0], met[1], met[2], met[3], mf,
+                  NV == 7 && fdist ? fdist[f0_idx(b, 1, 1, i, j, k, 1, 0)] : 0.0, Fv);
+    const int64_t o = f0_idx(b, npde, S, i, j, k, 1, n), st = (int64_t)b.im * b.jm * b.km;
 #pragma unroll
-      for (int m = 0; m < 3; ++m) { gr[m][0] = g[0][m + 1]; gr[m][1] = g[1][m + 1]; gr[m][2] = g[2][m + 1]; }
-      rtst_face(P, qf[0], qf[5], gr, vmf, mf, t6);
-      vflux_kom_face(P, V, qf, g, t6, vmf, s[e4], s[e4 + 1], s[e4 + 2], s[e4 + 3], mf,
-                     fdist ? fdist[f0_idx(b, 1, 1, i, j, k, 1, 0)] : -1.0, Fv);
-    } else {
-      vflux_face(V, qf, g, vmf, s[e4], s[e4 + 1], s[e4 + 2], s[e4 + 3], 0.0, Fv);
-    }
-#pragma unroll
-    for (int m = 0; m < NV; ++m) F[f0_idx(b, npde, S, i, j, k, m + 1, n)] = Fv[m];
+    for (int m = ADD ? 1 : 0; m < NV; ++m) F[o + m * st] = ADD ? F[o + m * st] + Fv[m] : Fv[m];
   }
 }
 
-// every face flux of the k-omega stage in one launch: grid (x, block, 6),
-// z = family - 1 for the convective fluxes (muscl + roflux) and 3 + family - 1
-// for the viscous ones, each into its own plane of rf (n0 npde S doubles per
-// plane); fd holds the three families' face wall distances (BSL/SST) or is null
+// the convective face fluxes of the k-omega stage (muscl + roflux), grid (x,
+// block, family), into the three planes of rf (n0 npde S doubles each)
 template <bool MIXED>
-__global__ void __launch_bounds__(128, 3) k_rans_faces(BlockList bs_, const cosa_params *__restrict__ Pp,
-                                                       const int *__restrict__ bct, const double *__restrict__ q,
-                                                       int nl, const double *__restrict__ si,
-                                                       const double *__restrict__ sj, const double *__restrict__ sk,
-                                                       const double *__restrict__ h0, const double *__restrict__ mut,
-                                                       const double *__restrict__ vm, int64_t n0,
-                                                       const double *__restrict__ fd, double *__restrict__ rf,
-                                                       FaceVel fvel = FaceVel{{nullptr, nullptr, nullptr}}) {
+__global__ void __launch_bounds__(128, kRansCtas)
+k_rans_conv(BlockList bs_, const cosa_params *__restrict__ Pp, const PhysPar ph, const int *__restrict__ bct,
+            const double *__restrict__ q, int nl, const double *__restrict__ si, const double *__restrict__ sj,
+            const double *__restrict__ sk, const double *__restrict__ h0, int64_t n0, double *__restrict__ rf,
+            FaceVel fvel) {
   const DevBlock b = bs_.get();
   const cosa_params &P = *Pp;
-  const int S = 2 * P.nharms + 1, z = blockIdx.z, d = z % 3 + 1;
-  const double *s = d == 1 ? si : (d == 2 ? sj : sk);
-  double *F = rf + (int64_t)z * n0 * P.npde * S;
-  if (z < 3) {
-    const double *h0b = h0 + ((int64_t)blockIdx.y * 3 + (d - 1)) * S * 2;
-    const double *fv = fvel.f[d - 1];
-    if (d == 1) rans_conv_faces<1, MIXED>(b, P, bct, q, nl, s, h0b, F, fv);
-    else if (d == 2) rans_conv_faces<2, MIXED>(b, P, bct, q, nl, s, h0b, F, fv);
-    else rans_conv_faces<3, MIXED>(b, P, bct, q, nl, s, h0b, F, fv);
-  } else {
-    const double *fdd = fd ? fd + (int64_t)(d - 1) * n0 : nullptr;
-    if (d == 1) rans_visc_faces<1>(b, blockIdx.y, P, bct, q, mut, vm, n0, s, fdd, F);
-    else if (d == 2) rans_visc_faces<2>(b, blockIdx.y, P, bct, q, mut, vm, n0, s, fdd, F);
-    else rans_visc_faces<3>(b, blockIdx.y, P, bct, q, mut, vm, n0, s, fdd, F);
-  }
+  const int S = 2 * P.nharms + 1, d = blockIdx.z + 1;
+  double *F = rf + (int64_t)(d - 1) * n0 * P.npde * S;
+  const double *h0b = h0 + ((int64_t)blockIdx.y * 3 + (d - 1)) * S * 2;
+  if (d == 1) rans_conv_faces<1, MIXED>(b, P, ph, bct, q, nl, si, h0b, F, fvel.f[0]);
+  else if (d == 2) rans_conv_faces<2, MIXED>(b, P, ph, bct, q, nl, sj, h0b, F, fvel.f[1]);
+  else rans_conv_faces<3, MIXED>(b, P, ph, bct, q, nl, sk, h0b, F, fvel.f[2]);
+}
+// the viscous ones, added to the same planes (the cell pass then reads three
+// planes instead of six); fd holds the three families' face wall distances
+// (BSL/SST) or is null.  Bound by FP64 latency and the stencil's loads (ten
+// cells a face, from L1); with the convective faces in one kernel both took 168
+// registers and 12 warps per SM, 165 us a stage with the reference's divisions
+// and 119 us without on the 512 x 128 x 2 aerofoil grid
+__global__ void __launch_bounds__(128, kRansCtas)
+k_rans_visc(BlockList bs_, const cosa_params *__restrict__ Pp, const VisK vk, const int *__restrict__ bct,
+            const double *__restrict__ q, const double *__restrict__ si, const double *__restrict__ sj,
+            const double *__restrict__ sk, const double *__restrict__ mut, const double *__restrict__ vm, int64_t n0,
+            const double *__restrict__ fd, double *__restrict__ rf) {
+  const DevBlock b = bs_.get();
+  const cosa_params &P = *Pp;
+  const int S = 2 * P.nharms + 1, d = blockIdx.z + 1;
+  double *F = rf + (int64_t)(d - 1) * n0 * P.npde * S;
+  const double *fdd = fd ? fd + (int64_t)(d - 1) * n0 : nullptr;
+  if (d == 1) rans_visc_faces<1, 7, true>(b, blockIdx.y, P, bct, q, mut, vm, n0, si, fdd, vk, F);
+  else if (d == 2) rans_visc_faces<2, 7, true>(b, blockIdx.y, P, bct, q, mut, vm, n0, sj, fdd, vk, F);
+  else rans_visc_faces<3, 7, true>(b, blockIdx.y, P, bct, q, mut, vm, n0, sk, fdd, vk, F);
 }
 
 // bresid of the three families on the summed convective + viscous face
-// fluxes of k_rans_faces (visc = 0: the convective ones alone), families in
-// the reference's order (src/cosa.f90:1149-1200)
+// fluxes of the low-speed preconditioned stage (visc = 0: the convective ones
+// alone), families in the reference's order (src/cosa.f90:1149-1200)
 __global__ void k_rans_resid(BlockList bs_, const cosa_params *__restrict__ Pp, int64_t n0,
                              const double *__restrict__ rf, double *__restrict__ res, int visc = 1) {
   const DevBlock b = bs_.get();
@@ -868,73 +900,110 @@ __global__ void k_rans_resid(BlockList bs_, const cosa_params *__restrict__ Pp, 
   }
 }
 
+// start of a k-omega iteration (or of a stage whose state is conservative):
+// q^n kept (qold, if given), cons2prim and bprtest of the interior
+__global__ void k_rans_prim(BlockList bs_, const cosa_params *__restrict__ Pp, double *__restrict__ q,
+                            double *__restrict__ qold, int *status) {
+  const DevBlock b = bs_.get();
+  const cosa_params &P = *Pp;
+  const int S = 2 * P.nharms + 1;
+  int st = 0;
+  KOM_CELL_LOOP
+    const int64_t o = p3_var(b, 7, S, 1, n) + p3_cell(b, i, j, k);
+    double v[7];
+#pragma unroll
+    for (int m = 0; m < 7; ++m) v[m] = q[o + m * b.P3];
+    if (qold) {
+#pragma unroll
+      for (int m = 0; m < 7; ++m) qold[o + m * b.P3] = v[m];
+    }
+    c2p7_nr(P.gamma, v);
+    if (v[4] <= P.qmin[4]) st |= COSA_ERR_NEG_P;
+    else if (v[0] <= P.qmin[0]) st |= COSA_ERR_NEG_RHO;
+#pragma unroll
+    for (int m = 1; m < 7; ++m) q[o + m * b.P3] = v[m];
+  }
+  if (st) atomicOr(status, st);
+}
+
 // update_b of the k-omega stage in one pass (src/update.f90:568-640): the
 // point-implicit rho omega / rho k of k_update_kom, the mean-flow update
-// q = q^n - ar R dt/V, and with ifixq the floors of fixq_b
-template <class BS>
-__global__ void k_update_rans(BS bs_, const cosa_params *__restrict__ Pp, const double *__restrict__ res,
+// q = q^n - ar R dt/V, and with ifixq the floors of fixq_b.  PRIM_IN: q's
+// interior holds the stage's primitive state (k and omega as they are);
+// PRIM_OUT: the new state is stored primitive, tested like bprtest does
+template <bool PRIM_IN, bool PRIM_OUT>
+__global__ void k_update_rans(BlockList bs_, const cosa_params *__restrict__ Pp, const double *__restrict__ res,
                               double *__restrict__ q, const double *__restrict__ qold,
                               const double *__restrict__ vol, const double *__restrict__ dtt,
                               const double *__restrict__ dtv, const double *__restrict__ delpls,
-                              const double *__restrict__ prd, double ar, const double *__restrict__ ttrm) {
+                              const double *__restrict__ prd, double ar, const double *__restrict__ ttrm,
+                              int *status) {
   const DevBlock b = bs_.get();
   const cosa_params &P = *Pp;
-  const int npde = P.npde, S = 2 * P.nharms + 1;
+  const int S = 2 * P.nharms + 1;
+  int st = 0;
   KOM_CELL_LOOP
+    const int64_t P3 = b.P3, c = p3_cell(b, i, j, k), o = p3s_idx(b, S, i, j, k, n), o1 = p1_idx(b, S, i, j, k, n);
+    const int64_t i1 = p3_var(b, 7, S, 1, n) + c;
+    double q0[7], r[7], w[7];
+#pragma unroll
+    for (int m = 0; m < 7; ++m) { q0[m] = qold[i1 + m * P3]; r[m] = res[i1 + m * P3]; }
+    const double rho = q[i1], qk = q[i1 + 5 * P3], qw = q[i1 + 6 * P3];
+    const double dp = delpls[o], pr = prd[o], dt = dtt[o1], dm = dtv[o1], vl = vol[p1_idx(b, 1, i, j, k, 0)];
     const double gav = ttrm ? ttrm[ttrm_idx(b, S, i, j, k, 2, n)] : P.gkw;
     const double bav = ttrm ? ttrm[ttrm_idx(b, S, i, j, k, 3, n)] : P.bkw;
-    const int64_t c = p3_cell(b, i, j, k), o = p3s_idx(b, S, i, j, k, n);
-    const int64_t i1 = p3_var(b, npde, S, 1, n) + c, i6 = p3_var(b, npde, S, 6, n) + c, i7 = p3_var(b, npde, S, 7, n) + c;
-    const double rho = q[i1], ome = q[i7] / q[i1], tke = q[i6] / q[i1];
-    const double dt = dtt[p1_idx(b, S, i, j, k, n)];
-    const double dtau = dt * vol[p1_idx(b, 1, i, j, k, 0)];
-    const double dp = delpls[o];
-    double rhomega = (qold[i7] - ar * res[i7] * dt + ar * dtau * rho * ome * (gav * dp + 2 * bav * ome)) /
-                     (1 + ar * dtau * (gav * dp + 2 * bav * ome));
-    const double rhomegamin = gav * P.cmu * rho * sqrt(prd[o]);
+    const double ir = PRIM_IN ? 1.0 : rcp_nr(rho);
+    const double ome = qw * ir, tke = qk * ir;
+    const double dtau = ar * dt * vl;
+    const double dw_ = dtau * (gav * dp + 2 * bav * ome), dk_ = dtau * (dp + P.bstrkw * ome);
+    double rhomega = (q0[6] - ar * r[6] * dt + rho * ome * dw_) * rcp_nr(1 + dw_);
+    const double rhomegamin = gav * P.cmu * rho * sqrt(pr);
     if (rhomega < rhomegamin) rhomega = rhomegamin;
     const double drhomega = rhomega - rho * ome;
-    double rk = (qold[i6] - ar * res[i6] * dt + ar * dtau * rho * tke * (dp + P.bstrkw * ome) -
-                 ar * dtau * P.bstrkw * tke * drhomega) /
-                (1 + ar * dtau * (dp + P.bstrkw * ome));
-    const double dm = dtv[p1_idx(b, S, i, j, k, n)];
-    double rho1 = rho;
+    double rk = (q0[5] - ar * r[5] * dt + rho * tke * dk_ - dtau * P.bstrkw * tke * drhomega) * rcp_nr(1 + dk_);
 #pragma unroll
-    for (int m = 1; m <= 5; ++m) {
-      const int64_t om = p3_var(b, npde, S, m, n) + c;
-      const double v = qold[om] - ar * res[om] * dm;
-      q[om] = v;
-      if (m == 1) rho1 = v;
-    }
+    for (int m = 0; m < 5; ++m) w[m] = q0[m] - ar * r[m] * dm;
     if (P.ifixq) {
       // fixq_b (src/update.f90:2216-2269) on the updated cell
-      if (rk / rho1 < P.qmin[5]) rk = rho1 * P.qmin[5];
-      if (rhomega / rho1 < P.qmin[6]) rhomega = rho1 * P.qmin[6];
+      if (rk < w[0] * P.qmin[5]) rk = w[0] * P.qmin[5];
+      if (rhomega < w[0] * P.qmin[6]) rhomega = w[0] * P.qmin[6];
     }
-    q[i6] = rk;
-    q[i7] = rhomega;
+    w[5] = rk;
+    w[6] = rhomega;
+    if (PRIM_OUT) {
+      c2p7_nr(P.gamma, w);
+      if (w[4] <= P.qmin[4]) st |= COSA_ERR_NEG_P;
+      else if (w[0] <= P.qmin[0]) st |= COSA_ERR_NEG_RHO;
+    }
+#pragma unroll
+    for (int m = 0; m < 7; ++m) q[i1 + m * P3] = w[m];
   }
+  if (PRIM_OUT && st) atomicOr(status, st);
 }
 
 // the cell side of the k-omega stage in one pass over the cells
-// (src/cosa.f90:1878-1901): q_face + q_der_c of the three families (the
-// differences still written to dx, dy, dz), turprod_b on the levels that
-// compute production (else the restricted prd and div u are read), under
-// BSL/SST update_ttrm_b, and srckw_b / srckw_sst_b into res; the state is
-// primitive
+// (src/cosa.f90:1797-1824, 1878-1922): bresid of the three families' fluxes,
+// q_face + q_der_c of the three families (the differences written to dx, dy,
+// dz where given: SST's eddy viscosity reads the last stage's),
+// turprod_b on the levels that compute production (else the restricted prd
+// and div u are read), under BSL/SST update_ttrm_b, srckw_b / srckw_sst_b,
+// and (hb) src_bhb of the conservative snapshots; the state is primitive, res
+// is written once
 template <bool BLEND>
-__global__ void k_rans_cellsrc(BlockList bs_, const cosa_params *__restrict__ Pp, int nl, const int *__restrict__ bct,
-                               const double *__restrict__ q, double *__restrict__ dx, double *__restrict__ dy,
-                               double *__restrict__ dz, const double *__restrict__ vm, int64_t n0,
-                               const double *__restrict__ mut, const double *__restrict__ dist,
-                               const double *__restrict__ vol, double *__restrict__ prd, double *__restrict__ divvel,
-                               double *__restrict__ delpls, double *__restrict__ ttrm, double *__restrict__ res) {
+__global__ void __launch_bounds__(128, kRansCtas)
+k_rans_cell(BlockList bs_, const cosa_params *__restrict__ Pp, const VisK V, int nl, const int *__restrict__ bct,
+            const double *__restrict__ q, const double *__restrict__ rf, double *__restrict__ dx,
+            double *__restrict__ dy, double *__restrict__ dz, const double *__restrict__ vm, int64_t n0,
+            const double *__restrict__ mut, const double *__restrict__ dist, const double *__restrict__ vol,
+            double *__restrict__ prd, double *__restrict__ divvel, double *__restrict__ delpls,
+            double *__restrict__ ttrm, double *__restrict__ res, int hb) {
   const DevBlock b = bs_.get();
   const cosa_params &P = *Pp;
   const int npde = P.npde, S = 2 * P.nharms + 1;
   constexpr int vhi = BLEND ? 7 : 4;
   const bool own_prod = nl == 1 || P.prd_all_lvls;
-  const double fact = 2.0 / 3.0, mor = P.machfs / P.reyno;
+  const double fact = 2.0 / 3.0, mor = V.mr;
+  const int64_t plane = n0 * npde * S;
   KOM_CELL_LOOP
     const int64_t c0 = p3_cell(b, i, j, k), o = p3s_idx(b, S, i, j, k, n);
     // dc[d][v - 2]: differences of u, v, w (and k, omega) across the cell
@@ -957,7 +1026,7 @@ __global__ void k_rans_cellsrc(BlockList bs_, const cosa_params *__restrict__ Pp
         const double flo = wlo ? qm : (qm + qc) / 2;
         const double fhi = whi ? qp : (qc + qp) / 2;
         dc[d - 1][v - 2] = fhi - flo;
-        dd[ov + c0] = dc[d - 1][v - 2];
+        if (dd) dd[ov + c0] = dc[d - 1][v - 2];
       }
     }
     double met[3][3];
@@ -986,9 +1055,8 @@ __global__ void k_rans_cellsrc(BlockList bs_, const cosa_params *__restrict__ Pp
     double cdif = 0.0, gav = P.gkw, bav = P.bkw;
     if (BLEND) {
       // update_ttrm_b (src/update.f90:3036-3161)
-      const BlendPar cb = make_blend(P);
-      const double tt = P.gamma * Q(5) / rho;
-      const double mu = sutherland(tt, P.stemp);
+      const double ir = rcp_nr(rho);
+      const double mu = sutherland_nr(P.gamma * Q(5) * ir, P.stemp);
       const double tkexi = dc[0][4], tkeeta = dc[1][4], tkezeta = dc[2][4];
       const double omexi = dc[0][5], omeeta = dc[1][5], omezeta = dc[2][5];
       const double dtkedx = tkexi * met[0][0] + tkeeta * met[1][0] + tkezeta * met[2][0];
@@ -998,11 +1066,12 @@ __global__ void k_rans_cellsrc(BlockList bs_, const cosa_params *__restrict__ Pp
       const double domedy = omexi * met[0][1] + omeeta * met[1][1] + omezeta * met[2][1];
       const double domedz = omexi * met[0][2] + omeeta * met[1][2] + omezeta * met[2][2];
       double cdt;
-      const double f1 = blend_f1(cb, P, rho, tke, ome, mu, dtkedx * domedx + dtkedy * domedy + dtkedz * domedz,
-                                 dist[p1_idx(b, 1, i, j, k, 0)], cdt);
+      const double f1 = blend_f1_nr(V, rho, ir, tke, rcp_nr(ome), mu,
+                                    dtkedx * domedx + dtkedy * domedy + dtkedz * domedz,
+                                    dist[p1_idx(b, 1, i, j, k, 0)], cdt);
       cdif = cdt * (1 - f1);
-      gav = f1 * cb.g1 + (1 - f1) * cb.g2;
-      bav = f1 * cb.b1 + (1 - f1) * cb.b2;
+      gav = f1 * V.g1 + (1 - f1) * V.g2;
+      bav = f1 * V.b1 + (1 - f1) * V.b2;
       ttrm[ttrm_idx(b, S, i, j, k, 1, n)] = cdif;
       ttrm[ttrm_idx(b, S, i, j, k, 2, n)] = gav;
       ttrm[ttrm_idx(b, S, i, j, k, 3, n)] = bav;
@@ -1018,11 +1087,39 @@ __global__ void k_rans_cellsrc(BlockList bs_, const cosa_params *__restrict__ Pp
       }
     }
     const double v = vol[p1_idx(b, 1, i, j, k, 0)];
-    double *r6 = res + p3_var(b, npde, S, 6, n) + c0, *r7 = res + p3_var(b, npde, S, 7, n) + c0;
-    *r6 = *r6 - v * (mor * mt * prodk - fact * divv * rho * tke - P.bstrkw * rho * tke * ome);
+    // bresid (families in the reference's order, src/cosa.f90:1149-1200)
+    const int64_t st = (int64_t)b.im * b.jm * b.km, sj_ = b.im, sk_ = (int64_t)b.im * b.jm;
+    const double *f0 = rf + f0_idx(b, 7, S, i, j, k, 1, n);
+    double r[7];
+#pragma unroll
+    for (int m = 0; m < 7; ++m) {
+      const double *f = f0 + m * st;
+      const double x = f[1] - f[0] + f[plane + sj_] - f[plane];
+      r[m] = x + f[2 * plane + sk_] - f[2 * plane];
+    }
+    r[5] = r[5] - v * (mor * mt * prodk - fact * divv * rho * tke - P.bstrkw * rho * tke * ome);
     if (BLEND)
-      *r7 = *r7 - v * (gav * P.cmu * rho * prodw - gav * fact * divv * rho * ome - bav * rho * (ome * ome) + cdif);
+      r[6] = r[6] - v * (gav * P.cmu * rho * prodw - gav * fact * divv * rho * ome - bav * rho * (ome * ome) + cdif);
     else
-      *r7 = *r7 - v * (P.gkw * P.cmu * rho * prodw - P.gkw * fact * divv * rho * ome - P.bkw * rho * (ome * ome));
+      r[6] = r[6] - v * (P.gkw * P.cmu * rho * prodw - P.gkw * fact * divv * rho * ome - P.bkw * rho * (ome * ome));
+    if (hb) {
+      // src_bhb (src/src.f90:556-613) of the snapshots' conservative values
+      for (int n2 = 0; n2 < S; ++n2) {
+        const double *qs = q + p3_var(b, 7, S, 1, n2) + c0;
+        const double w = P.omega * v * P.dhb[n * S + n2];
+        const double r2 = qs[0], u2 = qs[b.P3], v2 = qs[2 * b.P3], w2 = qs[3 * b.P3], p2 = qs[4 * b.P3];
+        const double k2 = qs[5 * b.P3], o2 = qs[6 * b.P3];
+        r[0] = r[0] + w * r2;
+        r[1] = r[1] + w * (r2 * u2);
+        r[2] = r[2] + w * (r2 * v2);
+        r[3] = r[3] + w * (r2 * w2);
+        r[4] = r[4] + w * (p2 * V.igm1 + r2 * (0.5 * (u2 * u2 + v2 * v2 + w2 * w2) + k2));
+        r[5] = r[5] + w * (r2 * k2);
+        r[6] = r[6] + w * (r2 * o2);
+      }
+    }
+    double *ro = res + p3_var(b, 7, S, 1, n) + c0;
+#pragma unroll
+    for (int m = 0; m < 7; ++m) ro[m * b.P3] = r[m];
   }
 }

@@ -98,7 +98,7 @@ __global__ void k_rest3(DevBlock b1, DevBlock b2, int S, const double *__restric
   const int ni = (b1.im - 1) / 2, nj = (b1.jm - 1) / 2, nk = (b1.km - 1) / 2;
   const int64_t total = (int64_t)ni * nj * nk * S;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-    int64_t r = t;
+    Dec r(t);
     const int i2 = (int)(r % ni) + 1; r /= ni;
     const int j2 = (int)(r % nj) + 1; r /= nj;
     const int k2 = (int)(r % nk) + 1;
@@ -255,16 +255,16 @@ __global__ void __launch_bounds__(128, 3) k_lsp_faces(BlockList bs_, const cosa_
                                                       const double *__restrict__ si, const double *__restrict__ sj,
                                                       const double *__restrict__ sk, const double *__restrict__ cpg,
                                                       const double *__restrict__ cvs, const double *__restrict__ vm,
-                                                      int64_t n0, double *__restrict__ rf) {
+                                                      int64_t n0, const VisK vk, double *__restrict__ rf) {
   const DevBlock b = bs_.get();
   const cosa_params &P = *Pp;
   const int npde = P.npde, S = 2 * P.nharms + 1, z = blockIdx.z, d = z % 3 + 1;
   const double *s = d == 1 ? si : (d == 2 ? sj : sk);
   double *F = rf + (int64_t)z * n0 * npde * S;
   if (z >= 3) {
-    if (d == 1) rans_visc_faces<1, 5>(b, blockIdx.y, P, bct, q, nullptr, vm, n0, s, nullptr, F);
-    else if (d == 2) rans_visc_faces<2, 5>(b, blockIdx.y, P, bct, q, nullptr, vm, n0, s, nullptr, F);
-    else rans_visc_faces<3, 5>(b, blockIdx.y, P, bct, q, nullptr, vm, n0, s, nullptr, F);
+    if (d == 1) rans_visc_faces<1, 5>(b, blockIdx.y, P, bct, q, nullptr, vm, n0, s, nullptr, vk, F);
+    else if (d == 2) rans_visc_faces<2, 5>(b, blockIdx.y, P, bct, q, nullptr, vm, n0, s, nullptr, vk, F);
+    else rans_visc_faces<3, 5>(b, blockIdx.y, P, bct, q, nullptr, vm, n0, s, nullptr, vk, F);
     return;
   }
   const double eps2 = P.epsp[nl - 1] * P.epsp[nl - 1];

@@ -156,31 +156,33 @@ __device__ __forceinline__ double edge_fit(const int x[4], const int y[4], doubl
 }
 // one thread per (edge cell, variable, snapshot); nvar variables of stride
 // P3 per snapshot (q: npde, mut: 1)
+// edge cell r (0 .. 4 (nk + nj + ni) - 1) of one variable plane a of block b
+__device__ __forceinline__ void edge_cell(const DevBlock &b, int r, double *__restrict__ a) {
+  const int nk = b.km - 1, nj = b.jm - 1;
+  int fam;
+  if (r < 4 * nk) fam = 0;
+  else if ((r -= 4 * nk) < 4 * nj) fam = 1;
+  else { r -= 4 * nj; fam = 2; }
+  const int ic = r & 3, tt = (r >> 2) + 1;
+  const int m1 = fam == 2 ? b.jm : b.im, m2 = fam == 0 ? b.jm : b.km;
+  int x[4], y[4];
+  edge_pts(ic, m1, m2, x, y);
+  auto at = [&](int p) -> int64_t {
+    if (fam == 0) return p3_cell(b, x[p], y[p], tt);
+    if (fam == 1) return p3_cell(b, x[p], tt, y[p]);
+    return p3_cell(b, tt, x[p], y[p]);
+  };
+  a[at(0)] = edge_fit(x, y, a[at(1)], a[at(2)], a[at(3)]);
+}
 template <class BS>
 __global__ void k_edges(BS bs_, int nvar, int S, double *__restrict__ q, int64_t base) {
   const DevBlock b = bs_.get();
   if (base < 0) base = b.op3 * nvar * S;  // multi-block launch: the block's own offset
-  const int nk = b.km - 1, nj = b.jm - 1;
-  const int64_t per = 4 * ((int64_t)nk + nj + (b.im - 1));
-  const int64_t total = per * nvar * S;
+  const int per = 4 * ((b.km - 1) + (b.jm - 1) + (b.im - 1));
+  const int64_t total = (int64_t)per * nvar * S;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-    int64_t r = t % per;
-    const int64_t vn = t / per;
-    double *a = q + base + vn * b.P3;
-    int fam;
-    if (r < 4 * (int64_t)nk) fam = 0;
-    else if ((r -= 4 * (int64_t)nk) < 4 * (int64_t)nj) fam = 1;
-    else { r -= 4 * (int64_t)nj; fam = 2; }
-    const int ic = (int)(r % 4), tt = (int)(r / 4) + 1;
-    const int m1 = fam == 2 ? b.jm : b.im, m2 = fam == 0 ? b.jm : b.km;
-    int x[4], y[4];
-    edge_pts(ic, m1, m2, x, y);
-    auto at = [&](int p) -> int64_t {
-      if (fam == 0) return p3_cell(b, x[p], y[p], tt);
-      if (fam == 1) return p3_cell(b, x[p], tt, y[p]);
-      return p3_cell(b, tt, x[p], y[p]);
-    };
-    a[at(0)] = edge_fit(x, y, a[at(1)], a[at(2)], a[at(3)]);
+    const Dec d(t);
+    edge_cell(b, d % per, q + base + (d / per) * b.P3);
   }
 }
 

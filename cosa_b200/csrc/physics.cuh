@@ -84,6 +84,13 @@ __device__ __forceinline__ void c2p7(double g, double *q) {
   q[1] = u; q[2] = v; q[3] = w; q[5] = tke; q[6] = q[6] / rho;
   q[4] = (g - 1) * (q[4] - rho * (u * u + v * v + w * w) / 2 - rho * tke);
 }
+// c2p7 with one reciprocal of rho (fused k-omega stage)
+__device__ __forceinline__ void c2p7_nr(double g, double *q) {
+  const double rho = q[0], ri = rcp_nr(rho);
+  const double u = q[1] * ri, v = q[2] * ri, w = q[3] * ri, k = q[5] * ri;
+  q[1] = u; q[2] = v; q[3] = w; q[5] = k; q[6] = q[6] * ri;
+  q[4] = (g - 1) * (q[4] - rho * (0.5 * (u * u + v * v + w * w) + k));
+}
 __device__ __forceinline__ void p2c(double g, double *q, int npde) {
   const double tke = npde > 5 ? q[5] : 0.0;
   const double rho = q[0];
@@ -440,6 +447,92 @@ __device__ __forceinline__ void roe_flux_mixed_tke(const PhysPar &P, double kx, 
   flux[2] = ((rhor * vr * unr + pr * ky) + (rhol * vl * unl + pl * ky) - (double)df3) / 2 * ds;
   flux[3] = ((rhor * wr * unr + pr * kz) + (rhol * wl * unl + pl * kz) - (double)df4) / 2 * ds;
   flux[4] = (rhor * h0r * unr + pr * ubn + rhol * h0l * unl + pl * ubn - (double)df5) / 2 * ds;
+}
+
+// The seven convective fluxes of a k-omega face (roflux_b's mean-flow flux
+// with the turbulent kinetic energy, src/flux.f90:45-238, and the upwinded
+// rho k u_n and rho omega u_n with the turbulence entropy-fix settings,
+// src/flux.f90:240-330) on roe_flux_euler's arithmetic: the Roe averages are
+// computed once for both, four reciprocal roots and one reciprocal where the
+// two routines of the reference take six roots and seventeen divisions.
+// h0l/h0r: the values the mean-flow loop left behind, those of the block's
+// last face of the snapshot (the reference does not recompute them in the
+// turbulence loop); ubn: the face's normal grid speed (0 on fixed grids)
+__device__ __forceinline__ void roe_flux_rans(const PhysPar &P, const cosa_params &C, double kx, double ky, double kz,
+                                              double ds, const double *qr, const double *ql, double h0r, double h0l,
+                                              double ubn, double *flux) {
+  auto mul = [](double a, double b) { return __dmul_rn(a, b); };
+  auto add = [](double a, double b) { return __dadd_rn(a, b); };
+  auto sub = [](double a, double b) { return __dsub_rn(a, b); };
+  auto mad = [](double a, double b, double c) { return __fma_rn(a, b, c); };
+  auto fix = [](double r, double d) { return r <= d ? 0.5 * (r * r + d * d) / d : r; };
+  const double rhor = qr[0], ur = qr[1], vr = qr[2], wr = qr[3], pr = qr[4];
+  const double rhol = ql[0], ul = ql[1], vl = ql[2], wl = ql[3], pl = ql[4];
+  const double rsr = rsqrt_nr(rhor), rsl = rsqrt_nr(rhol);
+  const double unr = sub(mad(wr, kz, mad(vr, ky, mul(ur, kx))), ubn);
+  const double unl = sub(mad(wl, kz, mad(vl, ky, mul(ul, kx))), ubn);
+  const double er = mad(rhor, mad(0.5, mad(wr, wr, mad(vr, vr, mul(ur, ur))), qr[5]), mul(P.g_gm1, pr));
+  const double el = mad(rhol, mad(0.5, mad(wl, wl, mad(vl, vl, mul(ul, ul))), ql[5]), mul(P.g_gm1, pl));
+  const double du = sub(ur, ul), dv = sub(vr, vl), dw = sub(wr, wl), dun = sub(unr, unl);
+  const double dk = sub(qr[5], ql[5]), dom = sub(qr[6], ql[6]);
+  const double srr = mul(rhor, rsr), srl = mul(rhol, rsl);
+  const double rden = rcp_nr(add(srl, srr));
+  const double wgt = mul(srr, rden);
+  const double u = mad(wgt, du, ul), v = mad(wgt, dv, vl), w = mad(wgt, dw, wl), un = mad(wgt, dun, unl);
+  const double tke = mad(wgt, dk, ql[5]), ome = mad(wgt, dom, ql[6]);
+  const double h0 = mul(mad(er, rsr, mul(el, rsl)), rden);
+  const double h0t = mul(mad(srr, h0r, mul(srl, h0l)), rden);
+  const double ek = mad(0.5, mad(w, w, mad(v, v, mul(u, u))), tke);
+  const double a2 = mul(P.gm1, sub(h0, ek)), at2 = mul(P.gm1, sub(h0t, ek));
+  const double ra = rsqrt_nr(a2), a = mul(a2, ra), rat = rsqrt_nr(at2), at = mul(at2, rat);
+  double e1 = fabs(un), e4 = fabs(add(un, a)), e5 = fabs(sub(un, a));
+  double t1 = e1, t4 = fabs(add(un, at)), t5 = fabs(sub(un, at));
+  if (P.efx_setup_f) {
+    const double d = fmax(1.0e-12, P.cntrpy_f * (P.w1 * P.entfxctf_f + P.w2 * (sqrt(2 * (ek - tke)) + a) +
+                                                 P.w3 * 0.2 * (fabs(un + ubn) + a + fabs(ubn))));
+    if (P.efx_all_f) e1 = fix(e1, d);
+    e4 = fix(e4, d); e5 = fix(e5, d);
+  }
+  if (P.eig_limit_f) {
+    e1 = fmax(e1, P.eig_cutoff_f);
+    if (P.eig_lim_all_f) { e4 = fmax(e4, P.eig_cutoff_f); e5 = fmax(e5, P.eig_cutoff_f); }
+  }
+  if (C.efx_setup_t) {
+    const double d = fmax(1.0e-12, C.cntrpy_t * (C.entfx_t_w[0] * C.entfxctf_t +
+                                                 C.entfx_t_w[1] * (sqrt(2 * (ek - tke)) + at) +
+                                                 C.entfx_t_w[2] * 0.2 * (fabs(un + ubn) + at + fabs(ubn))));
+    if (C.efx_all_t) t1 = fix(t1, d);
+    t4 = fix(t4, d); t5 = fix(t5, d);
+  }
+  if (C.eig_limit_t) {
+    t1 = fmax(t1, C.eig_cutoff_t);
+    if (C.eig_lim_all_t) { t4 = fmax(t4, C.eig_cutoff_t); t5 = fmax(t5, C.eig_cutoff_t); }
+  }
+  const double drho = sub(rhor, rhol), dp = sub(pr, pl), rho = mul(srl, srr), rdu = mul(rho, dun);
+  const double hds = mul(0.5, ds);
+  const double mr = mul(rhor, unr), ml = mul(rhol, unl);
+  {
+    const double dpa2 = mul(dp, mul(rat, rat)), rdua = mul(rdu, rat);
+    const double b34 = mad(mul(0.5, t4), add(dpa2, rdua), mul(mul(0.5, t5), sub(dpa2, rdua)));
+    const double b1 = mad(t1, sub(drho, dpa2), b34), b2 = mul(t1, rho);
+    flux[5] = mul(mad(-b2, dk, mad(-b1, tke, mad(mr, qr[5], mul(ml, ql[5])))), hds);
+    flux[6] = mul(mad(-b2, dom, mad(-b1, ome, mad(mr, qr[6], mul(ml, ql[6])))), hds);
+  }
+  const double dpa2 = mul(dp, mul(ra, ra)), rdua = mul(rdu, ra);
+  const double al1 = mul(e1, sub(drho, dpa2)), al2 = mul(e1, rho);
+  const double al3 = mul(mul(0.5, e4), add(dpa2, rdua)), al4 = mul(mul(0.5, e5), sub(dpa2, rdua));
+  const double a34 = add(al3, al4), df1 = add(al1, a34), c2 = mad(-al2, dun, mul(a, sub(al3, al4)));
+  auto mom = [&](double xr, double xl, double xa, double dx, double k) {
+    const double f = add(mad(mr, xr, mul(pr, k)), mad(ml, xl, mul(pl, k)));
+    return mul(sub(f, mad(df1, xa, mad(al2, dx, mul(c2, k)))), hds);
+  };
+  flux[0] = mul(sub(add(mr, ml), df1), hds);
+  flux[1] = mom(ur, ul, u, du, kx);
+  flux[2] = mom(vr, vl, v, dv, ky);
+  flux[3] = mom(wr, wl, w, dw, kz);
+  const double udu = add(mad(w, dw, mad(v, dv, mul(u, du))), dk);
+  const double fe = mad(add(pr, pl), ubn, mad(er, unr, mul(el, unl)));
+  flux[4] = mul(mad(-c2, add(un, ubn), mad(-a34, h0, mad(-al1, ek, mad(-al2, udu, fe)))), hds);
 }
 
 // ---- eig_eul (src/cosa.f90:4183-4233); gv: the cell's grid velocity on

@@ -130,7 +130,7 @@ __global__ void k_vmetrix(DevBlock b, int d, const double *__restrict__ x, const
   const int64_t total = (int64_t)ni * nj * nk;
   const int mx = d == 1 ? im : (d == 2 ? jm : km);
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-    int64_t r = t;
+    Dec r(t);
     const int i = (int)(r % ni) + 1; r /= ni;
     const int j = (int)(r % nj) + 1;
     const int k = (int)(r / nj) + 1;
@@ -336,6 +336,98 @@ __device__ __forceinline__ void vflux_face(const ViscPar &V, const double qf[5],
            ds) + (qx * kx + qy * ky + qz * kz) * ds;
 }
 
+// constants of the fused face kernels' viscous fluxes, passed by value
+struct VisK {
+  double g, stemp, mr, cl, ct;  // gamma, Sutherland, M/Re, M/Re/(g-1)/Pr (laminar, turbulent)
+  double turcmp, sigk, sigw;
+  // BSL/SST (make_blend)
+  int blend;
+  double sigk1, sigk2, sigw1, sigw2, b1, b2, g1, g2, epst;
+  double igm1;  // 1/(gamma - 1)
+};
+inline VisK make_visk(const cosa_params &P) {
+  VisK k;
+  k.g = P.gamma; k.stemp = P.stemp; k.mr = P.machfs / P.reyno;
+  k.cl = k.mr / (P.gamma - 1) / P.pranl; k.ct = k.mr / (P.gamma - 1) / P.prant;
+  k.turcmp = P.turcmp; k.sigk = P.sigk; k.sigw = P.sigw;
+  k.blend = P.kom_bsl || P.kom_sst;
+  k.sigk1 = P.kom_sst ? 0.85 : 0.5; k.sigk2 = 1.0; k.sigw1 = 0.5; k.sigw2 = 0.856; k.epst = P.epst;
+  const double bstr = 0.09, kap2 = P.kappa * P.kappa / std::sqrt(bstr);
+  k.b1 = 3.0 / 40.0; k.b2 = 0.0828;
+  k.g1 = k.b1 / bstr - k.sigw1 * kap2; k.g2 = k.b2 / bstr - k.sigw2 * kap2;
+  k.igm1 = 1 / (P.gamma - 1);
+  return k;
+}
+// Sutherland's law with t^1.5 = t^2 / sqrt(t), no division
+__device__ __forceinline__ double sutherland_nr(double t, double stemp) {
+  return (stemp + 1) * rcp_nr(t + stemp) * (t * t * rsqrt_nr(t));
+}
+// F1 of BSL/SST (blend_f1 in kom.cuh) from the reciprocals of rho and omega
+__device__ __forceinline__ double blend_f1_nr(const VisK &V, double rho, double ir, double tke, double io, double mu,
+                                              double gradkw, double dist, double &cdt) {
+  const double id = rcp_nr(dist + V.epst), id2 = id * id;
+  const double a = fmax(sqrt(tke) * (1 / 0.09) * io * id, 500 * mu * V.mr * ir * io * id2);
+  cdt = 2 * rho * V.sigw2 * io * gradkw;
+  const double arg = fmin(a, 4 * rho * V.sigw2 * tke * id2 * rcp_nr(fmax(cdt, 1.0e-20)));
+  const double a2 = arg * arg;
+  const double e = exp(2 * fmin(a2 * a2, 1.0e2));
+  return (e - 1) * rcp_nr(e + 1);
+}
+// Viscous flux of one face with NV = 5 (laminar: vflux_face's terms) or NV =
+// 7 (k-omega: rtst_face and vflux_kom_face with the face's eddy viscosity mut
+// and, under BSL/SST, its wall distance fd), their sums collected: laminar and
+// Reynolds stresses share the velocity gradients, the temperature gradient is
+// t/p grad p - t/rho grad rho = (g grad p - t grad rho) / rho, and two
+// reciprocals and a reciprocal root replace the fifteen divisions and the root
+// of the reference's form.  The energy row keeps its (u txy + v tyy + w tyz)
+// kz term, the omega row its dk/dz.
+template <int NV>
+__device__ __forceinline__ void visc_flux(const VisK &V, const double *qf, const double (*g)[NV], const double *vmf,
+                                          double kx, double ky, double kz, double ds, double mut, double fd, double *F) {
+  const double rho = qf[0], u = qf[1], v = qf[2], w = qf[3], ir = rcp_nr(rho);
+  const double t = V.g * qf[4] * ir;
+  const double mu = sutherland_nr(t, V.stemp);
+  auto ddx = [&](int m, int c) { return g[0][m] * vmf[c] + g[1][m] * vmf[3 + c] + g[2][m] * vmf[6 + c]; };
+  const double ux = ddx(1, 0), uy = ddx(1, 1), uz = ddx(1, 2), vx = ddx(2, 0), vy = ddx(2, 1), vz = ddx(2, 2);
+  const double wx = ddx(3, 0), wy = ddx(3, 1), wz = ddx(3, 2);
+  const double div = ux + vy + wz;
+  // 2 (mu + mut) S_ij M/Re, the trace terms of the two parts apart (turcmp)
+  const double ml = V.mr * mu, mm = NV == 7 ? V.mr * (mu + mut) : ml;
+  double tr = ml * div * (2.0 / 3.0), trl = tr;
+  if (NV == 7) tr = tr + (V.mr * mut * V.turcmp * div + rho * qf[5]) * (2.0 / 3.0);
+  const double txx = 2 * mm * ux - tr, tyy = 2 * mm * vy - tr, tzz = 2 * mm * wz - tr;
+  const double txy = mm * (uy + vx), txz = mm * (uz + wx), tyz = mm * (vz + wy);
+  F[0] = 0.0;
+  F[1] = -((txx * kx + txy * ky + txz * kz) * ds);
+  F[2] = -((txy * kx + tyy * ky + tyz * kz) * ds);
+  F[3] = -((txz * kx + tyz * ky + tzz * kz) * ds);
+  // heat flux and the work of the laminar stresses
+  const double gx = V.g * g[0][4] - t * g[0][0], ge = V.g * g[1][4] - t * g[1][0], gz = V.g * g[2][4] - t * g[2][0];
+  const double nx = vmf[0] * kx + vmf[1] * ky + vmf[2] * kz, ne = vmf[3] * kx + vmf[4] * ky + vmf[5] * kz;
+  const double nz = vmf[6] * kx + vmf[7] * ky + vmf[8] * kz;
+  const double dtn = (gx * nx + ge * ne + gz * nz) * ir;  // dT/dn
+  const double cq = NV == 7 ? V.cl * mu + V.ct * mut : V.cl * mu;
+  const double lxx = NV == 7 ? 2 * ml * ux - trl : txx, lyy = NV == 7 ? 2 * ml * vy - trl : tyy;
+  const double lxy = NV == 7 ? ml * (uy + vx) : txy, lxz = NV == 7 ? ml * (uz + wx) : txz;
+  const double lyz = NV == 7 ? ml * (vz + wy) : tyz;
+  const double wkx = u * lxx + v * lxy + w * lxz, wky = u * lxy + v * lyy + w * lyz;
+  F[4] = -((wkx * kx + wky * (ky + kz) + cq * dtn) * ds);
+  if constexpr (NV == 7) {
+    const double kxx = ddx(5, 0), kyy = ddx(5, 1), kzz = ddx(5, 2), ox = ddx(6, 0), oy = ddx(6, 1);
+    double sigk = V.sigk, sigw = V.sigw;
+    if (V.blend) {
+      double cdt;
+      const double f1 = blend_f1_nr(V, rho, ir, qf[5], rcp_nr(qf[6]), mu, kxx * ox + kyy * oy + kzz * ddx(6, 2), fd, cdt);
+      sigk = f1 * V.sigk1 + (1 - f1) * V.sigk2;
+      sigw = f1 * V.sigw1 + (1 - f1) * V.sigw2;
+    }
+    const double dk = (mu + sigk * mut) * V.mr * (kxx * kx + kyy * ky + kzz * kz) * ds;
+    F[4] -= dk;
+    F[5] = -dk;
+    F[6] = -((mu + sigw * mut) * V.mr * (ox * kx + oy * ky + kzz * kz) * ds);
+  }
+}
+
 __device__ __forceinline__ void load_vm(const double *__restrict__ vm, const DevBlock &b, int64_t n0, int d, int i,
                                         int j, int k, double vmf[9]) {
 #pragma unroll
@@ -375,7 +467,7 @@ __global__ void k_prim(const DevBlock *__restrict__ blocks, const cosa_params *_
 
 // viscous flux of every face: grid (x, nblocks, 3 families)
 template <int D>
-__device__ __forceinline__ void vface_one(const DevBlock &b, const ViscPar &V, const QView &Q,
+__device__ __forceinline__ void vface_one(const DevBlock &b, const VisK &V, const QView &Q,
                                           const double *__restrict__ s, int S2, const double *__restrict__ vm,
                                           int64_t n0, int i, int j, int k, int nh, double *__restrict__ F) {
   double qf[5], g[3][5], vmf[9], F5[5];
@@ -384,7 +476,7 @@ __device__ __forceinline__ void vface_one(const DevBlock &b, const ViscPar &V, c
   const int64_t e = p2_idx(b, S2, 1, i, j, k, nh);
   const double2 a = __ldg(reinterpret_cast<const double2 *>(s + e));
   const double2 c = __ldg(reinterpret_cast<const double2 *>(s + e + 2));
-  vflux_face(V, qf, g, vmf, a.x, a.y, c.x, c.y, 0.0, F5);
+  visc_flux<5>(V, qf, g, vmf, a.x, a.y, c.x, c.y, 0.0, 0.0, F5);
 #pragma unroll
   for (int m = 0; m < 5; ++m) F[m] = F5[m];
 }
@@ -392,18 +484,17 @@ __device__ __forceinline__ void vface_one(const DevBlock &b, const ViscPar &V, c
 __global__ void k_vface(const DevBlock *__restrict__ blocks, const cosa_params *__restrict__ Pp,
                         const double *__restrict__ qp, const double *__restrict__ si, const double *__restrict__ sj,
                         const double *__restrict__ sk, const double *__restrict__ vm, int64_t n0,
-                        double *__restrict__ fv) {
+                        const VisK V, double *__restrict__ fv) {
   const DevBlock b = blocks[blockIdx.y];
   const int d = blockIdx.z + 1;
   const cosa_params &P = *Pp;
   const int S = 2 * P.nharms + 1, S2 = 2 * P.nharms * P.hbmove + 1;
-  const ViscPar V = make_visc(P);
   const int ni = d == 1 ? b.im : b.im - 1, nj = d == 2 ? b.jm : b.jm - 1, nk = d == 3 ? b.km : b.km - 1;
   const int64_t nf = (int64_t)ni * nj * nk, total = nf * S;
   const double *s = d == 1 ? si : (d == 2 ? sj : sk);
   double *F = fv + (int64_t)(d - 1) * n0 * 5 * S;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-    int64_t r = t;
+    Dec r(t);
     const int i = (int)(r % ni) + 1; r /= ni;
     const int j = (int)(r % nj) + 1; r /= nj;
     const int k = (int)(r % nk) + 1;
@@ -422,10 +513,10 @@ __global__ void k_vface(const DevBlock *__restrict__ blocks, const cosa_params *
 __global__ void k_vwall(const DevBlock *__restrict__ blocks, const WallFace *__restrict__ walls, int nw,
                         const cosa_params *__restrict__ Pp, const double *__restrict__ qp,
                         const double *__restrict__ si, const double *__restrict__ sj, const double *__restrict__ sk,
-                        const double *__restrict__ vm, int64_t n0, double *__restrict__ fv) {
+                        const double *__restrict__ vm, int64_t n0, const VisK V,
+                        double *__restrict__ fv) {
   const cosa_params &P = *Pp;
   const int S = 2 * P.nharms + 1, S2 = 2 * P.nharms * P.hbmove + 1;
-  const ViscPar V = make_visc(P);
   const int64_t total = (int64_t)nw * S;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
     const WallFace w = walls[t % nw];
@@ -438,7 +529,7 @@ __global__ void k_vwall(const DevBlock *__restrict__ blocks, const WallFace *__r
     load_vm(vm + (int64_t)nh * 27 * n0, b, n0, w.d, w.fi, w.fj, w.fk, vmf);
     const double *s = w.d == 1 ? si : (w.d == 2 ? sj : sk);
     const int64_t e = p2_idx(b, S2, 1, w.fi, w.fj, w.fk, nh);
-    vflux_face(V, qf, g, vmf, s[e], s[e + 1], s[e + 2], s[e + 3], 0.0, F);
+    visc_flux<5>(V, qf, g, vmf, s[e], s[e + 1], s[e + 2], s[e + 3], 0.0, 0.0, F);
     double *Fd = fv + (int64_t)(w.d - 1) * n0 * 5 * S;
 #pragma unroll
     for (int m = 0; m < 5; ++m) Fd[f0_idx(b, 5, S, w.fi, w.fj, w.fk, m + 1, n)] = F[m];
@@ -455,7 +546,7 @@ __global__ void k_vdiv(const DevBlock *__restrict__ blocks, const cosa_params *_
   const int64_t total = (int64_t)ni * nj * nk * S;
   const double *Fi = fv, *Fj = fv + n0 * 5 * S, *Fk = fv + 2 * n0 * 5 * S;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-    int64_t r = t;
+    Dec r(t);
     const int i = (int)(r % ni) + 1; r /= ni;
     const int j = (int)(r % nj) + 1; r /= nj;
     const int k = (int)(r % nk) + 1;
@@ -551,7 +642,7 @@ __global__ void k_dt_ns(const DevBlock *__restrict__ blocks, const cosa_params *
   const int ni = b.im - 1, nj = b.jm - 1, nk = b.km - 1;
   const int64_t total = (int64_t)ni * nj * nk * S;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-    int64_t r = t;
+    Dec r(t);
     const int i = (int)(r % ni) + 1; r /= ni;
     const int j = (int)(r % nj) + 1; r /= nj;
     const int k = (int)(r % nk) + 1;
@@ -589,7 +680,7 @@ __global__ void k_lambda_ns(BS bs_, const cosa_params *__restrict__ Pp, const do
   const int ni = b.im - 1, nj = b.jm - 1, nk = b.km - 1;
   const int64_t total = (int64_t)ni * nj * nk * S;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-    int64_t r = t;
+    Dec r(t);
     const int i = (int)(r % ni) + 1; r /= ni;
     const int j = (int)(r % nj) + 1; r /= nj;
     const int k = (int)(r % nk) + 1;
@@ -629,7 +720,7 @@ __global__ void k_deltat_ns(BS bs_, const cosa_params *__restrict__ Pp, double *
   const int ni = b.im - 1, nj = b.jm - 1, nk = b.km - 1;
   const int64_t total = (int64_t)ni * nj * nk * S;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-    int64_t r = t;
+    Dec r(t);
     const int i = (int)(r % ni) + 1; r /= ni;
     const int j = (int)(r % nj) + 1; r /= nj;
     const int k = (int)(r % nk) + 1;
@@ -663,7 +754,7 @@ __global__ void k_qface_qder(BS bs_, int S, const double *__restrict__ q, double
   const int ni = D == 1 ? b.im : b.im - 1, nj = D == 2 ? b.jm : b.jm - 1, nk = D == 3 ? b.km : b.km - 1;
   const int64_t total = (int64_t)ni * nj * nk * S;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-    int64_t r = t;
+    Dec r(t);
     const int i = (int)(r % ni) + 1; r /= ni;
     const int j = (int)(r % nj) + 1; r /= nj;
     const int k = (int)(r % nk) + 1;
@@ -716,7 +807,7 @@ __global__ void k_vflux_ref(DevBlock b, int d, const cosa_params *__restrict__ P
   const int ni = d == 1 ? b.im : b.im - 1, nj = d == 2 ? b.jm : b.jm - 1, nk = d == 3 ? b.km : b.km - 1;
   const int64_t total = (int64_t)ni * nj * nk * S;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-    int64_t r = t;
+    Dec r(t);
     const int i = (int)(r % ni) + 1; r /= ni;
     const int j = (int)(r % nj) + 1; r /= nj;
     const int k = (int)(r % nk) + 1;

@@ -73,7 +73,6 @@ struct LevelState {
   const double *d_vm = nullptr;
   double *d_qprim = nullptr;  // primitive stage state (P3)
   double *d_vflux = nullptr;  // viscous face fluxes of the three families (3 x F0)
-  double *d_vres = nullptr;   // viscous flux balance (P3)
   // k-omega: production, div u, delta+ (scalar P3) and the turbulence IRS
   // coefficients (P1 x S)
   double *d_prd = nullptr, *d_divvel = nullptr, *d_delpls = nullptr;
@@ -817,7 +816,7 @@ int launch_edges(cosa_ctx *c, LevelState &L, double *q, double *mut);
 
 // x extent of a (x, nblocks[, 3]) grid covering `n` items per block
 // viscous part of one stage on the primitive copy of the halo-filled state:
-// q_edges, [time step], face fluxes, wall faces, flux balance -> L.d_vres
+// q_edges, [time step], face fluxes, wall faces -> L.d_vflux
 int launch_visc(cosa_ctx *c, LevelState &L, bool dt, double *bx, double *by, double *bz) {
   const cosa_params &p = c->p;
   const int S = 2 * p.nharms + 1;
@@ -846,8 +845,7 @@ int launch_visc(cosa_ctx *c, LevelState &L, bool dt, double *bx, double *by, dou
                                                          P.sk, L.d_vm, L.n0, vk, L.d_vflux);
     if ((r = after_launch(c))) return r;
   }
-  k_vdiv<<<dim3(grid_x(mc, L.nb), L.nb), 256, 0, c->s>>>(L.d_blocks, c->d_p, L.d_vflux, L.n0, L.d_vres);
-  return after_launch(c);
+  return COSA_OK;
 }
 
 constexpr int kRmsMidRows = 4096, kRmsMid = 148;  // partial rows summed by one CTA; rows left by k_rms_mid
@@ -900,7 +898,8 @@ int launch_faces(cosa_ctx *c, LevelState &L, StageArgs &A, bool want_rms, const 
   A.part = want_rms ? L.d_part : nullptr;
   const LinePar lp = make_line_par(p);
   LineArgs la{L.d_blocks, nullptr, qsrc, {A.si, A.sj, A.sk}, L.d_strong, L.d_smap, A.first_order, 0, nullptr,
-              c->d_status, face_vel_of(c, L)};
+              p.viscous ? L.d_vflux : nullptr, L.n0, c->d_status, face_vel_of(c, L)};
+  const bool vis = p.viscous;
   if (L.schedule == 1 && !p.moving) {
     la.cf = L.d_div;
     if (c->prof.on) cudaEventRecord(c->prof.ev[1][0], c->s);
@@ -909,14 +908,15 @@ int launch_faces(cosa_ctx *c, LevelState &L, StageArgs &A, bool want_rms, const 
       la.tasks = L.d_ctasks + t0;
       const unsigned n = (unsigned)L.nctasks[fam - 1];
       t0 += n;
-#define COSA_CHAIN(M, CV, LM)                                                                                   \
-  (fam == 1 ? k_line_chain<1, M, CV, LM, false> : fam == 2 ? k_line_chain<2, M, CV, LM, false>                  \
-                                                : want_rms ? k_line_chain<3, M, CV, LM, true>                   \
-                                                           : k_line_chain<3, M, CV, LM, false>)
-      auto k = mixed ? (conv ? (lim1 ? COSA_CHAIN(true, true, true) : COSA_CHAIN(true, true, false))
-                             : (lim1 ? COSA_CHAIN(true, false, true) : COSA_CHAIN(true, false, false)))
-                     : (conv ? (lim1 ? COSA_CHAIN(false, true, true) : COSA_CHAIN(false, true, false))
-                             : (lim1 ? COSA_CHAIN(false, false, true) : COSA_CHAIN(false, false, false)));
+#define COSA_CHAIN(M, CV, LM, VI)                                                                               \
+  (fam == 1 ? k_line_chain<1, M, CV, LM, false, VI> : fam == 2 ? k_line_chain<2, M, CV, LM, false, VI>          \
+                                                    : want_rms ? k_line_chain<3, M, CV, LM, true, VI>           \
+                                                               : k_line_chain<3, M, CV, LM, false, VI>)
+      auto k = vis     ? (lim1 ? COSA_CHAIN(false, false, true, true) : COSA_CHAIN(false, false, false, true))
+               : mixed ? (conv ? (lim1 ? COSA_CHAIN(true, true, true, false) : COSA_CHAIN(true, true, false, false))
+                               : (lim1 ? COSA_CHAIN(true, false, true, false) : COSA_CHAIN(true, false, false, false)))
+                       : (conv ? (lim1 ? COSA_CHAIN(false, true, true, false) : COSA_CHAIN(false, true, false, false))
+                               : (lim1 ? COSA_CHAIN(false, false, true, false) : COSA_CHAIN(false, false, false, false)));
 #undef COSA_CHAIN
       k<<<n, 32, 0, c->s>>>(lp, la, A, c->d_p);
       if ((r = after_launch(c))) return r;
@@ -930,11 +930,11 @@ int launch_faces(cosa_ctx *c, LevelState &L, StageArgs &A, bool want_rms, const 
     la.n0 = L.cflux_n0;
     la.tasks = L.d_ftasks + G.t0;
     if (c->prof.on) cudaEventRecord(c->prof.ev[1][0], c->s);
-#define COSA_STORE(M, CV, MV) (lim1 ? k_line_store<M, CV, MV, true> : k_line_store<M, CV, MV, false>)
-    auto k = p.moving ? (mixed ? (conv ? COSA_STORE(true, true, true) : COSA_STORE(true, false, true))
-                               : (conv ? COSA_STORE(false, true, true) : COSA_STORE(false, false, true)))
-                      : (mixed ? (conv ? COSA_STORE(true, true, false) : COSA_STORE(true, false, false))
-                               : (conv ? COSA_STORE(false, true, false) : COSA_STORE(false, false, false)));
+#define COSA_STORE(M, CV, MV, VI) (lim1 ? k_line_store<M, CV, MV, true, VI> : k_line_store<M, CV, MV, false, VI>)
+    auto k = vis ? (p.moving ? COSA_STORE(false, false, true, true) : COSA_STORE(false, false, false, true))
+             : p.moving ? (mixed ? COSA_STORE(true, true, true, false) : COSA_STORE(false, true, true, false))
+                        : (mixed ? (conv ? COSA_STORE(true, true, false, false) : COSA_STORE(true, false, false, false))
+                                 : (conv ? COSA_STORE(false, true, false, false) : COSA_STORE(false, false, false, false)));
 #undef COSA_STORE
     k<<<(unsigned)G.nt, 32, 0, c->s>>>(lp, la);
     if ((r = after_launch(c))) return r;
@@ -999,12 +999,11 @@ int launch_stage(cosa_ctx *c, int nl, LevelState &L, double *qin, double *qout, 
   if (!p.viscous) return launch_faces(c, L, A, want_rms, qin, !prim_in);
   // primitive copy (with bprtest) shared by the viscous and convective faces;
   // the viscous terms and, on stage 1, the viscous time step come first
-  if (!L.d_vm || !L.d_vres || !L.d_qprim || !P.vol) return COSA_ERR_ARG;
+  if (!L.d_vm || !L.d_vflux || !L.d_qprim || !P.vol) return COSA_ERR_ARG;
   int64_t m3 = 0;
   for (const DevBlock &x : L.hb) m3 = std::max<int64_t>(m3, x.P3 * S);
   k_prim<<<dim3(grid_x(m3, L.nb), L.nb), 256, 0, c->s>>>(L.d_blocks, c->d_p, qin, L.d_qprim, c->d_status);
   if ((r = after_launch(c)) || (r = launch_visc(c, L, compute_dt != 0, A.bx, A.by, A.bz))) return r;
-  A.vres = L.d_vres;
   A.compute_dt = 0;
   A.bx = A.by = A.bz = nullptr;
   return launch_faces(c, L, A, want_rms, L.d_qprim, false);
@@ -2657,10 +2656,8 @@ int cosa_gpu_viscous_setup(cosa_ctx *c, int32_t nl, double *x, double *y, double
   const int S = 2 * c->p.nharms + 1;
   const size_t n3 = (size_t)L->n3 * 5 * S;
   if (!L->d_qprim && (r = dalloc(c, &L->d_qprim, n3))) return r;
-  if (!L->d_vres && (r = dalloc(c, &L->d_vres, n3))) return r;
   if (!L->d_vflux && (r = dalloc(c, &L->d_vflux, (size_t)3 * L->n0 * 5 * S))) return r;
   CK(cudaMemsetAsync(L->d_qprim, 0, n3 * sizeof(double), c->s));
-  CK(cudaMemsetAsync(L->d_vres, 0, n3 * sizeof(double), c->s));
   CK(cudaMemsetAsync(L->d_vflux, 0, (size_t)3 * L->n0 * 5 * S * sizeof(double), c->s));
   L->d_vm = vm;
   drop_graphs(c);
@@ -3593,7 +3590,7 @@ int ensure_chain(cosa_ctx *c, LevelState &L) {
 // cycle, store / chain in us: ducts of 33 k cells 85 / 110, 131 k
 // 148 / 179, 295 k 298 / 333, 590 k (one block) 509 / 495, (eight) 601 / 608,
 // 655 k 594 / 596; two-cell-thick channels of 131 k 175 / 186, 262 k 315 / 319,
-// 1.05 M 925 / 829; 30.7 M cells (24 blocks): store's fluxes no longer fit L2.
+// 1.05 M 925 / 829; larger grids leave store's fluxes no room in L2.
 constexpr int64_t kChainCells = 600000;
 int default_schedule(const cosa_ctx *c, const LevelState &L) {
   return c->nseg == 0 && !c->p.moving && level_cells(c, L) >= kChainCells ? 1 : 0;

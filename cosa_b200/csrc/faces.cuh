@@ -263,6 +263,8 @@ struct LineArgs {
   int first_order;
   int64_t n0;
   double *cf;                    // store: fluxes of the three families; chain: D (F0 layout)
+  const double *vf;              // viscous fluxes of the three families (F0 planes of nv cells), added to the faces', or null
+  int64_t nv;
   int *status;
   FaceVel fv;
 };
@@ -288,16 +290,19 @@ __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0
 // registers.  I: cells (with the two beyond the warp's) and metrics; M: the
 // next cell, the face's metrics and, in the chain, the running balance D, the
 // base state and the time step of the cell that the face closes
+template <bool VIS>
 struct StageI {
   double q[2][5][34];
   double2 met[2][2][32];
+  double vis[2][VIS ? 5 : 1][32];
 };
-template <int OUT>
+template <int OUT, bool VIS>
 struct StageM {
   double q[2][5][32];
   double2 met[2][2][32];
   double D[2][OUT >= 1 ? 5 : 1][32];
   double base[2][OUT == 2 ? 6 : 1][32];
+  double vis[2][VIS ? 5 : 1][32];
 };
 // normal speed of a face from its velocity: sijk(5)*kx + sijk(6)*ky +
 // sijk(7)*kz, roflux_b's order (src/flux.f90:110-113)
@@ -305,8 +310,8 @@ __device__ __forceinline__ double face_ubn(const double *__restrict__ v, double 
   return __fma_rn(__ldg(v + 2), kz, __fma_rn(__ldg(v + 1), ky, __dmul_rn(__ldg(v), kx)));
 }
 
-// what a cell's flux balance r goes through after the three families: viscous
-// balance, harmonic-balance source, norms, forcing, update (k_cells and the
+// what a cell's flux balance r goes through after the three families:
+// harmonic-balance source, norms, forcing, update (k_cells and the
 // last launch of the chain).  co: the cell in the state arrays (variable 1 of
 // snapshot n), P3 their variable stride; q0: the cell's base state (read when
 // A.update)
@@ -318,7 +323,6 @@ __device__ __forceinline__ void finish_cell(const StageArgs &A, const cosa_param
 #pragma unroll
   for (int m = 0; m < 5; ++m) {
     const int64_t o = co + m * P3;
-    if (A.vres) r[m] = r[m] + A.vres[o];
     if (A.vol) {
       // src_bhb (src/src.f90:556-613)
       double qhb = 0.0;
@@ -354,8 +358,8 @@ __device__ __forceinline__ void finish_cell(const StageArgs &A, const cosa_param
 
 // i-face rows of one task.  OUT 0: fluxes stored; 1: D = F(c+1) - F(c) of the
 // 30 cells between the task's 31 faces
-template <bool MIXED, bool CONV, bool MV, bool LIM1, int OUT>
-__device__ __forceinline__ void line_i(const FaceTask &T, const LinePar &LP, const LineArgs &L, StageI &B, int lane) {
+template <bool MIXED, bool CONV, bool MV, bool LIM1, int OUT, bool VIS>
+__device__ __forceinline__ void line_i(const FaceTask &T, const LinePar &LP, const LineArgs &L, StageI<VIS> &B, int lane) {
   const DevBlock &b = L.blocks[T.blk];
   const PhysPar &ph = LP.ph;
   const int n = T.n, nh = n * LP.hbmove, k = T.tb, mx = b.im;
@@ -379,6 +383,7 @@ __device__ __forceinline__ void line_i(const FaceTask &T, const LinePar &LP, con
   double *Fp = L.cf + f0_idx(b, 5, LP.S, min(max(c, 1), mx), T.ta, k, 1, n);
   const int64_t mrow = (int64_t)(b.im + 2) * 4;
   const int frow = b.im;
+  const double *Vp = VIS ? L.vf + f0_idx(b, 5, LP.S, min(max(c, 1), mx), T.ta, k, 1, n) : nullptr;
   auto issue = [&](int slot) {
 #pragma unroll
     for (int m = 0; m < 5; ++m) cp8(&B.q[slot][m][lane + 1], qb + (int)o0 + (int64_t)m * P3);
@@ -388,6 +393,10 @@ __device__ __forceinline__ void line_i(const FaceTask &T, const LinePar &LP, con
     }
     cp16(&B.met[slot][0][lane], sp);
     cp16(&B.met[slot][1][lane], sp + 2);
+    if (VIS) {
+#pragma unroll
+      for (int m = 0; m < 5; ++m) cp8(&B.vis[slot][VIS ? m : 0][lane], Vp + (int64_t)m * fv);
+    }
     cp_commit();
   };
   issue(0);
@@ -397,6 +406,7 @@ __device__ __forceinline__ void line_i(const FaceTask &T, const LinePar &LP, con
     if (row + 1 < T.nf) {
       qb += qrow;
       sp += mrow;
+      if (VIS) Vp += frow;
       issue(slot ^ 1);
       cp_wait<1>();
     } else {
@@ -482,6 +492,10 @@ __device__ __forceinline__ void line_i(const FaceTask &T, const LinePar &LP, con
       const double ubn = MV ? face_ubn(vp, met[0], met[1], met[2]) : 0.0;
       face_flux_mixed<MV>(ph, (float)ph.g, (float)ph.g_gm1, met, qm, bm1, b0, dlr, dqL, dqR, F, ubn);
     }
+    if (VIS) {
+#pragma unroll
+      for (int m = 0; m < 5; ++m) F[m] = F[m] + B.vis[slot][VIS ? m : 0][lane];
+    }
     if (OUT == 0) {
       if (face) {
 #pragma unroll
@@ -504,9 +518,9 @@ __device__ __forceinline__ void line_i(const FaceTask &T, const LinePar &LP, con
 // a segment of j or k faces, lanes along i.  OUT 0: fluxes stored; 1: the
 // flux differences of the segment's nf - 1 cells added to D; 2: D with them
 // added goes through finish_cell
-template <bool MIXED, bool CONV, bool MV, bool LIM1, int OUT, bool RMS>
+template <bool MIXED, bool CONV, bool MV, bool LIM1, int OUT, bool RMS, bool VIS>
 __device__ __forceinline__ void line_m(const FaceTask &T, const LinePar &LP, const LineArgs &L, const StageArgs &A,
-                                       const cosa_params *Pp, int part_row, StageM<OUT> &B, int lane) {
+                                       const cosa_params *Pp, int part_row, StageM<OUT, VIS> &B, int lane) {
   const DevBlock &b = L.blocks[T.blk];
   const PhysPar &ph = LP.ph;
   const int d = T.d, n = T.n, nh = n * LP.hbmove, tb = T.tb, f0 = T.f0, f1 = T.f0 + T.nf;
@@ -533,6 +547,9 @@ __device__ __forceinline__ void line_m(const FaceTask &T, const LinePar &LP, con
   const double *vp = MV ? (d == 2 ? L.fv.f[1] : L.fv.f[2]) + e0 / 4 * 3 : nullptr;
   double *Fp = L.cf + (OUT == 0 ? (int64_t)(d - 1) * L.n0 * 5 * LP.S : 0) +
                (d == 2 ? f0_idx(b, 5, LP.S, i, f0, tb, 1, n) : f0_idx(b, 5, LP.S, i, tb, f0, 1, n));
+  const double *Vp = VIS ? L.vf + (int64_t)(d - 1) * L.nv * 5 * LP.S +
+                               (d == 2 ? f0_idx(b, 5, LP.S, i, f0, tb, 1, n) : f0_idx(b, 5, LP.S, i, tb, f0, 1, n))
+                         : nullptr;
   double qc[5];
   double acc[5] = {0, 0, 0, 0, 0};
   // the running left state: cell f - 1 on face f; FP64: ql the state, a the
@@ -559,6 +576,11 @@ __device__ __forceinline__ void line_m(const FaceTask &T, const LinePar &LP, con
     cp16(&B.met[slot][0][lane], ns);
     cp16(&B.met[slot][1][lane], ns + 2);
     ns += mstep;
+    if (VIS) {
+#pragma unroll
+      for (int m = 0; m < 5; ++m) cp8(&B.vis[slot][VIS ? m : 0][lane], Vp + (int64_t)m * fv);
+      Vp += fstep;
+    }
     if (OUT >= 1 && !first) {
 #pragma unroll
       for (int m = 0; m < 5; ++m) cp8(&B.D[slot][m][lane], nD + (int64_t)m * fv);
@@ -680,6 +702,10 @@ __device__ __forceinline__ void line_m(const FaceTask &T, const LinePar &LP, con
         dm[m] = up[m];
       }
     }
+    if (VIS) {
+#pragma unroll
+      for (int m = 0; m < 5; ++m) F[m] = F[m] + B.vis[slot][VIS ? m : 0][lane];
+    }
     if (OUT == 0) {
       if (act) {
 #pragma unroll
@@ -730,28 +756,31 @@ __device__ __forceinline__ void line_m(const FaceTask &T, const LinePar &LP, con
 // precision fits 16 everywhere (18: 6.2 against 5.2 ms on the 4.2 M-cell duct).
 constexpr int kWarpsStore = 16, kWarpsI = 16, kWarpsM = 12, kWarpsMixed = 16;
 
-// store schedule: all faces, the task's family picks the loop
-template <bool MIXED, bool CONV, bool MV, bool LIM1>
+// store schedule: all faces, the task's family picks the loop.  VIS: viscous
+// flows, whose stage input is the primitive copy and whose faces add their
+// viscous flux (a flux balance of its own moved 200 B a cell more: one cycle of
+// the 4.2 M-cell laminar duct 7.27 ms with it, 6.17 ms without)
+template <bool MIXED, bool CONV, bool MV, bool LIM1, bool VIS>
 __global__ void __launch_bounds__(32, MIXED ? kWarpsMixed : kWarpsStore)
 k_line_store(const LinePar LP, const LineArgs L) {
   __shared__ union {
-    StageI i;
-    StageM<0> m;
+    StageI<VIS> i;
+    StageM<0, VIS> m;
   } B;
   const FaceTask T = L.tasks[blockIdx.x];
-  if (T.d == 1) line_i<MIXED, CONV, MV, LIM1, 0>(T, LP, L, B.i, threadIdx.x);
-  else line_m<MIXED, CONV, MV, LIM1, 0, false>(T, LP, L, StageArgs{}, nullptr, 0, B.m, threadIdx.x);
+  if (T.d == 1) line_i<MIXED, CONV, MV, LIM1, 0, VIS>(T, LP, L, B.i, threadIdx.x);
+  else line_m<MIXED, CONV, MV, LIM1, 0, false, VIS>(T, LP, L, StageArgs{}, nullptr, 0, B.m, threadIdx.x);
 }
 // chain schedule: family FAM; FAM 3 finishes the stage
-template <int FAM, bool MIXED, bool CONV, bool LIM1, bool RMS>
+template <int FAM, bool MIXED, bool CONV, bool LIM1, bool RMS, bool VIS>
 __global__ void __launch_bounds__(32, MIXED ? kWarpsMixed : FAM == 1 ? kWarpsI : kWarpsM)
 k_line_chain(const LinePar LP, const LineArgs L, const StageArgs A, const cosa_params *__restrict__ Pp) {
   const FaceTask T = L.tasks[blockIdx.x];
   if constexpr (FAM == 1) {
-    __shared__ StageI B;
-    line_i<MIXED, CONV, false, LIM1, 1>(T, LP, L, B, threadIdx.x);
+    __shared__ StageI<VIS> B;
+    line_i<MIXED, CONV, false, LIM1, 1, VIS>(T, LP, L, B, threadIdx.x);
   } else {
-    __shared__ StageM<FAM - 1> B;
-    line_m<MIXED, CONV, false, LIM1, FAM - 1, RMS>(T, LP, L, A, Pp, blockIdx.x, B, threadIdx.x);
+    __shared__ StageM<FAM - 1, VIS> B;
+    line_m<MIXED, CONV, false, LIM1, FAM - 1, RMS, VIS>(T, LP, L, A, Pp, blockIdx.x, B, threadIdx.x);
   }
 }

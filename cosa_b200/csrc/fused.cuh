@@ -208,7 +208,6 @@ struct StageArgs {
   double *res_out;       // if set, the residual is stored here (P3 layout)
   double *bx, *by, *bz;  // IRS coefficients written with the time step (irsop >= 2)
   const double *vol;     // cell volumes when the harmonic-balance source is on
-  const double *vres;    // viscous flux balance of each cell (P3 layout), added to the residual, or null
   const uint8_t *strong; // strong-boundary flags
   const StrongMap *smap; // per block
   int *status;

@@ -19,8 +19,7 @@
 //                            every face of the three families in one launch
 //   k_vwall                  the same on strong-boundary faces with the
 //                            one-sided wall formulas, overwriting k_vface
-//   k_vdiv                   flux balance of each cell; the fused stage
-//                            kernel adds it to the convective residual
+//   (the line kernels of faces.cuh add the viscous flux to their faces')
 // Per-routine kernels with the reference's array contract (q_face, q_der,
 // vflux, lambda/deltat) use the same device functions.
 #pragma once
@@ -291,6 +290,10 @@ __host__ __device__ __forceinline__ ViscPar make_visc(const cosa_params &P) {
 // Sutherland's law in the reference's non-dimensional form, t^1.5 = t sqrt(t)
 __device__ __forceinline__ double sutherland(double t, double stemp) { return (stemp + 1) / (t + stemp) * (t * sqrt(t)); }
 
+// Sutherland's law with t^1.5 = t^2 / sqrt(t), no division
+__device__ __forceinline__ double sutherland_nr(double t, double stemp) {
+  return (stemp + 1) * rcp_nr(t + stemp) * (t * t * rsqrt_nr(t));
+}
 // viscous flux of one face: qf primitive face state, g[dir][var] the
 // gradients along xi, eta, zeta, vmf[m*3+c] the face's inverse metrics,
 // (kx, ky, kz, ds) the face normal and area; the energy row keeps the
@@ -357,10 +360,6 @@ inline VisK make_visk(const cosa_params &P) {
   k.g1 = k.b1 / bstr - k.sigw1 * kap2; k.g2 = k.b2 / bstr - k.sigw2 * kap2;
   k.igm1 = 1 / (P.gamma - 1);
   return k;
-}
-// Sutherland's law with t^1.5 = t^2 / sqrt(t), no division
-__device__ __forceinline__ double sutherland_nr(double t, double stemp) {
-  return (stemp + 1) * rcp_nr(t + stemp) * (t * t * rsqrt_nr(t));
 }
 // F1 of BSL/SST (blend_f1 in kom.cuh) from the reciprocals of rho and omega
 __device__ __forceinline__ double blend_f1_nr(const VisK &V, double rho, double ir, double tke, double io, double mu,
@@ -536,32 +535,6 @@ __global__ void k_vwall(const DevBlock *__restrict__ blocks, const WallFace *__r
   }
 }
 
-// flux balance of each cell, summed like bresid (src/cosa.f90:1149-1200)
-__global__ void k_vdiv(const DevBlock *__restrict__ blocks, const cosa_params *__restrict__ Pp,
-                       const double *__restrict__ fv, int64_t n0, double *__restrict__ vres) {
-  const DevBlock b = blocks[blockIdx.y];
-  const cosa_params &P = *Pp;
-  const int S = 2 * P.nharms + 1;
-  const int ni = b.im - 1, nj = b.jm - 1, nk = b.km - 1;
-  const int64_t total = (int64_t)ni * nj * nk * S;
-  const double *Fi = fv, *Fj = fv + n0 * 5 * S, *Fk = fv + 2 * n0 * 5 * S;
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-    Dec r(t);
-    const int i = (int)(r % ni) + 1; r /= ni;
-    const int j = (int)(r % nj) + 1; r /= nj;
-    const int k = (int)(r % nk) + 1;
-    const int n = (int)(r / nk);
-    const int64_t cell = p3_cell(b, i, j, k);
-#pragma unroll
-    for (int m = 0; m < 5; ++m) {
-      double x = Fi[f0_idx(b, 5, S, i + 1, j, k, m + 1, n)] - Fi[f0_idx(b, 5, S, i, j, k, m + 1, n)];
-      x = x + Fj[f0_idx(b, 5, S, i, j + 1, k, m + 1, n)] - Fj[f0_idx(b, 5, S, i, j, k, m + 1, n)];
-      x = x + Fk[f0_idx(b, 5, S, i, j, k + 1, m + 1, n)] - Fk[f0_idx(b, 5, S, i, j, k, m + 1, n)];
-      vres[p3_var(b, 5, S, m + 1, n) + cell] = x;
-    }
-  }
-}
-
 // ---- lambdab viscous branch + eig_ns + bdeltat (src/cosa.f90:1349-1423,
 // 4239-4297, 4831-5010) ---------------------------------------------------------------
 // convective and viscous spectral radii of cell (i,j,k); the + neighbour's
@@ -587,20 +560,23 @@ __device__ __forceinline__ void eig_ns_cell(const DevBlock &b, const cosa_params
   else
     eig_eul(g, qc, sm[0], sp[0], sm[1], sp[1], sm[2], sp[2], lam[0], lam[1], lam[2], gv);
   const double rho = qc[0];
-  const double mu = sutherland(g * qc[4] / rho, st);
+  // seven temperatures and viscosities: reciprocals instead of divisions (a
+  // third of the kernel's time on the 4.2 M-cell duct)
+  const double mu = sutherland_nr(g * qc[4] * rcp_nr(rho), st);
   auto MUT = [&](int a, int c, int e) { return mut ? mut[b.op3 * S + (int64_t)n * b.P3 + p3_cell(b, a, c, e)] : 0.0; };
   const double mutc = MUT(i, j, k);
+  const double cv = P.cdff * g * P.machfs / P.reyno * rcp_nr(rho * volc), ipl = 1 / P.pranl, ipt = 1 / P.prant;
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
     const int a = d == 0, c = d == 1, e = d == 2;
-    const double rhom = Q(i - a, j - c, k - e, 0);
-    const double tm = g * Q(i - a, j - c, k - e, 4) / rhom;
-    const double tp = g * Q(i + a, j + c, k + e, 4) / rhom;
-    const double mum = sutherland(tm, st), mup = sutherland(tp, st);
+    const double irm = rcp_nr(Q(i - a, j - c, k - e, 0));
+    const double tm = g * Q(i - a, j - c, k - e, 4) * irm;
+    const double tp = g * Q(i + a, j + c, k + e, 4) * irm;
+    const double mum = sutherland_nr(tm, st), mup = sutherland_nr(tp, st);
     const double mud = (mum + 2 * mu + mup) / 4;
     const double mutd = (MUT(i - a, j - c, k - e) + 2 * mutc + MUT(i + a, j + c, k + e)) / 4;
     const double area = (sm[d][3] + sp[d][3]) / 2;
-    lamv[d] = P.cdff * area * area * g * P.machfs / P.reyno * (mud / P.pranl + mutd / P.prant) / (rho * volc);
+    lamv[d] = area * area * cv * (mud * ipl + mutd * ipt);
   }
 }
 
